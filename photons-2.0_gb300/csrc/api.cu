@@ -292,7 +292,7 @@ static void free_all(photons_ctx *c)
                     c->az, c->M, c->L, c->io, c->work_counter, c->t.chi, c->t.clo, c->t.w32, c->t.son2, c->M32,
                     b.lvl_begin, b.lvl_count, b.leaf_begin, b.leaf_count, c->t.depth_cnt, b.tn_boxid, b.tl_boxid,
                     c->t.boxid, b.boxes, c->far_gate, c->mu_sorted, c->mu_nrecv, c->mu_slot, c->mu_over,
-                    c->mu_size, c->mu_rbase, c->mu_total, c->mu_scan, c->mu_buf, c->mu_ev, c->mu_nev, c->mu_pq,
+                    c->mu_size, c->mu_rbase, c->mu_total, c->mu_scan, c->mu_buf, c->mu_ev, c->mu_nev, c->mu_pq, c->mu_items, c->mu_nitems,
                     b.tn_subroot, b.tl_subroot, b.ch_swap, c->t.depth_blk};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -500,9 +500,9 @@ static int mutual_status(int over)
 #ifndef MU_MIN_LEAF
 #define MU_MIN_LEAF 48
 #endif
-// FP64 passes use mutual pairs at every leaf size: the pair force is ~70
-// FP64 operations, so evaluating each symmetric pair once halves the pass
-// whatever the pairing costs.
+// FP64 passes use mutual pairs at every leaf size: the FP64 pipe bounds the
+// pass, and evaluating each symmetric pair once takes 13 FP64 instructions a
+// pair where both ways take 20, whatever the pairing costs.
 static bool uses_mutual(const photons_ctx *c, int precision)
 {
     if (c->mu_off || (c->pass_flags & PHOTONS_F_ONE_WAY)) return false;
@@ -519,15 +519,34 @@ static int alloc_mutual(photons_ctx *c, int precision)
     // floats per particle and entry (256^3 leaf 64 needs ~180 per particle);
     // a pass that needs more repeats once with the measured size
     long long want = (c->hint_mubuf ? c->hint_mubuf : (long long)c->n * 192 + 4096) * mu_per_value(precision);
-    // the reaction slots take ~700 bytes per particle: where they would not
-    // leave 1 GB of the device free, this context evaluates every pair one way
+    // FP64 work items: a leaf's evaluated entries in segments, rounded up
+    const long long want_items = precision == PHOTONS_FP64 ? c->w.p2p_cap / ph::mu64_seg(c->pp.maxleaf) + c->cap_u : 0;
+    // the reaction slots take ~700 bytes per particle (halos in FP64 several
+    // times that: their long lists are paired too).  Where they would not
+    // leave 1 GB of the device free, an FP64 pass pairs the shorter lists
+    // only, as the FP32 ones do; where that does not fit, this context
+    // evaluates every pair one way
     size_t grow = 0, free_b = 0, total_b = 0;
     if (c->w.p2p_cap > c->mu_slot_cap) grow += (size_t)(c->w.p2p_cap - c->mu_slot_cap) * (2 * sizeof(int) + sizeof(int2));
+    if (want_items > c->mu_items_cap) grow += (size_t)(want_items - c->mu_items_cap) * sizeof(int2);
     if (want > c->mu_buf_cap) grow += (size_t)(want - c->mu_buf_cap) * sizeof(float);
     if (grow && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && grow + ((size_t)1 << 30) > free_b) {
-        c->mu_off = true;
         c->epoch++;
+        if (precision == PHOTONS_FP64 && c->mu_sort_long) {
+            c->mu_sort_long = false;
+            c->hint_mubuf = 0;
+            return alloc_mutual(c, precision);
+        }
+        c->mu_off = true;
         return 0;
+    }
+    if (want_items > c->mu_items_cap) {
+        c->mu_items_cap = 0;
+        c->epoch++;
+        PH_TRY(dalloc(c->mu_items, (size_t)want_items));
+        if (!c->mu_nitems) PH_TRY(dalloc(c->mu_nitems, 1));
+        c->mu_items_cap = want_items;
+        c->epoch++;
     }
     if (c->w.p2p_cap > c->mu_slot_cap) {
         c->mu_slot_cap = 0;
@@ -894,6 +913,29 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
     return ph_set_error(PH_ERR_CAPACITY, "interaction lists did not fit after repeated growth");
 }
 
+// The reaction buffer for the pairing just enqueued: waits for its total and
+// grows the buffer to it where the device has the room (else every pair of
+// this pass runs one way)
+static int grow_reactions(photons_ctx *c, int precision)
+{
+    long long need = 0;
+    PH_CUDA_CHECK(cudaMemcpyAsync(&need, c->mu_total, sizeof need, cudaMemcpyDeviceToHost, c->stream));
+    PH_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+    if (need <= c->mu_buf_cap / mu_per_value(precision)) return 0;
+    const long long hint = need + need / 16 + 4096, want = hint * mu_per_value(precision);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+        (size_t)(want - c->mu_buf_cap) * sizeof(float) + ((size_t)1 << 30) > free_b)
+        return 0;
+    c->hint_mubuf = hint;
+    c->mu_buf_cap = 0;
+    c->epoch++;
+    PH_TRY(dalloc(c->mu_buf, (size_t)want));
+    c->mu_buf_cap = want;
+    c->epoch++;
+    return 0;
+}
+
 int ph_stage_p2p(photons_ctx *c, int precision, int zero)
 {
     cudaStream_t st = c->stream;
@@ -935,7 +977,14 @@ int ph_stage_p2p(photons_ctx *c, int precision, int zero)
         m.sorted = c->mu_sorted; m.nrecv = c->mu_nrecv; m.size = c->mu_size; m.rbase = c->mu_rbase;
         m.total = c->mu_total; m.scan_scratch = c->mu_scan; m.slot = c->mu_slot; m.over = c->mu_over;
         m.ev = c->mu_ev; m.nev = c->mu_nev; m.maxleaf = c->pp.maxleaf; m.pq = c->mu_pq;
-        m.buf = c->mu_buf; m.buf_cap = c->mu_buf_cap / mu_per_value(precision); m.cap_leaves = c->mu_cap_leaves;
+        m.items = c->mu_items; m.nitems = c->mu_nitems; m.sort_long = c->mu_sort_long;
+        m.repeats = c->capturing ? 1 : 0;
+        m.cap_leaves = c->mu_cap_leaves;
+        PH_TRY(ph::launch_mutual_pairing(a, m, precision == PHOTONS_FP64, st));
+        // outside a captured pass the reaction buffer is sized before the pairs
+        // are evaluated (a captured pass that needs more is repeated)
+        if (!c->capturing) PH_TRY(grow_reactions(c, precision));
+        m.buf = c->mu_buf; m.buf_cap = c->mu_buf_cap / mu_per_value(precision);
         PH_TRY(ph::launch_p2p_mutual(a, m, precision == PHOTONS_FP64, st));
     } else {
         if (a.variant == 2) a.variant = 0;

@@ -70,10 +70,14 @@ struct photons_ctx {
     long long *mu_size = nullptr, *mu_rbase = nullptr, *mu_total = nullptr, *mu_scan = nullptr;
     int *mu_nev = nullptr;
     int *mu_pq = nullptr;
+    int2 *mu_items = nullptr;  // FP64 work items
+    int *mu_nitems = nullptr;
     int2 *mu_ev = nullptr;
     float *mu_buf = nullptr;
     long long mu_buf_cap = 0, mu_slot_cap = 0, hint_mubuf = 0;
+    long long mu_items_cap = 0;
     bool mu_off = false;  // the reaction slots did not fit: every pair one way
+    bool mu_sort_long = true;  // FP64: lists above 1024 entries paired too (until their slots do not fit)
     int pass_flags = 0;   // PHOTONS_F_* of the pass being prepared
     int mu_cap_leaves = 0;
     // PM mesh (pm.cu): density / potential, half spectrum, gradient grids, FFT plans

@@ -60,11 +60,20 @@ struct MutualBufs {
     int *nev;                // per leaf: their number
     int maxleaf;             // selects the kernel build
     int *pq;                 // per pool entry: received rank, or the owned pair's partner position
+    // FP64 passes: the work items (leaf, segment of its evaluated entries), their
+    // number, and whether lists above 1024 entries are sorted too
+    int2 *items;
+    int *nitems;
+    int sort_long;
+    int repeats;             // a pass whose reactions do not fit is repeated: it evaluates nothing
 };
 
 SplitConsts make_split_consts(const PassParams &p);
-// FP32 P2P with mutual pairs (MAXLEAF <= 64; chosen for 48-64): sorts the
-// lists, pairs the entries, evaluates, adds the received reactions
+int mu64_seg(int maxleaf);  // evaluated entries per FP64 work item
+// P2P with mutual pairs (FP32: MAXLEAF <= 64, chosen for 48-64), in two
+// steps: sort the lists and pair the entries (m.total: reaction values
+// needed); assign the slots, evaluate, add the received reactions
+int launch_mutual_pairing(const P2PArgs &a, const MutualBufs &m, int fp64, cudaStream_t st);
 int launch_p2p_mutual(const P2PArgs &a, const MutualBufs &m, int fp64, cudaStream_t st);
 // the FP64 kernels' split factor g(u) at n device points (exact: erfc and exp)
 int launch_split_factor_fp64(const double *u, int n, int exact, double *g, cudaStream_t st);

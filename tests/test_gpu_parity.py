@@ -398,3 +398,22 @@ def test_c2_zeldovich256_full_size_lists_match_oracle(ph, fp, ics, port):
     pos, p = ics.make("zeldovich256", maxleaf=64)
     e = _full_size_parity(ph, fp, port, pos, p, ph.FP32_SPLIT, 1e-3)
     assert np.median(e) <= 2e-6, np.median(e)
+
+
+@pytest.mark.parametrize("workload,nside,maxleaf,eps", [
+    ("nfw128", 32, 2, None),     # lists of several thousand entries, one-particle leaves
+    ("nfw128", 24, 8, 0.0),      # no softening: close pairs below the pair tables
+    ("grid32", 16, 33, 2.0),     # softening of 2 rs: most pairs inside it; 33 targets (the 64-slot lanes)
+    ("grid32", 18, 100, None),   # leaves above 64: two chunks of targets
+    ("grid32", 16, 17, None)])
+def test_fp64_pair_paths_match_oracle(ph, fp, ics, port, workload, nside, maxleaf, eps):
+    """FP64 passes that leave the common path of the pair kernel (tolerance:
+    the FP64 bar of this file)."""
+    pos, p = ics.make(workload, nside=nside, maxleaf=maxleaf)
+    if eps is not None:
+        p["eps"] = eps * p["rs"]
+    r = port.run(pos, p, capture=False, tree=False, nthreads=8)
+    acc = fp.run(pos, p, precision=ph.FP64)
+    acc_ref = np.empty_like(r["acc"])
+    acc_ref[r["perm"]] = r["acc"]
+    assert rel_err(acc, acc_ref, p).max() <= FP64_TOL

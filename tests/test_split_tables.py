@@ -76,3 +76,48 @@ def test_device_split_factor_matches_erfc_and_exp(ph):
     err = np.abs(tab - exact)
     assert err.max() <= 5e-16, err.max()
     assert np.array_equal(tab[u >= 8.0], exact[u >= 8.0])  # beyond the table: erfc and exp
+
+
+# ---- the pair force's fixed-point tables (csrc/fit_pair_fp64.py) ----
+
+def pair_fit():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("fit_pair_fp64", os.path.join(CSRC, "fit_pair_fp64.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+def test_pair_table_is_the_fit_scripts_output():
+    pytest.importorskip("mpmath")
+    out = subprocess.run([sys.executable, os.path.join(CSRC, "fit_pair_fp64.py")], capture_output=True, text=True,
+                         check=True).stdout
+    assert out == open(os.path.join(CSRC, "pair_fp64_table.h")).read()
+
+
+@pytest.mark.parametrize("octave", [-14, -7, -1, 0, 1, 2, 3, 5])
+def test_pair_table_at_interval_edges(octave):
+    """The kernels' integer evaluation (replayed) next to interval and octave
+    edges: half an ulp of f's double plus half an ulp of the fixed-point sum
+    (2^-53 + 2^-54 of f) below q = 4, and 2^-54 of the Newtonian factor
+    (f over g) from there on, where the tables keep fewer bits of f."""
+    mp = pytest.importorskip("mpmath")
+    import struct
+    fit = pair_fit()
+    mp.mp.dps = 60
+    tab = {}
+    for i in (0, 1, 31, 62, 63):
+        j = ((octave - fit.OCT_LO) << fit.MB) + i
+        tab[j] = fit.interval(j)
+    mp.mp.dps = 40
+    for j in tab:
+        lo = 2.0 ** octave * (1 + (j & 63) / 64)
+        w = 2.0 ** (octave - 6)
+        for q in (lo, np.nextafter(lo, 1e9), lo + w / 2, np.nextafter(lo + w, 0)):
+            got = fit.evaluate(tab, int.from_bytes(struct.pack("<d", float(q)), "little"))
+            f = fit.g_over_u3(mp.mpf(float(q)))
+            rel = float(abs(mp.mpf(got) - f) / f)
+            if octave < 2:
+                assert rel <= 2.0 ** -53 + 2.0 ** -54, (q, rel)
+            else:
+                assert rel * float(f * mp.mpf(float(q)) ** 1.5) <= 2.0 ** -54, (q, rel)
