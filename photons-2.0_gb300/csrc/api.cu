@@ -501,8 +501,8 @@ static int mutual_status(int over)
 #define MU_MIN_LEAF 48
 #endif
 // FP64 passes use mutual pairs at every leaf size: the FP64 pipe bounds the
-// pass, and evaluating each symmetric pair once takes 13 FP64 instructions a
-// pair where both ways take 20, whatever the pairing costs.
+// pass, and evaluating each symmetric pair once takes 9 FP64 instructions a
+// pair where both ways take 12, whatever the pairing costs.
 static bool uses_mutual(const photons_ctx *c, int precision)
 {
     if (c->mu_off || (c->pass_flags & PHOTONS_F_ONE_WAY)) return false;

@@ -1511,7 +1511,7 @@ __global__ void __launch_bounds__(256, 3) k_mu_gather(P2PArgs A, const int *slot
 // ---------------------------------------------------------------------
 // FP64 P2P with mutual pairs: the pairing of the FP32 kernel (each
 // symmetric leaf pair, local or image, evaluated once by its owner) with
-// the FP64 pass's pair factor (pair64.cuh: 13 FP64 instructions a pair).
+// the FP64 pass's pair factor (pair64.cuh: 9 FP64 instructions a pair).
 // What bounds it is the FP64 pipe; everything else is spent freely.
 //
 // A warp takes one work item: up to seg evaluated entries of one target
@@ -1531,7 +1531,8 @@ __global__ void __launch_bounds__(256, 3) k_mu_gather(P2PArgs A, const int *slot
 //
 // Whole pass, against one leaf per warp (the list unsplit, lists above 1024
 // entries one way) and 33 FP64 instructions a pair: 96^3 Zel'dovich leaf 64
-// 159.1 -> 57.6 ms, 110,591 particles half in halos, leaf 16, 150.0 -> 39.3.
+// 160.1 -> 41.9 ms (57.6 with 13 instructions), 110,591 particles half in
+// halos, leaf 16, 138.9 -> 32.1.
 // ---------------------------------------------------------------------
 #define MU64_TB 512
 #define MU64_WARPS (MU64_TB / 32)

@@ -6,13 +6,13 @@
 //
 // GB300's FP64 pipe runs at 1/64 of the FP32 rate: one FP64 instruction
 // costs a warp scheduler about 64 issue slots, more than a whole 64-bit
-// fixed-point polynomial on the integer pipe.  So f is evaluated in
-// integers from q's bits (tables of fit_pair_fp64.py: 1280 intervals of
+// fixed-point polynomial on the integer pipe.  So q is formed and f
+// evaluated in integers (tables of fit_pair_fp64.py: 1280 intervals of
 // degree 7, the largest error of the rounded double 1.5e-16 relative for
-// q < 4 and 2.2e-17 of the Newtonian factor beyond), and a pair costs 13
-// FP64 instructions: 3 differences, 3 for r^2, one for q, 3 sums, and 3
-// reaction sums where both particles are wanted.  With 1/r from rsqrt and g
-// by Horner's rule in FP64 it was 33.
+// q < 4 and 2.2e-17 of the Newtonian factor beyond), and a pair costs 9 FP64
+// instructions: 3 differences, 3 sums, and 3 reaction sums where both
+// particles are wanted.  With 1/r from rsqrt and g by Horner's rule in FP64
+// it was 33; with only f in integers, 13.
 #pragma once
 
 #include <cmath>
@@ -77,24 +77,34 @@ __device__ __forceinline__ Pair64Tab pair64_load(unsigned char *smem)
     return Pair64Tab{p01, p23, t, e};
 }
 
-// interval of q's high word; outside [2^-14, 2^6) (and for negative q,
-// infinities and NaN) not below PAIR64_NI
-__device__ __forceinline__ unsigned pair64_index(int qhi)
+// the high 64 bits of a product, up to a few units in the last place
+__device__ __forceinline__ unsigned long long mulhi64_near(unsigned long long a, unsigned long long b)
 {
-    return ((unsigned)qhi >> (20 - PAIR64_MB)) - ((1023 + PAIR64_LO) << PAIR64_MB);
+    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
+    return (unsigned long long)ah * bh + __umulhi(ah, bl) + __umulhi(al, bh);
+}
+
+// |v| with 62 fraction bits below 2^(e + 1), e the biased exponent of the
+// largest component (v below 2^-1022 counts as 0, bits below 2^(e - 61) are
+// cut off)
+__device__ __forceinline__ unsigned long long pair64_fixed(double v, int e)
+{
+    const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu, lo = (unsigned)__double2loint(v);
+    const int ev = (int)(hi >> 20);
+    const unsigned h = ev ? (hi & 0xfffffu) | 0x100000u : 0u;
+    const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, h, 10) << 32) | (lo << 10);
+    return m >> min(e - ev, 63);
 }
 
 // f(q) on interval i, in integers: 32-bit Horner for P[7..4], 64-bit for
-// P[3..0], then the double's bits (rounded to nearest)
-__device__ __forceinline__ double pair64_poly(unsigned i, double q, const Pair64Tab &tab)
+// P[3..0], then the double's bits (rounded to nearest).  d: the position in
+// the interval, in [-1/2, 1/2) with 64 fraction bits.
+__device__ __forceinline__ double pair64_poly(unsigned i, long long d, const Pair64Tab &tab)
 {
-    const unsigned hi = (unsigned)__double2hiint(q), lo = (unsigned)__double2loint(q);
     const int4 t = tab.t[i];
     const longlong2 p01 = tab.p01[i], p23 = tab.p23[i];
     const int es = tab.e[i];
-    // the mantissa bits below the interval's, as d in [-1/2, 1/2) with 64 fraction bits
-    const int dh = (int)(__funnelshift_l(lo, hi, 12 + PAIR64_MB) ^ 0x80000000u);
-    const long long d = (long long)(((unsigned long long)(unsigned)dh << 32) | (lo << (12 + PAIR64_MB)));
+    const int dh = (int)(d >> 32);
     int v = t.w;
     v = t.z + __mulhi(v, dh);
     v = t.y + __mulhi(v, dh);
@@ -112,31 +122,33 @@ __device__ __forceinline__ double pair64_poly(unsigned i, double q, const Pair64
 // f where the tables do not reach (r < eps, q outside their range): 1/r
 // from rsqrt and g from its own polynomials; two coincident particles get
 // the softened factor.  Rare: not inlined.
-__device__ __noinline__ double pair64_slow(double r2, double eps, double rs)
+__device__ __noinline__ double pair64_slow(double dx, double dy, double dz, double eps, double rs)
 {
     const double hrs = 0.5 / rs, cube = 8.0 * rs * rs * rs;
+    const double r2 = dx * dx + dy * dy + dz * dz;
     const double rinv = r2 > 0.0 ? rsqrt(r2) : 0.0;
     const double dr = r2 * rinv;
     const double w = dr < eps ? 1.0 / (eps * eps * eps) : rinv * rinv * rinv;
     return w * split_g_fp64(dr * hrs, &g_split64[0][0], 2.0 / sqrt(M_PI)) * cube;
 }
 
-// Per-box constants: f's argument is r^2 ia2, the tables serve r^2 >= eps^2
-// (compared as bit patterns: r^2 is not negative), and sums of f dx are
-// multiplied by scale
+// Per-box constants: q = r^2 ia2 with ia2 = k 2^(ke - 63), k in [2^63, 2^64);
+// the tables serve high words of q above qeps (that of eps^2 ia2)
 struct Pair64 {
-    double ia2, eps, rs;
-    long long eps2_bits;
+    unsigned long long k;
+    int ke, qeps;
+    double eps, rs;
 };
 
 __device__ __forceinline__ Pair64 pair64_consts(double eps, double rs)
 {
     Pair64 c;
-    const double ia = 0.5 / rs;
-    c.ia2 = ia * ia;
+    const double ia = 0.5 / rs, ia2 = ia * ia;
+    c.k = (1ull << 63) | ((unsigned long long)__double_as_longlong(ia2) << 11);
+    c.ke = (__double2hiint(ia2) >> 20) - 1023;
+    c.qeps = __double2hiint(eps * eps * ia2);
     c.eps = eps;
     c.rs = rs;
-    c.eps2_bits = __double_as_longlong(eps * eps);
     return c;
 }
 
@@ -146,16 +158,28 @@ __device__ __forceinline__ double pair64_scale(double mass, double rs)
     return mass * (ia * ia * ia);
 }
 
-// f for a source dx away; 0 where !on
+// f for a source dx away; 0 where !on.  q = r^2 ia2 in fixed point too (the
+// squares of the components aligned to the largest, good to 2^-58), which
+// takes r^2's three FP64 instructions and the product off the FP64 pipe.
 __device__ __forceinline__ double pair64_f(double dx, double dy, double dz, bool on, const Pair64 &c,
                                            const Pair64Tab &tab)
 {
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double q = r2 * c.ia2;
-    const unsigned i = pair64_index(__double2hiint(q));
-    const bool fast = i < PAIR64_NI && __double_as_longlong(r2) >= c.eps2_bits;
-    double f = pair64_poly(fast ? i : 0u, q, tab);
-    if (on && !fast) f = pair64_slow(r2, c.eps, c.rs);
+    const unsigned hx = (unsigned)__double2hiint(dx) & 0x7fffffffu, hy = (unsigned)__double2hiint(dy) & 0x7fffffffu,
+                   hz = (unsigned)__double2hiint(dz) & 0x7fffffffu;
+    const int e = (int)(max(hx, max(hy, hz)) >> 20);
+    const unsigned long long x = pair64_fixed(dx, e), y = pair64_fixed(dy, e), z = pair64_fixed(dz, e);
+    unsigned long long s = mulhi64_near(x, x) + mulhi64_near(y, y) + mulhi64_near(z, z);  // < 3 2^62
+    const int ls = __clzll((long long)s);
+    s = mulhi64_near(s << ls, c.k);
+    const int l2 = (long long)s < 0 ? 0 : 1;
+    s <<= l2;  // q's mantissa, leading one at bit 63 (s = 0 only for r = 0)
+    // r^2 = s 2^(2 (e - 1023) - 60) before the shifts
+    const int eq = 2 * (e - 1023) + 4 - ls - l2 + c.ke;
+    const int qhi = ((eq + 1022) << 20) + (int)(s >> 43);
+    const unsigned i = ((unsigned)(eq - PAIR64_LO) << PAIR64_MB) + ((unsigned)(s >> (63 - PAIR64_MB)) & ((1u << PAIR64_MB) - 1u));
+    const bool fast = i < PAIR64_NI && qhi > c.qeps;
+    double f = pair64_poly(fast ? i : 0u, (long long)((s << (PAIR64_MB + 1)) ^ (1ull << 63)), tab);
+    if (on && !fast) f = pair64_slow(dx, dy, dz, c.eps, c.rs);
     return on ? f : 0.0;
 }
 
