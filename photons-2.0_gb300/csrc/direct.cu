@@ -7,63 +7,143 @@
 //  * photons_fp32_fma_peak: FFMA throughput probe, the denominator of the
 //    P2P roofline fraction; photons_fp64_fma_peak: the DFMA one, for the
 //    FP64 drop-in pass.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "api_internal.cuh"
+#include "pair64.cuh"
 
 namespace {
 
-__global__ void k_direct(const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
-                         const int *__restrict__ cell_start, int ncell, double cellw, const double *__restrict__ tx,
-                         const double *__restrict__ ty, const double *__restrict__ tz, const int *__restrict__ tself,
-                         int nt, double L, double rmax2, double eps, double mass, double rs, double *out)
+// FP32 copies of the binned sources, for the distance filter below
+__global__ void k_direct_f32(const double *__restrict__ sx, const double *__restrict__ sy,
+                             const double *__restrict__ sz, int n, float4 *__restrict__ s4)
 {
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    const double coeff = 2.0 / sqrt(M_PI);
-    const double soft3 = mass / (eps * eps * eps);
-    for (int t = gw; t < nt; t += nw) {
-        double px = tx[t], py = ty[t], pz = tz[t];
-        int self = tself[t];
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        s4[j] = make_float4((float)sx[j], (float)sy[j], (float)sz[j], 0.f);
+}
+
+// Minimum image of a coordinate difference: |d| > L/2 (compared as bit
+// patterns, on the integer pipe) takes one side off
+__device__ __forceinline__ double nearest_image(double d, double L, long long half_bits)
+{
+    const long long b = __double_as_longlong(d);
+    if ((b & 0x7fffffffffffffffLL) > half_bits) d = b < 0 ? d + L : d - L;
+    return d;
+}
+
+// One block per target.  What bounds the sum is the FP64 pipe (1/64 of the
+// FP32 rate on GB300), and most candidates of the 27 cells lie beyond rmax:
+// a warp tests 32 candidates in FP32, with a margin above the FP32 error,
+// and queues those that may be within rmax; full batches of 32 queued
+// sources get the exact FP64 distance, the rmax test and the pair force
+// (pair64.cuh), so no FP64 lane idles.  A candidate then costs the FP64 pipe
+// nothing and a source within rmax 12 instructions (15 and ~130 with the
+// whole test and erfc, exp, sqrt and division in FP64), and a target in a
+// halo, with ten times the sources of the others, is spread over 8 warps.
+// 262,144 particles half in halos, 2,000 targets, rmax 2 rcut: the call 39.4
+// ms with a warp per target (the kernel 34.3), 4.6 now.  Warps take the candidates in a fixed order, so sums
+// are deterministic.
+#define DIRECT_TB 256
+#define DIRECT_WARPS (DIRECT_TB / 32)
+
+__global__ void __launch_bounds__(DIRECT_TB) k_direct(const double *__restrict__ sx, const double *__restrict__ sy,
+                                                      const double *__restrict__ sz, const float4 *__restrict__ s4,
+                                                      const int *__restrict__ cell_start, int ncell, double cellw,
+                                                      const double *__restrict__ tx, const double *__restrict__ ty,
+                                                      const double *__restrict__ tz, const int *__restrict__ tself,
+                                                      int nt, double L, double most, double rmax2, double eps,
+                                                      double mass, double rs, double *out)
+{
+    __shared__ int s_queue[DIRECT_WARPS][64];
+    __shared__ double s_sum[DIRECT_WARPS][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    int *queue = s_queue[warp];
+    const ph::Pair64Tab tab = ph::pair64_global();
+    const ph::Pair64 pc = ph::pair64_consts(eps, rs);
+    const long long half_bits = __double_as_longlong(0.5 * L), rmax2_bits = __double_as_longlong(rmax2);
+    const float Lf = (float)L, halff = 0.5f * Lf;
+    // with every coordinate and L at most `most`: an FP32 coordinate is within
+    // 2^-24 most of its double, a difference (at most 2 most) and its image
+    // shift round by 2^-23 most each, so 4 units of 2^-23 most bound a
+    // component's error and 8 the distance's; the square's rounding is 2^-21
+    // of itself
+    const float reach = (float)sqrt(rmax2) * 1.000001f + 8.f * 1.1920929e-7f * (float)most;
+    const float limit = reach * reach * 1.000001f;
+    const int span = ncell >= 3 ? 1 : 0;
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const double px = tx[t], py = ty[t], pz = tz[t];
+        const float fx = (float)px, fy = (float)py, fz = (float)pz;
+        const int self = tself[t];
         int ci[3] = {(int)(px / cellw), (int)(py / cellw), (int)(pz / cellw)};
         for (int d = 0; d < 3; d++) ci[d] = min(max(ci[d], 0), ncell - 1);
         double ax = 0, ay = 0, az = 0;
-        int span = ncell >= 3 ? 1 : 0;
-        for (int ox = -span; ox <= span; ox++)
-            for (int oy = -span; oy <= span; oy++)
-                for (int oz = -span; oz <= span; oz++) {
-                    int cx = (ci[0] + ox + ncell) % ncell, cy = (ci[1] + oy + ncell) % ncell,
-                        cz = (ci[2] + oz + ncell) % ncell;
-                    int c = ncell >= 3 ? (cx * ncell + cy) * ncell + cz : 0;
-                    int b = ncell >= 3 ? cell_start[c] : 0;
-                    int e = ncell >= 3 ? cell_start[c + 1] : cell_start[ncell * ncell * ncell];
-                    for (int j = b + lane; j < e; j += 32) {
-                        if (j == self) continue;
-                        double dx = sx[j] - px, dy = sy[j] - py, dz = sz[j] - pz;
-                        if (dx > 0.5 * L) dx -= L; else if (dx < -0.5 * L) dx += L;
-                        if (dy > 0.5 * L) dy -= L; else if (dy < -0.5 * L) dy += L;
-                        if (dz > 0.5 * L) dz -= L; else if (dz < -0.5 * L) dz += L;
-                        double r2 = dx * dx + dy * dy + dz * dz;
-                        if (r2 >= rmax2) continue;
-                        double dr = sqrt(r2);
-                        double ir3 = dr < eps ? soft3 : mass / (dr * dr * dr);
-                        double u = 0.5 * dr / rs;
-                        ir3 *= erfc(u) + coeff * u * exp(-u * u);
-                        ax += dx * ir3;
-                        ay += dy * ir3;
-                        az += dz * ir3;
-                    }
+        int waiting = 0;
+        auto evaluate = [&](int count) {
+            const bool on = lane < count;
+            const int j = queue[on ? lane : 0];
+            const double dx = nearest_image(sx[j] - px, L, half_bits), dy = nearest_image(sy[j] - py, L, half_bits),
+                         dz = nearest_image(sz[j] - pz, L, half_bits);
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            // !(r2 >= rmax2) on bit patterns: a NaN stays in
+            const long long rb = __double_as_longlong(r2);
+            const bool near = on && (rb < rmax2_bits || rb > 0x7ff0000000000000LL);
+            double f = ph::pair64_f(dx, dy, dz, near, pc, tab);
+            if (near && rb == 0 && eps == 0.0) f = INFINITY;  // coincident and unsoftened: m / r^3
+            ax = fma(dx, f, ax);
+            ay = fma(dy, f, ay);
+            az = fma(dz, f, az);
+        };
+        for (int o = 0; o < (span ? 27 : 1); o++) {
+            int c = 0;
+            if (span) {
+                const int cx = (ci[0] + o / 9 - 1 + ncell) % ncell, cy = (ci[1] + o / 3 % 3 - 1 + ncell) % ncell,
+                          cz = (ci[2] + o % 3 - 1 + ncell) % ncell;
+                c = (cx * ncell + cy) * ncell + cz;
+            }
+            const int b = span ? cell_start[c] : 0;
+            const int e = span ? cell_start[c + 1] : cell_start[ncell * ncell * ncell];
+            for (int j0 = b + 32 * warp; j0 < e; j0 += DIRECT_TB) {
+                const int j = j0 + lane;
+                bool in = j < e && j != self;
+                if (in) {
+                    const float4 s = s4[j];
+                    float dx = fabsf(s.x - fx), dy = fabsf(s.y - fy), dz = fabsf(s.z - fz);
+                    if (dx > halff) dx = fabsf(dx - Lf);
+                    if (dy > halff) dy = fabsf(dy - Lf);
+                    if (dz > halff) dz = fabsf(dz - Lf);
+                    in = !(dx * dx + dy * dy + dz * dz > limit);  // (a NaN goes on to the exact test)
                 }
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (in) queue[waiting + __popc(m & lt)] = j;
+                waiting += __popc(m);
+                __syncwarp();
+                if (waiting >= 32) {
+                    evaluate(32);
+                    __syncwarp();
+                    const int rest = waiting - 32, moved = lane < rest ? queue[32 + lane] : 0;
+                    __syncwarp();
+                    if (lane < rest) queue[lane] = moved;
+                    waiting = rest;
+                    __syncwarp();
+                }
+            }
+        }
+        if (waiting) evaluate(waiting);
         ax = warp_sum_d(ax);
         ay = warp_sum_d(ay);
         az = warp_sum_d(az);
-        if (lane == 0) {
-            out[3 * t] = ax;
-            out[3 * t + 1] = ay;
-            out[3 * t + 2] = az;
+        if (lane == 0) { s_sum[warp][0] = ax; s_sum[warp][1] = ay; s_sum[warp][2] = az; }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double v = 0.0;
+            for (int w = 0; w < DIRECT_WARPS; w++) v += s_sum[w][threadIdx.x];
+            out[3 * (size_t)t + threadIdx.x] = v * ph::pair64_scale(mass, rs);
         }
+        __syncthreads();
     }
 }
 
@@ -134,9 +214,11 @@ extern "C" int photons_direct_sum(const photons_params *p, int n, const double *
     const double cw = L / ncell;
     const size_t nc3 = (size_t)ncell * ncell * ncell;
     std::vector<int> cnt(nc3 + 1, 0), cellof(n);
+    double most = L;  // largest coordinate, for the distance filter's margin
     for (int j = 0; j < n; j++) {
         int c[3];
         for (int d = 0; d < 3; d++) {
+            most = std::max(most, std::fabs(pos[3 * (size_t)j + d]));
             c[d] = (int)(pos[3 * (size_t)j + d] / cw);
             if (c[d] < 0) c[d] = 0;
             if (c[d] >= ncell) c[d] = ncell - 1;
@@ -166,6 +248,7 @@ extern "C" int photons_direct_sum(const photons_params *p, int n, const double *
     }
     double *d_sx = nullptr, *d_sy = nullptr, *d_sz = nullptr, *d_tx = nullptr, *d_ty = nullptr, *d_tz = nullptr,
            *d_out = nullptr;
+    float4 *d_s4 = nullptr;
     int *d_cell = nullptr, *d_ts = nullptr;
     int rc = 0;
     auto al = [&](void **ptr, size_t bytes) {
@@ -178,7 +261,7 @@ extern "C" int photons_direct_sum(const photons_params *p, int n, const double *
     al((void **)&d_sx, sizeof(double) * n); al((void **)&d_sy, sizeof(double) * n); al((void **)&d_sz, sizeof(double) * n);
     al((void **)&d_tx, sizeof(double) * nt); al((void **)&d_ty, sizeof(double) * nt); al((void **)&d_tz, sizeof(double) * nt);
     al((void **)&d_out, sizeof(double) * 3 * nt); al((void **)&d_cell, sizeof(int) * (nc3 + 1));
-    al((void **)&d_ts, sizeof(int) * nt);
+    al((void **)&d_ts, sizeof(int) * nt); al((void **)&d_s4, sizeof(float4) * n);
     if (!rc) {
         cudaMemcpy(d_sx, sx.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
         cudaMemcpy(d_sy, sy.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
@@ -188,15 +271,16 @@ extern "C" int photons_direct_sum(const photons_params *p, int n, const double *
         cudaMemcpy(d_tz, tz.data(), sizeof(double) * nt, cudaMemcpyHostToDevice);
         cudaMemcpy(d_ts, ts.data(), sizeof(int) * nt, cudaMemcpyHostToDevice);
         cudaMemcpy(d_cell, cnt.data(), sizeof(int) * (nc3 + 1), cudaMemcpyHostToDevice);
-        int blocks = ph::device_sm_count() * 8;
-        ph::note_launch(), k_direct<<<blocks, 256>>>(d_sx, d_sy, d_sz, d_cell, ncell, cw, d_tx, d_ty, d_tz, d_ts, nt, L, rmax * rmax,
+        const int blocks = ph::device_sm_count() * 8;
+        ph::note_launch(), k_direct_f32<<<blocks, 256>>>(d_sx, d_sy, d_sz, n, d_s4);
+        ph::note_launch(), k_direct<<<nt, DIRECT_TB>>>(d_sx, d_sy, d_sz, d_s4, d_cell, ncell, cw, d_tx, d_ty, d_tz, d_ts, nt, L, most, rmax * rmax,
                                   p->eps, p->mass, p->rs, d_out);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpy(acc, d_out, sizeof(double) * 3 * nt, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = ph_set_cuda_error(e, "direct sum", __FILE__, __LINE__);
     }
     cudaFree(d_sx); cudaFree(d_sy); cudaFree(d_sz); cudaFree(d_tx); cudaFree(d_ty); cudaFree(d_tz);
-    cudaFree(d_out); cudaFree(d_cell); cudaFree(d_ts);
+    cudaFree(d_out); cudaFree(d_cell); cudaFree(d_ts); cudaFree(d_s4);
     return rc;
 }
 
