@@ -61,6 +61,10 @@ __device__ __forceinline__ void scaled_monomials(double dx, double dy, double dz
 }
 
 // ---------------- P2M ----------------
+// A thread per leaf.  The FP64 pipe bounds it: sums of the bare monomials
+// (28 FP64 instructions a particle), scaled by the mass and 1 / a! at the
+// end (summing the scaled monomials took ~80: 250,047 particles, 14.5k
+// leaves, 87 -> 51 us).
 __global__ void k_p2m(const double *px, const double *py, const double *pz, const int *ipart, const int *npart,
                       const double *cx, const double *cy, const double *cz, const int *tree_cnt, const int *boxid,
                       const BoxParams *boxes, double *M, const int *gate)
@@ -74,14 +78,28 @@ __global__ void k_p2m(const double *px, const double *py, const double *pz, cons
         double c0 = cx[l], c1 = cy[l], c2 = cz[l];
         int ip = ipart[l], np = npart[l];
         const double mass = boxes[boxid[l]].mass;
+#pragma unroll 2
         for (int p = ip; p < ip + np; p++) {
-            double mono[PH_NMULTI];
-            scaled_monomials(-(px[p] - c0), -(py[p] - c1), -(pz[p] - c2), mono);
+            const double x[3] = {c0 - px[p], c1 - py[p], c2 - pz[p]};
+            double xx[3][3];
 #pragma unroll
-            for (int i = 0; i < PH_NMULTI; i++) acc[i] += mass * mono[i];
+            for (int d = 0; d < 3; d++)
+#pragma unroll
+                for (int q = d; q < 3; q++) xx[d][q] = x[d] * x[q];
+#pragma unroll
+            for (int i = 1; i < PH_NMULTI; i++) {
+                // the axes of component i in ascending order
+                const int e0 = h_mi.e[i][0], e1 = h_mi.e[i][1];
+                const int d0 = e0 > 0 ? 0 : (e1 > 0 ? 1 : 2), d1 = e0 > 1 ? 0 : (e0 + e1 > 1 ? 1 : 2),
+                          d2 = e0 > 2 ? 0 : (e0 + e1 > 2 ? 1 : 2);
+                if (h_mi.ord[i] == 1) acc[i] += x[d0];
+                else if (h_mi.ord[i] == 2) acc[i] += xx[d0][d1];
+                else acc[i] = fma(xx[d0][d1], x[d2], acc[i]);
+            }
         }
+        acc[0] = (double)np;
 #pragma unroll
-        for (int i = 0; i < PH_NMULTI; i++) M[(size_t)l * PH_NMULTI + i] = acc[i];
+        for (int i = 0; i < PH_NMULTI; i++) M[(size_t)l * PH_NMULTI + i] = acc[i] * mass * h_mi.invf[i];
     }
 }
 
@@ -104,12 +122,133 @@ __device__ __forceinline__ void m2m_add(double dx, double dy, double dz, const d
     }
 }
 
+// The M2M and L2L of a depth take one of two forms, by its width: a thread
+// per target (the fewest FP64 instructions: ~125 a warp of 32 translations
+// against 16 a translation, but 250 in a row in each thread), or a warp per
+// target, for depths that leave most of the chip idle anyway: lane i (< 20)
+// holds component i, and a target is done after ~32 instructions.  The two
+// cross near 5,000 targets (an FP64 instruction of a warp takes a scheduler
+// ~64 cycles).  Per launch at 250,047 halo particles (23 depths), threads
+// alone -> both forms: M2M 14.3 -> 8.2 us, L2L 10.0 -> 8.2; at 2,097,152 (26
+// depths) 11.3 and 11.2.
+#define WIDE_DEPTH 5000
+
+// Per lane, packed a byte each: the terms of its component.  M2M: M_b
+// mono_(a-b), b <= a (at most 8); L2L: L_(b+g) mono_g (10; lane 20 has the
+// second half of component 0's).  Index 20 is a zero term.
+struct OpTerms {
+    alignas(16) unsigned char m2m_b[PH_NMULTI + 1][8];
+    alignas(16) unsigned char m2m_g[PH_NMULTI + 1][8];
+    alignas(16) unsigned char l2l_l[PH_NMULTI + 1][16];
+    alignas(16) unsigned char l2l_g[PH_NMULTI + 1][16];
+};
+
+constexpr OpTerms make_op_terms()
+{
+    constexpr MITab t = make_mitab();
+    OpTerms T{};
+    for (int a = 0; a <= PH_NMULTI; a++) {
+        int n = 0;
+        for (int b = 0; b < PH_NMULTI && a < PH_NMULTI; b++) {
+            const int g0 = t.e[a][0] - t.e[b][0], g1 = t.e[a][1] - t.e[b][1], g2 = t.e[a][2] - t.e[b][2];
+            if (g0 < 0 || g1 < 0 || g2 < 0) continue;
+            T.m2m_b[a][n] = (unsigned char)b;
+            T.m2m_g[a][n++] = (unsigned char)t.idx[g0][g1][g2];
+        }
+        for (; n < 8; n++) { T.m2m_b[a][n] = PH_NMULTI; T.m2m_g[a][n] = 0; }
+        const int b = a < PH_NMULTI ? a : 0;
+        n = 0;
+        for (int g = a < PH_NMULTI ? 0 : 10; g < PH_NMULTI && n < 10; g++) {
+            if (t.ord[b] + t.ord[g] > 3) continue;
+            T.l2l_l[a][n] = (unsigned char)t.idx[t.e[b][0] + t.e[g][0]][t.e[b][1] + t.e[g][1]][t.e[b][2] + t.e[g][2]];
+            T.l2l_g[a][n++] = (unsigned char)g;
+        }
+        for (; n < 16; n++) { T.l2l_l[a][n] = PH_NMULTI; T.l2l_g[a][n] = 0; }
+    }
+    return T;
+}
+
+constexpr __device__ OpTerms c_terms = make_op_terms();
+
+// a warp's staging area; src[20] = 0 for the padding terms
+struct OpWarp {
+    double src[PH_NMULTI + 1], mono[PH_NMULTI];
+};
+
+__device__ __forceinline__ int term(const unsigned *w, int n) { return (w[n >> 2] >> (8 * (n & 3))) & 255; }
+
+// lane i's scaled monomial d^e(i) / e(i)!: its exponents' running sums, 1 / e(i)!
+struct LaneMono {
+    int e0, e1, e2;
+    double invf;
+};
+
+__device__ __forceinline__ LaneMono lane_mono(int lane)
+{
+    const int i = lane < PH_NMULTI ? lane : 0;
+    const int e0 = h_mi.e[i][0], e1 = e0 + h_mi.e[i][1];
+    return LaneMono{e0, e1, e1 + h_mi.e[i][2], h_mi.invf[i]};
+}
+
+__device__ __forceinline__ double lane_monomial(double dx, double dy, double dz, const LaneMono &q)
+{
+    const double f0 = q.e0 > 0 ? dx : (q.e1 > 0 ? dy : (q.e2 > 0 ? dz : 1.0)),
+                 f1 = q.e0 > 1 ? dx : (q.e1 > 1 ? dy : (q.e2 > 1 ? dz : 1.0)),
+                 f2 = q.e0 > 2 ? dx : (q.e1 > 2 ? dy : (q.e2 > 2 ? dz : 1.0));
+    return (f0 * f1) * (f2 * q.invf);
+}
+
+// v_a = sum_{b <= a} M_b mono_(a-b): lane a's component of a multipole (lane
+// b's component in `m`) moved by the displacement whose monomials are `mono`
+__device__ __forceinline__ double m2m_lanes(double m, double mono, OpWarp &w, const unsigned *tb, const unsigned *tg,
+                                            int lane)
+{
+    __syncwarp();
+    if (lane < PH_NMULTI) {
+        w.src[lane] = m;
+        w.mono[lane] = mono;
+    }
+    __syncwarp();
+    double v = 0.0, u = 0.0;
+#pragma unroll
+    for (int n = 0; n < 8; n += 2) {
+        v = fma(w.src[term(tb, n)], w.mono[term(tg, n)], v);
+        u = fma(w.src[term(tb, n + 1)], w.mono[term(tg, n + 1)], u);
+    }
+    return v + u;
+}
+
 __global__ void k_m2m_depth(const int *list, const int *depth_off, int d, const int *tree_cnt, const int *son0,
                             const int *son1, const double *cx, const double *cy, const double *cz, double *M,
                             const int *gate)
 {
     if (gate && !*gate) return;
     const int begin = depth_off[d], end = depth_off[d + 1], nleaf = tree_cnt[BC_LEAVES];
+    if (begin == end) return;
+    if (end - begin <= WIDE_DEPTH) {
+        __shared__ OpWarp s_w[MP_TB / 32];
+        const int lane = threadIdx.x & 31, mine = lane < PH_NMULTI ? lane : 0;
+        const uint2 b2 = *reinterpret_cast<const uint2 *>(c_terms.m2m_b[mine]),
+                    g2 = *reinterpret_cast<const uint2 *>(c_terms.m2m_g[mine]);
+        const unsigned tb[2] = {b2.x, b2.y}, tg[2] = {g2.x, g2.y};
+        OpWarp &w = s_w[threadIdx.x >> 5];
+        if (lane == 0) w.src[PH_NMULTI] = 0.0;
+        const LaneMono lm = lane_mono(lane);
+        const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+        for (int i = begin + gw; i < end; i += nw) {
+            const int u = list[i];
+            if (u < nleaf) continue;
+            const int l0 = son0[u], l1 = son1[u];
+            const double c0 = cx[u], c1 = cy[u], c2 = cz[u];
+            const double ma = M[(size_t)l0 * PH_NMULTI + mine], mb = M[(size_t)l1 * PH_NMULTI + mine];
+            const double ga = lane_monomial(c0 - cx[l0], c1 - cy[l0], c2 - cz[l0], lm),
+                         gb = lane_monomial(c0 - cx[l1], c1 - cy[l1], c2 - cz[l1], lm);
+            const double va = m2m_lanes(ma, ga, w, tb, tg, lane);
+            const double out = va + m2m_lanes(mb, gb, w, tb, tg, lane);
+            if (lane < PH_NMULTI) M[(size_t)u * PH_NMULTI + lane] = out;
+        }
+        return;
+    }
     for (int i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
         int u = list[i];
         if (u < nleaf) continue;
@@ -246,6 +385,41 @@ __global__ void k_l2l_depth(const int *list, const int *depth_off, int d, const 
 {
     if (gate && !*gate) return;
     const int begin = depth_off[d], end = depth_off[d + 1];
+    if (begin == end) return;
+    if (end - begin <= WIDE_DEPTH) {
+        __shared__ OpWarp s_w[MP_TB / 32];
+        const int lane = threadIdx.x & 31, row = lane <= PH_NMULTI ? lane : 0;
+        const uint4 l4 = *reinterpret_cast<const uint4 *>(c_terms.l2l_l[row]),
+                    g4 = *reinterpret_cast<const uint4 *>(c_terms.l2l_g[row]);
+        const unsigned tl[3] = {l4.x, l4.y, l4.z}, tg[3] = {g4.x, g4.y, g4.z};
+        OpWarp &w = s_w[threadIdx.x >> 5];
+        if (lane == 0) w.src[PH_NMULTI] = 0.0;
+        const LaneMono lm = lane_mono(lane);
+        const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+        for (int i = begin + gw; i < end; i += nw) {
+            const int u = list[i], p = parent[u];
+            if (p < 0) continue;
+            const double mono = lane_monomial(cx[u] - cx[p], cy[u] - cy[p], cz[u] - cz[p], lm);
+            const double own = lane < PH_NMULTI ? L[(size_t)u * PH_NMULTI + lane] : 0.0;
+            __syncwarp();
+            if (lane < PH_NMULTI) {
+                w.src[lane] = L[(size_t)p * PH_NMULTI + lane];
+                w.mono[lane] = mono;
+            }
+            __syncwarp();
+            double v = 0.0, q = 0.0;
+#pragma unroll
+            for (int n = 0; n < 10; n += 2) {
+                v = fma(w.src[term(tl, n)], w.mono[term(tg, n)], v);
+                q = fma(w.src[term(tl, n + 1)], w.mono[term(tg, n + 1)], q);
+            }
+            v += q;
+            const double second = __shfl_sync(0xffffffffu, v, PH_NMULTI);  // the second half of component 0
+            if (lane == 0) v += second;
+            if (lane < PH_NMULTI) L[(size_t)u * PH_NMULTI + lane] = own + v;
+        }
+        return;
+    }
     for (int i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
         int u = list[i];
         int p = parent[u];
@@ -526,7 +700,7 @@ int run_m2l(const MultipoleArgs &a, cudaStream_t st)
 static void launch_l2l(const MultipoleArgs &a, cudaStream_t st)
 {
     for (int d = 1; d < a.ndepth; d++)
-        ph::note_launch(), k_l2l_depth<<<grid_cap(), MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.parent, a.cx, a.cy,
+        ph::note_launch(), k_l2l_depth<<<device_sm_count() * 8, MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.parent, a.cx, a.cy,
                                                                        a.cz, a.L, a.gate_l);
 }
 
@@ -567,7 +741,7 @@ int run_p2m_m2m(const MultipoleArgs &a, cudaStream_t st)
     ph::note_launch(), k_p2m<<<grid_cap(), MP_TB, 0, st>>>(a.px, a.py, a.pz, a.ipart, a.npart, a.cx, a.cy, a.cz,
                                                              a.tree_cnt, a.boxid, a.boxes, a.M, a.gate_m);
     for (int d = a.ndepth - 1; d >= 0; d--)
-        ph::note_launch(), k_m2m_depth<<<grid_cap(), MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.tree_cnt, a.son0,
+        ph::note_launch(), k_m2m_depth<<<device_sm_count() * 8, MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.tree_cnt, a.son0,
                                                                        a.son1, a.cx, a.cy, a.cz, a.M, a.gate_m);
     ph::note_launch(), k_zero_L<<<grid_cap(), 256, 0, st>>>(a.L, a.tree_cnt, a.gate_m);
     PH_CUDA_CHECK(cudaGetLastError());
