@@ -238,7 +238,7 @@ static int alloc_walk(photons_ctx *c, long long p2p_cap, long long pd_cap, long 
     ph::WalkBufs &w = c->w;
     if (!w.ctr) { PH_TRY(dalloc(w.ctr, ph::WC_N)); c->epoch++; }
     if (!c->far_gate) { PH_TRY(dalloc(c->far_gate, 2)); c->epoch++; }
-    if (!c->work_counter) { PH_TRY(dalloc(c->work_counter, 4)); c->epoch++; }
+    if (!c->work_counter) { PH_TRY(dalloc(c->work_counter, 8)); c->epoch++; }
     if (p2p_cap > w.p2p_cap) {
         w.p2p_cap = 0;
         c->epoch++;
@@ -957,6 +957,7 @@ int ph_stage_p2p(photons_ctx *c, int precision, int zero)
     a.boxid = c->t.boxid;
     a.boxes = c->b.boxes;
     a.nbox = c->b.nbox;
+    a.leaf_cap = c->b.rule_cap;
     a.p2p_pool = c->w.p2p_pool; a.p2p_off = c->w.p2p_off; a.p2p_cnt = c->w.p2p_cnt;
     a.pos4 = c->pos4;
     a.chi = c->t.chi;
@@ -964,6 +965,9 @@ int ph_stage_p2p(photons_ctx *c, int precision, int zero)
     a.px = c->b.x; a.py = c->b.y; a.pz = c->b.z;
     a.ax = c->ax; a.ay = c->ay; a.az = c->az;
     a.work_counter = c->work_counter;
+    a.ow_ctl = c->work_counter + 4;
+    a.ow_long = c->mu_sorted;  // (the mutual kernels' list flags: not in use with the packed kernel)
+    a.p2p_fill = c->w.ctr + ph::WC_P2P_FILL;
     a.boxsize = c->pp.boxsize; a.eps = c->pp.eps; a.mass = c->pp.mass; a.rs = c->pp.rs;
     a.k = ph::make_split_consts(c->pp);
     a.variant = p2p_variant();

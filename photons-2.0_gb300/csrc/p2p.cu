@@ -237,8 +237,10 @@ __global__ void __launch_bounds__(P2P_TB) k_p2p_split(P2PArgs A)
 //   where the subtraction is exact; then (hi_s - hi_t) + (lo_s - lo_t) is
 //   exact up to the final rounding.
 // * Staging: one lane per staged source (coalesced loads, conflict-free
-//   shared stores); the lane finds its list entry by a binary search over
-//   the 32 entries' prefix counts held in the warp.
+//   shared stores); the lane finds its list entry by counting the entries
+//   that start at or before it in a bit mask of 32 sources (a warp-wide OR).
+// * Long lists (k_ow_long) are shared by a block's warps, a contiguous part
+//   each; the others go a leaf to a warp.
 // * Lanes: a block of up to 64 targets is taken in at most two rounds of
 //   m = 32, 16, ..., 1 targets with 32/m source streams each; both rounds
 //   run over every staged batch, accumulating in registers.
@@ -411,12 +413,127 @@ __device__ __forceinline__ float centre_diff(float hs, float ls, float ht, float
     return (hs - ht) + (ls - lt);
 }
 
+// one batch of a list's entries staged relative to the target centre
+// (scaled): the entries taken (lane i owns entry i), the sources staged
+__device__ __forceinline__ int ow_stage(const P2PArgs &A, const uint32_t *list, int left, const float4 &cth,
+                                        const float4 &ctl, float sig, float Lhi, float Llo, float *sx, float *sy,
+                                        float *sz, float4 *meta, int lane, int &nstaged)
+{
+    const int ne = min(32, left);
+    int is = 0, ns = 0;
+    float d0 = 0.f, d1 = 0.f, d2 = 0.f;
+    if (lane < ne) {
+        const uint32_t en = list[lane];
+        const int s = PH_ENTRY_ID(en), img = PH_ENTRY_IMG(en);
+        is = A.ipart[s];
+        ns = A.npart[s];
+        const float4 csh = A.chi[s], csl = A.clo[s];
+        int mi, mj, mk;
+        image_offsets(img, mi, mj, mk);
+        d0 = centre_diff(csh.x, csl.x, cth.x, ctl.x, mi, Lhi, Llo) * sig;
+        d1 = centre_diff(csh.y, csl.y, cth.y, ctl.y, mj, Lhi, Llo) * sig;
+        d2 = centre_diff(csh.z, csl.z, cth.z, ctl.z, mk, Lhi, Llo) * sig;
+    }
+    const int incl = warp_incl_scan(ns), pre = incl - ns;
+    const int nfit = __popc(__ballot_sync(0xffffffffu, lane < ne && incl <= STAGE2));
+    nstaged = 0;
+    if (nfit == 0) return 0;  // unreachable under the MAXLEAF bound; the caller stops
+    nstaged = __shfl_sync(0xffffffffu, incl, nfit - 1);
+    // per non-empty entry: centre difference, first particle - first staged source
+    const bool some = lane < nfit && ns > 0;
+    const unsigned upto = (2u << lane) - 1u;
+    const unsigned nz = __ballot_sync(0xffffffffu, some);
+    if (some) meta[__popc(nz & upto) - 1] = make_float4(d0, d1, d2, __int_as_float(is - pre));
+    __syncwarp();
+    int first = -1;  // the entry that holds source s0 - 1
+    for (int s0 = 0; s0 < nstaged; s0 += 64) {
+        float4 o[2], m[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            // bit i: an entry starts at source s0 + 32 k + i
+            const unsigned at = (unsigned)(pre - (s0 + 32 * k));
+            const unsigned starts = __reduce_or_sync(0xffffffffu, some && at < 32u ? 1u << at : 0u);
+            const int idx = min(s0 + 32 * k + lane, nstaged - 1);
+            m[k] = meta[first + __popc(starts & upto)];
+            o[k] = __ldg(A.pos4 + __float_as_int(m[k].w) + idx);
+            first += __popc(starts);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int idx = s0 + 32 * k + lane;
+            if (idx < nstaged) {
+                sx[idx] = fmaf(o[k].x, sig, m[k].x);
+                sy[idx] = fmaf(o[k].y, sig, m[k].y);
+                sz[idx] = fmaf(o[k].z, sig, m[k].z);
+            }
+        }
+    }
+    // an odd count gets one far-away source whose force is exactly 0
+    if (lane == 0 && (nstaged & 1)) sx[nstaged] = sy[nstaged] = sz[nstaged] = 1e18f;
+    __syncwarp();
+    return nfit;
+}
+
+// compensated sums (s - c): b added to a, the rounding of s + s' kept in c
+__device__ __forceinline__ void comp_merge(float2 &a, float2 b)
+{
+    const float t = a.x + b.x, v = t - a.x;
+    const float err = (a.x - (t - v)) + (b.x - v);
+    a = make_float2(t, (a.y + b.y) - err);
+}
+
+// the streams of each target (lanes equal modulo m) into one, in a fixed tree
+__device__ __forceinline__ void comp_streams(float2 *v, int m)
+{
+    for (int o = m; o < 32; o <<= 1) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            comp_merge(v[d], make_float2(__shfl_xor_sync(0xffffffffu, v[d].x, o), __shfl_xor_sync(0xffffffffu, v[d].y, o)));
+    }
+}
+
+// Leaves whose lists are long against a warp's even share of the pass's
+// entries: the kernel below gives each to a whole block, and takes them
+// first.  Halo lists run to several thousand entries, and a small pass has
+// fewer leaves than the chip has warps.  (ctl[0]: the list length above
+// which a leaf is long, ctl[1]: long leaves found, ctl[2], ctl[3]: the
+// kernel's counters of the long and of all leaves)
+// P2P of a pass, a warp per leaf -> with the long leaves split (share 32; 4
+// to 64 lie within 5 % of it): 4,096 grid particles leaf 16, 0.129 -> 0.046
+// ms; 32,768, 0.199 -> 0.159; 250,047 half in halos, leaf 24, 3.60 -> 3.00;
+// 2,097,152 of them 26.0 -> 25.9; 100,003, leaf 8, 1.74 -> 1.34.
+#define OW_SHARE 32  // long: more than 1 / OW_SHARE of a warp's share
+__global__ void k_ow_long(const int *tree_cnt, const unsigned long long *walk_flags, const unsigned long long *fill,
+                          const int *cnt, int nwarps, int share, int *ctl, int *longs)
+{
+    const int nleaf = *walk_flags ? 0 : tree_cnt[BC_LEAVES];
+    const unsigned long long even = *fill / ((unsigned long long)nwarps * share);
+    const int limit = even < 32 ? 32 : (even > 0x7fffffffull ? 0x7fffffff : (int)even);
+    const int lane = warp_lane();
+    const int stride = gridDim.x * blockDim.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[0] = limit;
+    for (int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; t0 < nleaf; t0 += stride) {
+        const int t = t0 + lane;
+        const bool is = t < nleaf && cnt[t] > limit;
+        const unsigned m = __ballot_sync(0xffffffffu, is);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(ctl + 1, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (is) longs[at + __popc(m & ((1u << lane) - 1u))] = t;
+    }
+}
+
+// W = P2P_WARPS: the long leaves, a block each; W = 1: the others, a warp
+// each.  (Two kernels: one that did both in turn spilled registers and ran
+// 5-8 % slower.)
+template <int W>
 __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A)
 {
     __shared__ __align__(16) float s_x[P2P_WARPS][STAGE2 + 2];
     __shared__ __align__(16) float s_y[P2P_WARPS][STAGE2 + 2];
     __shared__ __align__(16) float s_z[P2P_WARPS][STAGE2 + 2];
-    __shared__ double s_red[P2P_WARPS][32][3];
+    __shared__ __align__(16) float4 s_meta[P2P_WARPS][32];
+    __shared__ int s_leaf;
     const int lane = warp_lane();
     const int wib = threadIdx.x >> 5;
     float *sx = s_x[wib], *sy = s_y[wib], *sz = s_z[wib];
@@ -425,24 +542,33 @@ __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A
     const float2 *Z2 = reinterpret_cast<const float2 *>(sz);
     SplitConsts K = A.k;  // polynomial coefficients; the rest per target box below
 
-    const int nleaf = p2p_targets(A);
+    const int nleaf = p2p_targets(A), limit = A.ow_ctl[0];
     for (;;) {
         int t;
-        if (lane == 0) t = atomicAdd(A.work_counter, 1);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= nleaf) break;
+        if (W > 1) {
+            // (every warp has read s_leaf before the barriers at a leaf's end)
+            if (threadIdx.x == 0) s_leaf = atomicAdd(A.ow_ctl + 2, 1);
+            __syncthreads();
+            if (nleaf == 0 || s_leaf >= A.ow_ctl[1]) break;
+            t = A.ow_long[s_leaf];
+        } else {
+            if (lane == 0) t = atomicAdd(A.ow_ctl + 3, 1);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t >= nleaf) break;
+            if (A.p2p_cnt[t] > limit) continue;
+        }
         const int nt = A.npart[t], it = A.ipart[t];
-        if (nt == 0) continue;
         const BoxParams &B = A.boxes[A.boxid[t]];
         K.sig = B.sig;
         K.e2s = B.e2s;
         K.pias = B.pias;
         K.cs = B.cs;
         const float Lhi = B.Lhi, Llo = B.Llo;
-        const double acc_scale = B.acc_scale;
         const float4 cth = A.chi[t], ctl = A.clo[t];
-        const long long eoff = A.p2p_off[t];
-        const int ecnt = A.p2p_cnt[t];
+        // this warp's part of the list
+        const int all = A.p2p_cnt[t], per = (all + W - 1) / W;
+        const int first = W > 1 ? min(all, wib * per) : 0, ecnt = min(all, first + per) - first;
+        const uint32_t *list = A.p2p_pool + A.p2p_off[t] + first;
 
         for (int tb = 0; tb < nt; tb += 64) {
             // rounds: m1 = largest power of two <= min(nb, 32); m2 covers the rest
@@ -458,126 +584,68 @@ __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A
             // round-2 lanes beyond the block's last target reuse it; their sums are discarded
             const float4 o2 = m2 ? scaled(A.pos4[it + tb + m1 + min(q2, rest - 1)], K.sig)
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-            float s1x = 0.f, s1y = 0.f, s1z = 0.f, c1x = 0.f, c1y = 0.f, c1z = 0.f;
-            float s2x = 0.f, s2y = 0.f, s2z = 0.f, c2x = 0.f, c2y = 0.f, c2z = 0.f;
-
-            int e = 0;
-            while (e < ecnt) {
-                // lane i owns entry e+i: source leaf, size, centre offset
-                const int ne = min(32, ecnt - e);
-                int is = 0, ns = 0;
-                float d0 = 0.f, d1 = 0.f, d2 = 0.f;
-                if (lane < ne) {
-                    uint32_t en = A.p2p_pool[eoff + e + lane];
-                    int s = PH_ENTRY_ID(en), img = PH_ENTRY_IMG(en);
-                    is = A.ipart[s];
-                    ns = A.npart[s];
-                    const float4 csh = A.chi[s], csl = A.clo[s];
-                    int mi, mj, mk;
-                    image_offsets(img, mi, mj, mk);
-                    d0 = centre_diff(csh.x, csl.x, cth.x, ctl.x, mi, Lhi, Llo) * K.sig;
-                    d1 = centre_diff(csh.y, csl.y, cth.y, ctl.y, mj, Lhi, Llo) * K.sig;
-                    d2 = centre_diff(csh.z, csl.z, cth.z, ctl.z, mk, Lhi, Llo) * K.sig;
-                }
-                const int incl = warp_incl_scan(ns);
-                const unsigned fit = __ballot_sync(0xffffffffu, lane < ne && incl <= STAGE2);
-                const int nfit = __popc(fit);
-                if (nfit == 0) break;  // unreachable under the MAXLEAF bound; never spin
-                const int nstaged = __shfl_sync(0xffffffffu, incl, nfit - 1);
-                const int pre = incl - ns;
-                // cooperative staging: staged source idx -> its entry by binary search
-                for (int s0 = 0; s0 < nstaged; s0 += 32) {
-                    const int idx = s0 + lane;
-                    int lo = 0;
+            float2 v1[3], v2[3];  // running sums and their compensations
 #pragma unroll
-                    for (int step = 16; step >= 1; step >>= 1) {
-                        const int cand = lo + step;
-                        const int pc = __shfl_sync(0xffffffffu, pre, cand & 31);
-                        if (cand < nfit && pc <= idx) lo = cand;
-                    }
-                    const int eis = __shfl_sync(0xffffffffu, is, lo);
-                    const int epre = __shfl_sync(0xffffffffu, pre, lo);
-                    const float e0 = __shfl_sync(0xffffffffu, d0, lo);
-                    const float e1 = __shfl_sync(0xffffffffu, d1, lo);
-                    const float e2 = __shfl_sync(0xffffffffu, d2, lo);
-                    if (idx < nstaged) {
-                        const float4 o = A.pos4[eis + idx - epre];
-                        sx[idx] = fmaf(o.x, K.sig, e0);
-                        sy[idx] = fmaf(o.y, K.sig, e1);
-                        sz[idx] = fmaf(o.z, K.sig, e2);
-                    }
-                }
-                // an odd count gets one far-away source whose force is exactly 0
-                if (lane == 0 && (nstaged & 1)) {
-                    sx[nstaged] = 1e18f;
-                    sy[nstaged] = 1e18f;
-                    sz[nstaged] = 1e18f;
-                }
-                __syncwarp();
+            for (int d = 0; d < 3; d++) v1[d] = v2[d] = make_float2(0.f, 0.f);
+
+            for (int e = 0; e < ecnt;) {
+                int nstaged;
+                const int took = ow_stage(A, list + e, ecnt - e, cth, ctl, K.sig, Lhi, Llo, sx, sy, sz, s_meta[wib],
+                                          lane, nstaged);
+                if (took == 0) break;
+                e += took;
                 const int npairs = (nstaged + 1) >> 1;
                 float px, py, pz;
                 if (m2 == m1) {
                     // equal rounds (a block of 2m targets): one sweep for both
                     float qx, qy, qz;
                     p2p_round_dual(X2, Y2, Z2, npairs, k1, G1, o1, o2, K, px, py, pz, qx, qy, qz);
-                    kahan_add(s1x, c1x, px);
-                    kahan_add(s1y, c1y, py);
-                    kahan_add(s1z, c1z, pz);
-                    kahan_add(s2x, c2x, qx);
-                    kahan_add(s2y, c2y, qy);
-                    kahan_add(s2z, c2z, qz);
-                    __syncwarp();
-                    e += nfit;
-                    continue;
+                    kahan_add(v2[0].x, v2[0].y, qx);
+                    kahan_add(v2[1].x, v2[1].y, qy);
+                    kahan_add(v2[2].x, v2[2].y, qz);
+                } else {
+                    p2p_round(X2, Y2, Z2, npairs, k1, G1, o1.x, o1.y, o1.z, K, px, py, pz);
                 }
-                p2p_round(X2, Y2, Z2, npairs, k1, G1, o1.x, o1.y, o1.z, K, px, py, pz);
-                kahan_add(s1x, c1x, px);
-                kahan_add(s1y, c1y, py);
-                kahan_add(s1z, c1z, pz);
-                if (m2) {
+                kahan_add(v1[0].x, v1[0].y, px);
+                kahan_add(v1[1].x, v1[1].y, py);
+                kahan_add(v1[2].x, v1[2].y, pz);
+                if (m2 && m2 != m1) {
                     p2p_round(X2, Y2, Z2, npairs, k2, G2, o2.x, o2.y, o2.z, K, px, py, pz);
-                    kahan_add(s2x, c2x, px);
-                    kahan_add(s2y, c2y, py);
-                    kahan_add(s2z, c2z, pz);
+                    kahan_add(v2[0].x, v2[0].y, px);
+                    kahan_add(v2[1].x, v2[1].y, py);
+                    kahan_add(v2[2].x, v2[2].y, pz);
                 }
                 __syncwarp();
-                e += nfit;
             }
-            // combine the streams of each target in a fixed order
-            double *red = &s_red[wib][0][0];
-            red[3 * lane + 0] = (double)s1x - (double)c1x;
-            red[3 * lane + 1] = (double)s1y - (double)c1y;
-            red[3 * lane + 2] = (double)s1z - (double)c1z;
-            __syncwarp();
-            if (lane < m1) {
-                double b0 = 0.0, b1 = 0.0, b2 = 0.0;
-                for (int k = 0; k < G1; k++) {
-                    const int l = k * m1 + lane;
-                    b0 += red[3 * l]; b1 += red[3 * l + 1]; b2 += red[3 * l + 2];
+            // the streams of each target, then the group's warps, in a fixed order
+            comp_streams(v1, m1);
+            if (m2) comp_streams(v2, m2);
+            const double acc_scale = B.acc_scale;
+            double *const out[3] = {A.ax + it + tb, A.ay + it + tb, A.az + it + tb};
+            if (W == 1) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    if (lane < m1) out[d][lane] += ((double)v1[d].x - (double)v1[d].y) * acc_scale;
+                    if (lane < rest) out[d][m1 + lane] += ((double)v2[d].x - (double)v2[d].y) * acc_scale;
                 }
-                const int ip = it + tb + lane;
-                A.ax[ip] += b0 * acc_scale;
-                A.ay[ip] += b1 * acc_scale;
-                A.az[ip] += b2 * acc_scale;
-            }
-            __syncwarp();
-            if (m2) {
-                red[3 * lane + 0] = (double)s2x - (double)c2x;
-                red[3 * lane + 1] = (double)s2y - (double)c2y;
-                red[3 * lane + 2] = (double)s2z - (double)c2z;
-                __syncwarp();
-                if (lane < rest) {
-                    double b0 = 0.0, b1 = 0.0, b2 = 0.0;
-                    for (int k = 0; k < G2; k++) {
-                        const int l = k * m2 + lane;
-                        b0 += red[3 * l]; b1 += red[3 * l + 1]; b2 += red[3 * l + 2];
-                    }
-                    const int ip = it + tb + m1 + lane;
-                    A.ax[ip] += b0 * acc_scale;
-                    A.ay[ip] += b1 * acc_scale;
-                    A.az[ip] += b2 * acc_scale;
+            } else {
+                // the warps' sums through their stages, [3][64] each
+                float2 *red = reinterpret_cast<float2 *>(sx);
+                static_assert(3 * 64 * sizeof(float2) <= sizeof s_x[0], "the sums fit a stage");
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    if (lane < m1) red[64 * d + lane] = v1[d];
+                    if (lane < rest) red[64 * d + m1 + lane] = v2[d];
                 }
-                __syncwarp();
+                __syncthreads();
+                for (int i = threadIdx.x; i < 3 * nb; i += P2P_TB) {
+                    const int d = i / nb, q = i - d * nb;
+                    float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < P2P_WARPS; k++) comp_merge(v, reinterpret_cast<float2 *>(s_x[k])[64 * d + q]);
+                    (d == 0 ? out[0] : (d == 1 ? out[1] : out[2]))[q] += ((double)v.x - (double)v.y) * acc_scale;
+                }
+                __syncthreads();
             }
         }
     }
@@ -1959,10 +2027,19 @@ int launch_p2p(const P2PArgs &a, int fp64, cudaStream_t st)
     if (!fp64 && a.variant == 1 && a.nbox != 1)
         return ph_set_error(8, "the scalar FP32 P2P kernel runs one box per pass");
     PH_CUDA_CHECK(cudaMemsetAsync(a.work_counter, 0, sizeof(int), st));
-    int blocks = device_sm_count() * (fp64 ? 4 : 4);
-    if (fp64) ph::note_launch(), k_p2p_fp64<<<blocks, P2P_TB, 0, st>>>(a);
-    else if (a.variant == 1) ph::note_launch(), k_p2p_split<<<blocks, P2P_TB, 0, st>>>(a);
-    else ph::note_launch(), k_p2p_split_packed<<<blocks, P2P_TB, 0, st>>>(a);
+    int blocks = device_sm_count() * 4;
+    if (fp64) {
+        ph::note_launch(), k_p2p_fp64<<<blocks, P2P_TB, 0, st>>>(a);
+    } else if (a.variant == 1) {
+        ph::note_launch(), k_p2p_split<<<blocks, P2P_TB, 0, st>>>(a);
+    } else {
+        const int resident = device_sm_count() * P2P_MINB;
+        PH_CUDA_CHECK(cudaMemsetAsync(a.ow_ctl, 0, 4 * sizeof(int), st));
+        ph::note_launch(), k_ow_long<<<device_sm_count(), 256, 0, st>>>(a.tree_cnt, a.walk_flags, a.p2p_fill, a.p2p_cnt,
+                                                                         resident * P2P_WARPS, OW_SHARE, a.ow_ctl, a.ow_long);
+        ph::note_launch(), k_p2p_split_packed<P2P_WARPS><<<resident, P2P_TB, 0, st>>>(a);
+        ph::note_launch(), k_p2p_split_packed<1><<<resident, P2P_TB, 0, st>>>(a);
+    }
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

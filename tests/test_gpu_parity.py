@@ -417,3 +417,22 @@ def test_fp64_pair_paths_match_oracle(ph, fp, ics, port, workload, nside, maxlea
     acc_ref = np.empty_like(r["acc"])
     acc_ref[r["perm"]] = r["acc"]
     assert rel_err(acc, acc_ref, p).max() <= FP64_TOL
+
+
+@pytest.mark.parametrize("workload,nside,maxleaf", [
+    ("grid32", 12, 16),    # fewer leaves than warps: every list split over a block
+    ("nfw128", 32, 8),     # both kinds: long halo lists a block each, the others a warp each
+    ("nfw128", 28, 100),   # leaves above 64 particles: two blocks of targets
+    ("grid32", 16, 1),     # one-particle leaves
+    ("grid32", 20, 33)])
+def test_fp32_long_lists_split_over_a_block(ph, fp, ics, workload, nside, maxleaf):
+    """The one-way FP32 kernel where lists are split over a block's warps,
+    against the FP64 pass on the same lists.  Bars: those of the clustered
+    inputs (median 1e-5, 99th percentile 1e-4); passes are deterministic."""
+    pos, p = ics.make(workload, nside=nside, maxleaf=maxleaf)
+    a64 = fp.run(pos, p, precision=ph.FP64)
+    a32 = fp.run(pos, p, precision=ph.FP32_SPLIT, flags=ph.F_ONE_WAY)
+    e = rel_err(a32, a64, p)
+    assert np.median(e) <= 1e-5, np.median(e)
+    assert np.percentile(e, 99) <= 1e-4, np.percentile(e, 99)
+    assert np.array_equal(a32, fp.run(pos, p, precision=ph.FP32_SPLIT, flags=ph.F_ONE_WAY))
