@@ -48,8 +48,9 @@
 // levels of at most this many nodes run their bookkeeping in one block
 #define SMALL_LEVEL 32
 
-// depth lists: unified ids per block (one warp) of the counting sort
-#define DEPTH_R 4096
+// depth lists: unified ids per block (one warp) of the counting sort (4096,
+// a load at a time: k_depth_place 66-75 us whatever the size of the tree)
+#define DEPTH_R 1024
 
 // temp-node modes: 0-2 the kinds of a split node (two-ended swap, nothing
 // above the mean, a pair), then the two states of a node not yet split
@@ -1007,6 +1008,7 @@ __global__ void __launch_bounds__(32) k_depth_count(BuildBufs b, TreeBufs T, int
     for (int d = lane; d < ndepth; d += 32) h[d] = 0;
     __syncwarp();
     const int u0 = k * DEPTH_R, u1 = min(nu, u0 + DEPTH_R);
+#pragma unroll 8
     for (int u = u0 + lane; u < u1; u += 32) {
         const int d = T.depth[u];
         if (d >= 0 && d < ndepth) atomicAdd(&h[d], 1);
@@ -1040,15 +1042,21 @@ __global__ void __launch_bounds__(32) k_depth_place(BuildBufs b, TreeBufs T, int
     }
     __syncwarp();
     const int u0 = k * DEPTH_R, u1 = min(nu, u0 + DEPTH_R);
-    for (int base = u0; base < u1; base += 32) {
-        const int u = base + lane;
-        int d = u < u1 ? T.depth[u] : -1;
-        if (d >= ndepth) d = -1;
-        const unsigned same = __match_any_sync(0xffffffffu, d);
-        if (d >= 0) T.depth_list[cur[d] + __popc(same & lt)] = u;
-        __syncwarp();
-        if (d >= 0 && (same & lt) == 0) cur[d] += __popc(same);
-        __syncwarp();
+    for (int b0 = u0; b0 < u1; b0 += 256) {
+        int dd[8];  // eight loads ahead of the placing, which is serial
+#pragma unroll
+        for (int q = 0; q < 8; q++) dd[q] = b0 + 32 * q + lane < u1 ? T.depth[b0 + 32 * q + lane] : -1;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int u = b0 + 32 * q + lane;
+            int d = dd[q];
+            if (d >= ndepth) d = -1;
+            const unsigned same = __match_any_sync(0xffffffffu, d);
+            if (d >= 0) T.depth_list[cur[d] + __popc(same & lt)] = u;
+            __syncwarp();
+            if (d >= 0 && (same & lt) == 0) cur[d] += __popc(same);
+            __syncwarp();
+        }
     }
 }
 
