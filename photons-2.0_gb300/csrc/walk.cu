@@ -412,13 +412,14 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
 #pragma unroll
             for (int s = 0; s < 2; s++) {
                 const int kd = kind[s];
+                // positions by ballots: a push takes one place, a self push and
+                // an opened source two
                 const unsigned mp = __ballot_sync(0xffffffffu, kd == OUT_P2P);
                 const unsigned mm = __ballot_sync(0xffffffffu, kd == OUT_M2L);
-                const int npush = (kd == OUT_PUSH) ? 1 : (kd == OUT_SELF_PUSH ? 2 : 0);
-                const int nopen = (kd == OUT_OPEN) ? 2 : 0;
-                const int push_incl = warp_incl_scan(npush);
-                const int open_incl = warp_incl_scan(nopen);
-                const int push_tot = shfl(push_incl, 31), open_tot = shfl(open_incl, 31);
+                const unsigned mu = __ballot_sync(0xffffffffu, kd == OUT_PUSH);
+                const unsigned ms = __ballot_sync(0xffffffffu, kd == OUT_SELF_PUSH);
+                const unsigned mo = __ballot_sync(0xffffffffu, kd == OUT_OPEN);
+                const int push_at = n_pd + __popc(mu & lt) + 2 * __popc(ms & lt);
                 if (kd == OUT_P2P) {
                     const int pos = n_p2p + __popc(mp & lt);
                     if (pos < W.stage_cap) put2(sh_p2p, WS_P2P, st_p2p, pos, e[s]);
@@ -426,16 +427,16 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
                     const int pos = n_m2l + __popc(mm & lt);
                     if (pos < W.stage_cap) put2(sh_m2l, WS_M2L, st_m2l, pos, e[s]);
                 } else if (kd == OUT_PUSH) {
-                    const int pos = n_pd + push_incl - 1;
+                    const int pos = push_at;
                     if (pos < W.stage_cap) put2(sh_pd, WS_PD, st_pd, pos, e[s]);
                 } else if (kd == OUT_SELF_PUSH) {
-                    const int pos = n_pd + push_incl - 2;
+                    const int pos = push_at;
                     if (pos + 1 < W.stage_cap) {
                         put2(sh_pd, WS_PD, st_pd, pos, PH_ENTRY(a0, 0));
                         put2(sh_pd, WS_PD, st_pd, pos + 1, PH_ENTRY(a1, 0));
                     }
                 } else if (kd == OUT_OPEN) {
-                    const int pos = top + open_incl - 2;
+                    const int pos = top + 2 * __popc(mo & lt);
                     if (pos + 1 < W.stack_cap) {
                         put2(sh_stack, WS_STACK, stack, pos, PH_ENTRY(ch[s].x, img[s]));
                         put2(sh_stack, WS_STACK, stack, pos + 1, PH_ENTRY(ch[s].y, img[s]));
@@ -443,8 +444,8 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
                 }
                 n_p2p += __popc(mp);
                 n_m2l += __popc(mm);
-                n_pd += push_tot;
-                top += open_tot;
+                n_pd += __popc(mu) + 2 * __popc(ms);
+                top += 2 * __popc(mo);
                 if (top > W.stack_cap) {
                     flags |= PH_FLAG_STACK_OVERFLOW;
                     top = W.stack_cap;  // entries beyond were dropped; results are invalid
@@ -504,8 +505,9 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         if (c_pl) atomicAdd(&W.ctr[WC_PAIRS_LOCAL], c_pl);
         if (c_pi) atomicAdd(&W.ctr[WC_PAIRS_IMAGE], c_pi);
         if (flags) atomicOr(&W.ctr[WC_FLAGS], (unsigned long long)flags);
-        atomicMax(&W.ctr[WC_MAX_STACK], (unsigned long long)max_stack);
-        atomicMax(&W.ctr[WC_MAX_STAGE], (unsigned long long)max_stage);
+        // (warps without a target touch no counter but their ticket's)
+        if (max_stack) atomicMax(&W.ctr[WC_MAX_STACK], (unsigned long long)max_stack);
+        if (max_stage) atomicMax(&W.ctr[WC_MAX_STAGE], (unsigned long long)max_stage);
     }
 }
 
