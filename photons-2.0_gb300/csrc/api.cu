@@ -957,7 +957,6 @@ int ph_stage_p2p(photons_ctx *c, int precision, int zero)
     a.boxid = c->t.boxid;
     a.boxes = c->b.boxes;
     a.nbox = c->b.nbox;
-    a.leaf_cap = c->b.rule_cap;
     a.p2p_pool = c->w.p2p_pool; a.p2p_off = c->w.p2p_off; a.p2p_cnt = c->w.p2p_cnt;
     a.pos4 = c->pos4;
     a.chi = c->t.chi;
@@ -967,7 +966,7 @@ int ph_stage_p2p(photons_ctx *c, int precision, int zero)
     a.work_counter = c->work_counter;
     a.ow_ctl = c->work_counter + 4;
     a.ow_long = c->mu_sorted;  // (the mutual kernels' list flags: not in use with the packed kernel)
-    a.p2p_fill = c->w.ctr + ph::WC_P2P_FILL;
+    a.maxleaf = c->pp.maxleaf;
     a.boxsize = c->pp.boxsize; a.eps = c->pp.eps; a.mass = c->pp.mass; a.rs = c->pp.rs;
     a.k = ph::make_split_consts(c->pp);
     a.variant = p2p_variant();

@@ -492,32 +492,33 @@ __device__ __forceinline__ void comp_streams(float2 *v, int m)
     }
 }
 
-// Leaves whose lists are long against a warp's even share of the pass's
+// Leaves whose lists are long against a warp's even share of their box's
 // entries: the kernel below gives each to a whole block, and takes them
 // first.  Halo lists run to several thousand entries, and a small pass has
-// fewer leaves than the chip has warps.  (ctl[0]: the list length above
-// which a leaf is long, ctl[1]: long leaves found, ctl[2], ctl[3]: the
-// kernel's counters of the long and of all leaves)
-// P2P of a pass, a warp per leaf -> with the long leaves split (share 32; 4
-// to 64 lie within 5 % of it): 4,096 grid particles leaf 16, 0.129 -> 0.046
-// ms; 32,768, 0.199 -> 0.159; 250,047 half in halos, leaf 24, 3.60 -> 3.00;
-// 2,097,152 of them 26.0 -> 25.9; 100,003, leaf 8, 1.74 -> 1.34.
-#define OW_SHARE 32  // long: more than 1 / OW_SHARE of a warp's share
-__global__ void k_ow_long(const int *tree_cnt, const unsigned long long *walk_flags, const unsigned long long *fill,
-                          const int *cnt, int nwarps, int share, int *ctl, int *longs)
+// fewer leaves than the chip has warps.  A box of n particles has about 400 n
+// / MAXLEAF entries, 1/4,000 of that is a warp's share, and a list above
+// about a tenth of it is long; lists of up to 32 entries (one batch) never
+// are.  The rule looks at the leaf's own box only, so a box gives the same
+// forces in a batch and alone.  P2P of a pass, a warp per leaf -> with the
+// long leaves split: 4,096 grid particles leaf 16, 0.129 -> 0.046 ms; 32,768,
+// 0.199 -> 0.159; 250,047 half in halos, leaf 24, 3.60 -> 3.00; 2,097,152 of
+// them 26.0 -> 25.9; 100,003, leaf 8, 1.74 -> 1.34.
+__device__ __forceinline__ int ow_limit(const BoxParams &B, int maxleaf) { return max(32, B.count / (100 * maxleaf)); }
+
+// the long leaves (ctl[0]: their number; ctl[1], ctl[2]: the kernel's
+// counters of the long and of all leaves)
+__global__ void k_ow_long(const int *tree_cnt, const unsigned long long *walk_flags, const int *cnt, const int *boxid,
+                          const BoxParams *boxes, int maxleaf, int *ctl, int *longs)
 {
     const int nleaf = *walk_flags ? 0 : tree_cnt[BC_LEAVES];
-    const unsigned long long even = *fill / ((unsigned long long)nwarps * share);
-    const int limit = even < 32 ? 32 : (even > 0x7fffffffull ? 0x7fffffff : (int)even);
     const int lane = warp_lane();
     const int stride = gridDim.x * blockDim.x;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[0] = limit;
     for (int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; t0 < nleaf; t0 += stride) {
         const int t = t0 + lane;
-        const bool is = t < nleaf && cnt[t] > limit;
+        const bool is = t < nleaf && cnt[t] > ow_limit(boxes[boxid[t]], maxleaf);
         const unsigned m = __ballot_sync(0xffffffffu, is);
         int at = 0;
-        if (lane == 0 && m) at = atomicAdd(ctl + 1, __popc(m));
+        if (lane == 0 && m) at = atomicAdd(ctl, __popc(m));
         at = __shfl_sync(0xffffffffu, at, 0);
         if (is) longs[at + __popc(m & ((1u << lane) - 1u))] = t;
     }
@@ -542,20 +543,20 @@ __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A
     const float2 *Z2 = reinterpret_cast<const float2 *>(sz);
     SplitConsts K = A.k;  // polynomial coefficients; the rest per target box below
 
-    const int nleaf = p2p_targets(A), limit = A.ow_ctl[0];
+    const int nleaf = p2p_targets(A);
     for (;;) {
         int t;
         if (W > 1) {
             // (every warp has read s_leaf before the barriers at a leaf's end)
-            if (threadIdx.x == 0) s_leaf = atomicAdd(A.ow_ctl + 2, 1);
+            if (threadIdx.x == 0) s_leaf = atomicAdd(A.ow_ctl + 1, 1);
             __syncthreads();
-            if (nleaf == 0 || s_leaf >= A.ow_ctl[1]) break;
+            if (s_leaf >= A.ow_ctl[0]) break;
             t = A.ow_long[s_leaf];
         } else {
-            if (lane == 0) t = atomicAdd(A.ow_ctl + 3, 1);
+            if (lane == 0) t = atomicAdd(A.ow_ctl + 2, 1);
             t = __shfl_sync(0xffffffffu, t, 0);
             if (t >= nleaf) break;
-            if (A.p2p_cnt[t] > limit) continue;
+            if (A.p2p_cnt[t] > ow_limit(A.boxes[A.boxid[t]], A.maxleaf)) continue;
         }
         const int nt = A.npart[t], it = A.ipart[t];
         const BoxParams &B = A.boxes[A.boxid[t]];
@@ -2034,9 +2035,9 @@ int launch_p2p(const P2PArgs &a, int fp64, cudaStream_t st)
         ph::note_launch(), k_p2p_split<<<blocks, P2P_TB, 0, st>>>(a);
     } else {
         const int resident = device_sm_count() * P2P_MINB;
-        PH_CUDA_CHECK(cudaMemsetAsync(a.ow_ctl, 0, 4 * sizeof(int), st));
-        ph::note_launch(), k_ow_long<<<device_sm_count(), 256, 0, st>>>(a.tree_cnt, a.walk_flags, a.p2p_fill, a.p2p_cnt,
-                                                                         resident * P2P_WARPS, OW_SHARE, a.ow_ctl, a.ow_long);
+        PH_CUDA_CHECK(cudaMemsetAsync(a.ow_ctl, 0, 3 * sizeof(int), st));
+        ph::note_launch(), k_ow_long<<<device_sm_count(), 256, 0, st>>>(a.tree_cnt, a.walk_flags, a.p2p_cnt, a.boxid,
+                                                                         a.boxes, a.maxleaf, a.ow_ctl, a.ow_long);
         ph::note_launch(), k_p2p_split_packed<P2P_WARPS><<<resident, P2P_TB, 0, st>>>(a);
         ph::note_launch(), k_p2p_split_packed<1><<<resident, P2P_TB, 0, st>>>(a);
     }

@@ -32,15 +32,13 @@ struct P2PArgs {
     // output (tree order); written, not accumulated
     double *ax, *ay, *az;
     int *work_counter;
-    // packed kernel: its control words [4] and the long leaves (see k_ow_long),
-    // and the walk's count of list entries
+    // packed kernel: its control words [3] and the long leaves (see k_ow_long)
     int *ow_ctl, *ow_long;
-    const unsigned long long *p2p_fill;
+    int maxleaf;
     double boxsize, eps, mass, rs;  // scalar FP32 kernel (one box)
     const int *boxid;               // box of each unified id
     const BoxParams *boxes;         // per-box constants (packed FP32 and FP64 kernels)
     int nbox;
-    int leaf_cap;                   // upper bound of the leaves (2N/MAXLEAF); trees have about half to 0.7 of it
     SplitConsts k;                  // scalar kernel: all fields; packed: the polynomial coefficients
     int variant;  // FP32: 0 packed (default), 1 scalar
     int shape;    // mutual kernel build (0: by MAXLEAF; see launch_p2p_mutual)
