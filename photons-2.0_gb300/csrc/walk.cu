@@ -278,32 +278,25 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         int top = 0, in_pos = 0;
         int n_p2p = 0, n_m2l = 0, n_pd = 0;
         for (;;) {
-            // up to 64 entries per step, two per lane, stack first
-            int k;
+            // up to 64 entries per step, two per lane: from the stack, topped up
+            // from the list
+            const int k0 = min(64, top), k = k0 + min(64 - k0, n_in - in_pos);
+            if (k == 0) break;
+            top -= k0;
             uint32_t e[2] = {0u, 0u};
-            if (top > 0) {
-                k = min(64, top);
-                top -= k;
-                if (lane < k) e[0] = get2(sh_stack, WS_STACK, stack, top + lane);
-                if (lane + 32 < k) e[1] = get2(sh_stack, WS_STACK, stack, top + lane + 32);
-            } else if (in_pos < n_in) {
-                k = min(64, n_in - in_pos);
-                if (input) {
-                    if (lane < k) e[0] = input[in_pos + lane];
-                    if (lane + 32 < k) e[1] = input[in_pos + lane + 32];
-                } else {
+#pragma unroll
+            for (int s2 = 0; s2 < 2; s2++) {
+                const int j = lane + 32 * s2, i = in_pos + j - k0;
+                if (j < k0) {
+                    e[s2] = get2(sh_stack, WS_STACK, stack, top + j);
+                } else if (j < k) {
                     // the root's list: itself under each selected image, then the received trees
-                    for (int s2 = 0; s2 < 2; s2++) {
-                        const int i = in_pos + lane + 32 * s2;
-                        if (lane + 32 * s2 < k)
-                            e[s2] = i < A.nroot ? PH_ENTRY(a, A.root_img[i])
-                                                : PH_ENTRY(A.imp.root[i - A.nroot], PH_IMG_IMPORT);
-                    }
+                    if (input) e[s2] = input[i];
+                    else if (i < A.nroot) e[s2] = PH_ENTRY(a, A.root_img[i]);
+                    else e[s2] = PH_ENTRY(A.imp.root[i - A.nroot], PH_IMG_IMPORT);
                 }
-                in_pos += k;
-            } else {
-                break;
             }
+            in_pos += k - k0;
             __syncwarp();
             // load phase: everything both slots need, before any use
             int b[2], img[2], need[2], npb[2];
