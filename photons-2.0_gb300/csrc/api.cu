@@ -132,6 +132,7 @@ static int alloc_particles(photons_ctx *c, int n)
     c->epoch++;
     PH_TRY(dalloc(b.x, n)); PH_TRY(dalloc(b.y, n)); PH_TRY(dalloc(b.z, n));
     PH_TRY(dalloc(b.perm, n)); PH_TRY(dalloc(b.smallpos, n)); PH_TRY(dalloc(b.bigpos, n));
+    PH_TRY(dalloc(b.words, n / 32 + 1)); PH_TRY(dalloc(b.wordpre, n / 32 + 1));
     PH_TRY(dalloc(c->pos4, n));
     PH_TRY(dalloc(c->ax, n)); PH_TRY(dalloc(c->ay, n)); PH_TRY(dalloc(c->az, n));
     PH_TRY(dalloc(c->io, (size_t)3 * n));
@@ -155,18 +156,15 @@ static int alloc_tree(photons_ctx *c, int n, int cap)
         PH_TRY(dalloc(b.tn_mode, cap)); PH_TRY(dalloc(b.tn_S, cap)); PH_TRY(dalloc(b.tn_box, (size_t)6 * cap));
         PH_TRY(dalloc(b.tn_split, cap)); PH_TRY(dalloc(b.tn_nch, cap)); PH_TRY(dalloc(b.tn_chunk_base, cap));
         PH_TRY(dalloc(b.tn_nodeflag, cap)); PH_TRY(dalloc(b.tn_leafflag, cap)); PH_TRY(dalloc(b.tn_nodebase, cap));
-        PH_TRY(dalloc(b.tn_leafbase, cap)); PH_TRY(dalloc(b.tn_sub_nodes, cap)); PH_TRY(dalloc(b.tn_sub_leaves, cap));
-        PH_TRY(dalloc(b.tn_pre, cap)); PH_TRY(dalloc(b.tn_lbase, cap));
+        PH_TRY(dalloc(b.tn_leafbase, cap));
+        PH_TRY(dalloc(b.lf_depth, cap)); PH_TRY(dalloc(b.lf_top, cap)); PH_TRY(dalloc(b.lf_base, cap));
         PH_TRY(dalloc(b.tl_start, cap)); PH_TRY(dalloc(b.tl_len, cap)); PH_TRY(dalloc(b.tl_depth, cap));
-        PH_TRY(dalloc(b.tl_parent, cap)); PH_TRY(dalloc(b.tl_final, cap)); PH_TRY(dalloc(b.tl_box, (size_t)6 * cap));
+        PH_TRY(dalloc(b.tl_parent, cap)); PH_TRY(dalloc(b.tl_box, (size_t)6 * cap));
         PH_TRY(dalloc(b.tn_boxid, cap)); PH_TRY(dalloc(b.tl_boxid, cap));
-        PH_TRY(dalloc(b.tn_subroot, cap)); PH_TRY(dalloc(b.tl_subroot, cap));
         const size_t scratch = ph::scan_scratch_elems(cap > chunks ? cap : chunks) + 8;
         PH_TRY(dalloc(b.scan_scratch, scratch));
         b.scan_scratch_elems = scratch;
         PH_TRY(dalloc(b.cnt, ph::BC_NCOUNTERS));
-        PH_TRY(dalloc(b.lvl_begin, MAX_DEPTH_CAP + 2)); PH_TRY(dalloc(b.lvl_count, MAX_DEPTH_CAP + 2));
-        PH_TRY(dalloc(b.leaf_begin, MAX_DEPTH_CAP + 2)); PH_TRY(dalloc(b.leaf_count, MAX_DEPTH_CAP + 2));
         c->epoch++;
         b.cap_nodes = cap;
         b.cap_leaves = cap;
@@ -222,12 +220,14 @@ static int alloc_tree(photons_ctx *c, int n, int cap)
         PH_TRY(dalloc(b.ch_node, chunks)); PH_TRY(dalloc(b.ch_swap, chunks));
         c->epoch++;
         b.cap_chunks = chunks;
-        size_t need = ph::scan_scratch_elems(cap > chunks ? cap : chunks) + 8;
-        if (need > b.scan_scratch_elems) {
-            b.scan_scratch_elems = 0;
-            PH_TRY(dalloc(b.scan_scratch, need));
-            b.scan_scratch_elems = need;
-        }
+    }
+    // scans over the nodes or leaves, the chunks, and the words of the leaf-start mask
+    const size_t need = ph::scan_scratch_elems(std::max(std::max(cap, chunks), n / 32 + 1)) + 8;
+    if (need > b.scan_scratch_elems) {
+        b.scan_scratch_elems = 0;
+        c->epoch++;
+        PH_TRY(dalloc(b.scan_scratch, need));
+        b.scan_scratch_elems = need;
     }
     return 0;
 }
@@ -282,18 +282,18 @@ static void free_all(photons_ctx *c)
     ph::BuildBufs &b = c->b;
     void *ptrs[] = {b.x, b.y, b.z, b.perm, b.smallpos, b.bigpos, b.tn_start, b.tn_len, b.tn_depth, b.tn_parent,
                     b.tn_child0, b.tn_child1, b.tn_mode, b.tn_S, b.tn_box, b.tn_split, b.tn_nch, b.tn_chunk_base,
-                    b.tn_nodeflag, b.tn_leafflag, b.tn_nodebase, b.tn_leafbase, b.tn_sub_nodes, b.tn_sub_leaves,
-                    b.tn_pre, b.tn_lbase, b.tl_start, b.tl_len, b.tl_depth, b.tl_parent, b.tl_final, b.tl_box,
+                    b.tn_nodeflag, b.tn_leafflag, b.tn_nodebase, b.tn_leafbase, b.lf_depth, b.lf_top,
+                    b.lf_base, b.words, b.wordpre, b.tl_start, b.tl_len, b.tl_depth, b.tl_parent, b.tl_box,
                     b.ch_partial, b.ch_cnt, b.ch_small_base, b.ch_node, b.cnt, b.scan_scratch, c->t.ipart, c->t.npart,
                     c->t.depth, c->t.parent, c->t.son0, c->t.son1, c->t.cx, c->t.cy, c->t.cz, c->t.wx, c->t.wy,
                     c->t.wz, c->t.wsum, c->t.split, c->t.depth_list, c->t.depth_off, c->w.pd_pool[0],
                     c->w.pd_pool[1], c->w.pd_off, c->w.pd_cnt, c->w.p2p_pool, c->w.p2p_off, c->w.p2p_cnt,
                     c->w.m2l_pool, c->w.m2l_off, c->w.m2l_cnt, c->w.scratch, c->w.ctr, c->pos4, c->ax, c->ay,
                     c->az, c->M, c->L, c->io, c->work_counter, c->t.chi, c->t.clo, c->t.w32, c->t.son2, c->M32,
-                    b.lvl_begin, b.lvl_count, b.leaf_begin, b.leaf_count, c->t.depth_cnt, b.tn_boxid, b.tl_boxid,
+                    c->t.depth_cnt, b.tn_boxid, b.tl_boxid,
                     c->t.boxid, b.boxes, c->far_gate, c->mu_sorted, c->mu_nrecv, c->mu_slot, c->mu_over,
                     c->mu_size, c->mu_rbase, c->mu_total, c->mu_scan, c->mu_buf, c->mu_ev, c->mu_nev, c->mu_pq, c->mu_items, c->mu_nitems,
-                    b.tn_subroot, b.tl_subroot, b.ch_swap, c->t.depth_blk};
+                    b.ch_swap, c->t.depth_blk};
     for (void *p : ptrs)
         if (p) cudaFree(p);
 }
@@ -613,15 +613,18 @@ static int estimate_levels(int n, int maxleaf)
     return lv < MAX_DEPTH_CAP - 1 ? lv : MAX_DEPTH_CAP - 1;
 }
 
-// levels of wide nodes (more than CHUNK_ELEMS particles) to launch: the
-// last build's need with a margin, else an estimate from N; never above the
-// depth bound
-static int tree_top(const photons_ctx *c, int n, int levels)
+// levels of wide nodes (more than PH_MID particles) to launch: none if every
+// box is smaller, else the last build's need with a margin, else an estimate
+// from the largest; never above the depth bound
+static int tree_top(const photons_ctx *c, int levels)
 {
+    int big = 0;
+    for (const BoxParams &B : c->h_boxes) big = B.count > big ? B.count : big;
+    if (big <= c->b.mid) return 0;
     int top = c->hint_top;
     if (top <= 0) {
         top = 1;
-        while (top < 60 && (double)n / std::ldexp(1.0, top) > (double)CHUNK_ELEMS) top++;
+        while (top < 60 && (double)big / std::ldexp(1.0, top) > (double)c->b.mid) top++;
         top += 2;
     }
     return top < levels ? top : levels;
@@ -716,6 +719,11 @@ static int ph_prepare_boxes(photons_ctx *c, int nbox, const photons_params *p, c
     }
     c->b.nbox = nbox;
     c->b.rule_cap = (int)cap;
+    // Splitting nodes in shared memory saves launches, a block at a time per
+    // SM; above two million particles the levels' throughput is worth more
+    // (build, 2,097,152 near-uniform particles: 1.08 ms either way; 250,047
+    // half in halos 0.83 -> 0.70; 256^3 5.05 -> 5.32)
+    c->b.mid = n <= (1 << 21) ? PH_MID : CHUNK_ELEMS;
     c->pp.boxsize = p->boxsize;
     c->pp.theta = p->theta;
     c->pp.rs = p->rs;
@@ -754,7 +762,7 @@ static int ph_enqueue_tree(photons_ctx *c, const double *src, int levels)
 {
     cudaStream_t st = c->stream;
     PH_TRY(ph::launch_init_particles(c->b, src, c->n, st));
-    PH_TRY(ph::build_tree(c->b, c->t, c->pp, levels, tree_top(c, c->n, levels), st));
+    PH_TRY(ph::build_tree(c->b, c->t, c->pp, c->n, levels, tree_top(c, levels), st));
     PH_TRY(ph::launch_geom32(c->t, c->b.cnt, st));
     PH_TRY(ph::launch_leaf_offsets(c->b, c->t, c->pos4, st));
     c->ndepth = levels + 1;
@@ -772,7 +780,7 @@ static int ph_check_build(photons_ctx *c, int flags, int levels, int *grow)
     if (flags & PH_FLAG_NODE_CAPACITY)
         return ph_set_error(PH_ERR_CAPACITY, "node capacity 2N/MAXLEAF=%d exceeded by the mean-split tree", c->b.rule_cap);
     if (flags & (PH_FLAG_DEPTH | PH_FLAG_TOP)) {
-        const int top = tree_top(c, c->n, levels);
+        const int top = tree_top(c, levels);
         if (flags & PH_FLAG_TOP) c->hint_top = top * 2 > top + 4 ? top * 2 : top + 4;
         if (!(flags & PH_FLAG_DEPTH) && top < levels) {
             *grow = levels;
@@ -798,7 +806,8 @@ static void ph_tree_info_from(photons_ctx *c, const int *h, int levels)
     const int lv = c->info.depth;
     if (levels < lv + 1 || levels > lv + 6) c->hint_levels = lv + 3;
     else c->hint_levels = levels;
-    const int need = c->info.levels > 2 ? c->info.levels - 1 : 1, top = tree_top(c, c->n, levels);
+    const int need = c->info.levels > 2 ? c->info.levels - 1 : 1, top = tree_top(c, levels);
+    if (top == 0) return;
     if (top < need || top > need + 4) c->hint_top = need + 2;
     else c->hint_top = top;
 }
@@ -1067,7 +1076,7 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
 {
     PassKey k;
     memset(&k, 0, sizeof k);
-    k.n = n; k.nbox = c->b.nbox; k.levels = levels; k.top = tree_top(c, n, levels); k.maxleaf = p->maxleaf; k.precision = p->precision; k.flags = p->flags;
+    k.n = n; k.nbox = c->b.nbox; k.levels = levels; k.top = tree_top(c, levels); k.maxleaf = p->maxleaf; k.precision = p->precision; k.flags = p->flags;
     k.dio = dio; k.variant = p2p_variant(); k.nwarps = c->w.nwarps; k.mask = mask;
     k.stage_extra = stage_shortfall();
     k.boxsize = p->boxsize; k.theta = p->theta; k.rs = p->rs; k.rcut = p->rcut; k.eps = p->eps; k.mass = p->mass;

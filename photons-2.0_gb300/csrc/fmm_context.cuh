@@ -24,11 +24,14 @@ struct BuildBufs {
     double *tn_split = nullptr;
     int *tn_nch = nullptr, *tn_chunk_base = nullptr;
     int *tn_nodeflag = nullptr, *tn_leafflag = nullptr, *tn_nodebase = nullptr, *tn_leafbase = nullptr;
-    int *tn_sub_nodes = nullptr, *tn_sub_leaves = nullptr, *tn_pre = nullptr, *tn_lbase = nullptr;
-    int *tn_subroot = nullptr;  // nodes of a shared-memory subtree: the subtree's root
     // temp leaves
-    int *tl_start = nullptr, *tl_len = nullptr, *tl_depth = nullptr, *tl_parent = nullptr, *tl_final = nullptr;
-    int *tl_subroot = nullptr;
+    int *tl_start = nullptr, *tl_len = nullptr, *tl_depth = nullptr, *tl_parent = nullptr;
+    // numbering: bit i of word w: a leaf starts at particle 32 w + i; leaf
+    // starts before each word; per leaf in depth-first order: its depth, the
+    // depth of the topmost node or leaf starting where it does, and the nodes
+    // before it in preorder
+    int *words = nullptr, *wordpre = nullptr;
+    int *lf_depth = nullptr, *lf_top = nullptr, *lf_base = nullptr;
     double *tl_box = nullptr;  // [6][cap_leaves]
     // chunks
     double *ch_partial = nullptr;
@@ -36,11 +39,10 @@ struct BuildBufs {
     int4 *ch_swap = nullptr;  // per chunk: node start, first slot, slots to swap
     // small device counters
     int *cnt = nullptr;  // see BuildCounter
-    int *lvl_begin = nullptr, *lvl_count = nullptr;    // per node level: first temp node, count
-    int *leaf_begin = nullptr, *leaf_count = nullptr;  // per depth: temp leaves created by the level above
     int *scan_scratch = nullptr;
     size_t scan_scratch_elems = 0;
     int cap_nodes = 0, cap_leaves = 0, cap_chunks = 0, cap_n = 0;
+    int mid = 0;       // this build: nodes of at most this many particles are not split by the levels
     int rule_cap = 0;  // this pass's 2N/MAXLEAF capacity (src/fmm.c:203-209), <= cap_nodes
     int *level_begin_h = nullptr;  // host copy, per level
     // boxes: temp node / leaf -> box, and the per-box table
@@ -58,15 +60,23 @@ enum BuildCounter {
     BC_FLAGS = 5,
     BC_LEVEL_BEGIN = 6,   // first temp node of the current level
     BC_NODES = 7,         // temp nodes in total (after the build)
-    BC_NLEVELS = 8,       // node levels built
+    BC_NLEVELS = 8,       // node levels built by the levels, and those they left
     BC_DEPTH = 9,         // deepest depth holding a node or leaf
     BC_SUB_NODES = 10,    // nodes below the roots of shared-memory subtrees
     BC_SUB_LEAVES = 11,   // leaves of shared-memory subtrees
     BC_NEXT_WIDE = 12,    // wide nodes created by the current level
     BC_DEPTH_CELLS = 13,  // cells of the depth-list counting sort
     BC_DEPTH_TOTAL = 14,
-    BC_NCOUNTERS = 16
+    BC_MID_NODES = 15,    // nodes and leaves made by k_mid_build
+    BC_MID_LEAVES = 16,
+    BC_WORDS = 17,        // words of the leaf-start bit mask
+    BC_SCAN_TOTAL = 18,
+    BC_NCOUNTERS = 20
 };
+
+// nodes of at most this many particles are split in shared memory (30 bytes a
+// particle, 210 KB)
+#define PH_MID 7168
 
 // deepest tree the depth lists hold (depths 0..PH_MAX_DEPTH_CAP-1)
 #define PH_MAX_DEPTH_CAP 2048
@@ -151,7 +161,7 @@ int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxPar
                const PassParams &p, unsigned image_mask, cudaStream_t st, const WalkImports &imp = WalkImports());
 
 // top: launched levels of wide nodes (<= levels); levels: depth bound
-int build_tree(BuildBufs &b, TreeBufs &t, const PassParams &p, int levels, int top, cudaStream_t st);
+int build_tree(BuildBufs &b, TreeBufs &t, const PassParams &p, int n, int levels, int top, cudaStream_t st);
 int depth_sort_blocks(int cap_u);
 int read_tree_info(const BuildBufs &b, const TreeBufs &t, int levels, TreeInfo &info);
 
