@@ -1087,53 +1087,6 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
     return k;
 }
 
-static int ph_enqueue_far(photons_ctx *c, const photons_params *p)
-{
-    PH_TRY(ph_stage_multipoles(c));
-    PH_TRY(ph_stage_m2l(c, p->precision));
-    return ph_stage_downward(c, p->precision);
-}
-
-// The far field of a captured pass as the body of a conditional node, which
-// the graph enters only if the walk made an M2L task: ~45 launches that a
-// pass without one went through to find that out (72-82 us of passes over
-// 4,096 to 32,768 grid particles).  The body is captured on a stream of its
-// own; its kernels are counted apart (they run in some passes only).
-static int capture_far_branch(photons_ctx *c, const photons_params *p)
-{
-    cudaStreamCaptureStatus status;
-    cudaGraph_t graph = nullptr, body = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    if (!c->body_stream) PH_CUDA_CHECK(cudaStreamCreateWithFlags(&c->body_stream, cudaStreamNonBlocking));
-    PH_CUDA_CHECK(cudaStreamGetCaptureInfo(c->stream, &status, nullptr, &graph, nullptr, nullptr, nullptr));
-    cudaGraphConditionalHandle branch;
-    PH_CUDA_CHECK(cudaGraphConditionalHandleCreate(&branch, graph, 0, cudaGraphCondAssignDefault));
-    PH_TRY(ph::launch_far_branch(c->w.ctr, c->far_gate, branch, c->stream));
-    PH_CUDA_CHECK(cudaStreamGetCaptureInfo(c->stream, &status, nullptr, &graph, &deps, nullptr, &ndeps));
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = branch;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    PH_CUDA_CHECK(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &np));
-    PH_CUDA_CHECK(cudaStreamUpdateCaptureDependencies(c->stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-    PH_CUDA_CHECK(cudaStreamBeginCaptureToGraph(c->body_stream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                cudaStreamCaptureModeThreadLocal));
-    cudaStream_t outer = c->stream;
-    unsigned long long *tally = ph::t_capture_tally, inside = 0;
-    c->stream = c->body_stream;
-    ph::t_capture_tally = &inside;
-    const int rc = ph_enqueue_far(c, p);
-    ph::t_capture_tally = tally;
-    c->stream = outer;
-    c->branch_kernels = inside;
-    const cudaError_t e = cudaStreamEndCapture(c->body_stream, &body);
-    if (!rc && e != cudaSuccess) return ph_set_cuda_error(e, "cudaStreamEndCapture", __FILE__, __LINE__);
-    return rc;
-}
-
 // device part of a pass: positions already in src, accelerations to dst
 static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double *src, double *dst, int levels,
                            unsigned mask)
@@ -1145,26 +1098,17 @@ static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double
     const bool far = !(p->flags & PHOTONS_F_NO_FARFIELD);
     // the far field runs only if the walk made an M2L task (decided on the
     // device); multipoles also when the caller keeps them
-    c->branch_kernels = 0;
-    if (far && !(p->flags & PHOTONS_F_MULTIPOLES) && c->capturing) {
-        PH_TRY(capture_far_branch(c, p));
-        PH_TRY(ph_record(c, EV_FAR));
-        return ph_enqueue_gather(c, dst, p->flags & PHOTONS_F_TREE_ORDER);
-    }
     if (far || (p->flags & PHOTONS_F_MULTIPOLES))
         PH_TRY(ph::launch_far_gate(c->w.ctr, (p->flags & PHOTONS_F_MULTIPOLES) ? 1 : 0, c->far_gate, c->stream));
     if (far) {
-        PH_TRY(ph_enqueue_far(c, p));
+        PH_TRY(ph_stage_multipoles(c));
+        PH_TRY(ph_stage_m2l(c, p->precision));
+        PH_TRY(ph_stage_downward(c, p->precision));
     } else if (p->flags & PHOTONS_F_MULTIPOLES) {
         PH_TRY(ph_stage_multipoles(c));
     }
     PH_TRY(ph_record(c, EV_FAR));
     return ph_enqueue_gather(c, dst, p->flags & PHOTONS_F_TREE_ORDER);
-}
-
-static bool walk_made_m2l(const photons_ctx *c)
-{
-    return c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
 }
 
 static void drop_graph(photons_ctx *c)
@@ -1187,7 +1131,6 @@ static int capture_pass(photons_ctx *c, const photons_params *p, const double *s
     int rc = ph_enqueue_pass(c, p, src, dst, levels, mask);
     ph::t_capture_tally = nullptr;
     c->graph_kernels = tally;
-    c->graph_branch_kernels = c->branch_kernels;
     c->capturing = false;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &g);
@@ -1239,7 +1182,6 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
         long long mu_need = 0;
         int mu_over = 0;
         PH_TRY(ph_read_report(c, levels, h, &mu_need, &mu_over));
-        if (walk_made_m2l(c)) ph::g_launches += c->graph_branch_kernels;
         int grow = 0;
         PH_TRY(ph_check_build(c, h[ph::BC_FLAGS], levels, &grow));
         if (grow) { levels = grow; continue; }
@@ -1256,7 +1198,7 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
         c->info.depth_off.resize(c->info.depth + 2);
         c->have_lists = true;
         c->mask = mask;
-        const bool any_m2l = walk_made_m2l(c);
+        const bool any_m2l = c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
         c->have_multipoles = (!(p->flags & PHOTONS_F_NO_FARFIELD) && any_m2l) || (p->flags & PHOTONS_F_MULTIPOLES);
         keep_walk_hints(c, p2p_cap, pd_cap, m2l_cap);
         return 0;
@@ -1302,7 +1244,6 @@ static int capture_kdk(photons_ctx *c, const photons_params *q, int n, double *p
     if (!rc) rc = ph_enqueue_kick_dev(n, vel, acc, c->kdk_f, c->kdk_skip, st);
     ph::t_capture_tally = nullptr;
     c->kdk_kernels = tally;
-    c->kdk_branch_kernels = c->branch_kernels;
     c->capturing = false;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &g);
@@ -1374,7 +1315,6 @@ int ph_kdk_graph_step(photons_ctx *c, const photons_params *q, int n, double *po
     long long mu_need = 0;
     int mu_over = 0;
     PH_TRY(ph_read_report(c, levels, h, &mu_need, &mu_over));
-    if (walk_made_m2l(c)) ph::g_launches += c->kdk_branch_kernels;
     int grow = 0;
     PH_TRY(ph_check_build(c, h[ph::BC_FLAGS], levels, &grow));
     const unsigned long long fl = c->ws.c[ph::WC_FLAGS];
@@ -1394,7 +1334,7 @@ int ph_kdk_graph_step(photons_ctx *c, const photons_params *q, int n, double *po
     c->info.depth_off.resize(c->info.depth + 2);
     c->have_lists = true;
     c->mask = mask;
-    const bool any_m2l = walk_made_m2l(c);
+    const bool any_m2l = c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
     c->have_multipoles = (!(q->flags & PHOTONS_F_NO_FARFIELD) && any_m2l) || (q->flags & PHOTONS_F_MULTIPOLES);
     c->last_flags = q->flags;
     c->precision = q->precision;
@@ -1443,7 +1383,6 @@ extern "C" void photons_destroy(photons_ctx *c)
     free_all(c);
     for (int i = 0; i < EV_COUNT; i++) cudaEventDestroy(c->ev[i]);
     cudaStreamDestroy(c->own_stream);
-    if (c->body_stream) cudaStreamDestroy(c->body_stream);
     delete c;
 }
 

@@ -121,10 +121,6 @@ struct photons_ctx {
     bool capturing = false, have_key = false;
     cudaGraphExec_t gexec = nullptr;
     unsigned long long graph_kernels = 0;  // kernel nodes of gexec
-    // kernels of the captured far field (the body of a conditional node): of
-    // the capture in progress, and of gexec and kexec
-    unsigned long long branch_kernels = 0, graph_branch_kernels = 0, kdk_branch_kernels = 0;
-    cudaStream_t body_stream = nullptr;  // captures that body
     PassKey key{};
     // the captured kick-drift-kick step: the pass's key, velocity array and
     // box side; device factors (dkh, dd) and the flag that stops the second kick

@@ -674,16 +674,6 @@ __global__ void k_far_gate(const unsigned long long *walk_ctr, int keep_multipol
     }
 }
 
-// the same for a far field that is the body of a conditional graph node
-__global__ void k_far_branch(const unsigned long long *walk_ctr, int *gate, cudaGraphConditionalHandle branch)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const bool m2l = walk_ctr[WC_M2L_LOCAL] + walk_ctr[WC_M2L_IMAGE] > 0;
-        gate[0] = gate[1] = m2l;
-        cudaGraphSetConditional(branch, m2l ? 1u : 0u);
-    }
-}
-
 inline int grid_cap() { return device_sm_count() * 16; }
 
 inline int grid_for(long long n, int tpb)
@@ -761,13 +751,6 @@ int run_p2m_m2m(const MultipoleArgs &a, cudaStream_t st)
 int launch_far_gate(const unsigned long long *walk_ctr, int keep_multipoles, int *gate, cudaStream_t st)
 {
     ph::note_launch(), k_far_gate<<<1, 1, 0, st>>>(walk_ctr, keep_multipoles, gate);
-    PH_CUDA_CHECK(cudaGetLastError());
-    return 0;
-}
-
-int launch_far_branch(const unsigned long long *walk_ctr, int *gate, cudaGraphConditionalHandle branch, cudaStream_t st)
-{
-    ph::note_launch(), k_far_branch<<<1, 1, 0, st>>>(walk_ctr, gate, branch);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

@@ -39,8 +39,6 @@ int run_downward_f32(const MultipoleArgs &a, cudaStream_t st);
 int run_p2m_m2m(const MultipoleArgs &a, cudaStream_t st);
 // the far-field switches of a captured pass (gate[2], see MultipoleArgs)
 int launch_far_gate(const unsigned long long *walk_ctr, int keep_multipoles, int *gate, cudaStream_t st);
-// the same where the far field is the body of the conditional node `branch`
-int launch_far_branch(const unsigned long long *walk_ctr, int *gate, cudaGraphConditionalHandle branch, cudaStream_t st);
 // op: 0 m2l (in = M, inout = L, rs), 1 m2m (in = M, inout = M'), 2 l2l (in = L, inout = L')
 int launch_op_batch(int op, int n, const double *d, const double *in, double *inout, double rs, cudaStream_t st);
 
