@@ -1071,6 +1071,29 @@ int ph_stage_output(photons_ctx *c, double *acc, int device_io, int tree_order)
 // ------------------------------------------------------------------
 // the whole pass as one CUDA graph
 // ------------------------------------------------------------------
+static bool walk_made_m2l(const photons_ctx *c)
+{
+    return c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
+}
+
+// Whether the captured pass holds the far field.  Its ~45 launches only find
+// that there is nothing to do in a pass without an M2L task (72-82 us of
+// passes over 4,096 to 32,768 grid particles), so after two such passes in a
+// row it is left out; a pass that turns out to need it gets it afterwards
+// (run_far_after), and the next one holds it again.
+#define FAR_IDLE 2
+static bool capture_far(const photons_ctx *c, const photons_params *p)
+{
+    if (p->flags & PHOTONS_F_NO_FARFIELD) return false;
+    return (p->flags & PHOTONS_F_MULTIPOLES) || c->far_idle < FAR_IDLE;
+}
+
+static void note_far(photons_ctx *c)
+{
+    if (walk_made_m2l(c)) c->far_idle = 0;
+    else if (c->far_idle < FAR_IDLE) c->far_idle++;
+}
+
 static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const double *pos, double *acc, int dio,
                         int levels, unsigned mask)
 {
@@ -1079,12 +1102,34 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
     k.n = n; k.nbox = c->b.nbox; k.levels = levels; k.top = tree_top(c, levels); k.maxleaf = p->maxleaf; k.precision = p->precision; k.flags = p->flags;
     k.dio = dio; k.variant = p2p_variant(); k.nwarps = c->w.nwarps; k.mask = mask;
     k.stage_extra = stage_shortfall();
+    k.far = capture_far(c, p);
     k.boxsize = p->boxsize; k.theta = p->theta; k.rs = p->rs; k.rcut = p->rcut; k.eps = p->eps; k.mass = p->mass;
     k.pos = dio ? (const void *)pos : nullptr;
     k.acc = dio ? (const void *)acc : nullptr;
     k.stream = c->stream;
     k.epoch = c->epoch;
     return k;
+}
+
+static int ph_enqueue_far(photons_ctx *c, const photons_params *p)
+{
+    PH_TRY(ph_stage_multipoles(c));
+    PH_TRY(ph_stage_m2l(c, p->precision));
+    return ph_stage_downward(c, p->precision);
+}
+
+// the far field of a finished pass captured without it, added to its
+// accelerations, and the output again
+static int run_far_after(photons_ctx *c, const photons_params *p, int n, double *dst, double *acc, int dio, int levels)
+{
+    c->ndepth = levels + 1;
+    PH_TRY(ph_enqueue_far(c, p));
+    PH_TRY(ph_record(c, EV_FAR));
+    PH_TRY(ph_enqueue_gather(c, dst, p->flags & PHOTONS_F_TREE_ORDER));
+    if (!dio) PH_TRY(ph_copy_host(c, acc, c->io, (size_t)3 * n, false));
+    PH_TRY(ph_record(c, EV_END));
+    PH_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+    return 0;
 }
 
 // device part of a pass: positions already in src, accelerations to dst
@@ -1095,15 +1140,13 @@ static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double
     PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->ndepth, c->pp, mask, c->stream));
     PH_TRY(ph_record(c, EV_WALK));
     PH_TRY(ph_stage_p2p(c, p->precision, 1));
-    const bool far = !(p->flags & PHOTONS_F_NO_FARFIELD);
+    const bool far = capture_far(c, p);
     // the far field runs only if the walk made an M2L task (decided on the
     // device); multipoles also when the caller keeps them
     if (far || (p->flags & PHOTONS_F_MULTIPOLES))
         PH_TRY(ph::launch_far_gate(c->w.ctr, (p->flags & PHOTONS_F_MULTIPOLES) ? 1 : 0, c->far_gate, c->stream));
     if (far) {
-        PH_TRY(ph_stage_multipoles(c));
-        PH_TRY(ph_stage_m2l(c, p->precision));
-        PH_TRY(ph_stage_downward(c, p->precision));
+        PH_TRY(ph_enqueue_far(c, p));
     } else if (p->flags & PHOTONS_F_MULTIPOLES) {
         PH_TRY(ph_stage_multipoles(c));
     }
@@ -1198,7 +1241,10 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
         c->info.depth_off.resize(c->info.depth + 2);
         c->have_lists = true;
         c->mask = mask;
-        const bool any_m2l = c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
+        const bool any_m2l = walk_made_m2l(c);
+        if (any_m2l && !k.far && !(p->flags & PHOTONS_F_NO_FARFIELD))
+            PH_TRY(run_far_after(c, p, n, dst, acc, dio, levels));
+        note_far(c);
         c->have_multipoles = (!(p->flags & PHOTONS_F_NO_FARFIELD) && any_m2l) || (p->flags & PHOTONS_F_MULTIPOLES);
         keep_walk_hints(c, p2p_cap, pd_cap, m2l_cap);
         return 0;
@@ -1212,13 +1258,16 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
 namespace {
 
 // 1 when the pass just run did not fit (tree capacity, depth or levels,
-// walk pools, or a reaction buffer too small for its mutual pairs): the
+// walk pools, a reaction buffer too small for its mutual pairs, or an M2L
+// task in a pass captured without the far field): the
 // captured step's second kick then leaves the velocities alone
-__global__ void k_pass_failed(const int *tree_cnt, const unsigned long long *walk_ctr, const int *mu_over, int *out)
+__global__ void k_pass_failed(const int *tree_cnt, const unsigned long long *walk_ctr, const int *mu_over, int no_far,
+                              int *out)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0)
         *out = (tree_cnt[ph::BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH | PH_FLAG_TOP)) ||
-               walk_ctr[ph::WC_FLAGS] != 0 || *mu_over != 0;
+               walk_ctr[ph::WC_FLAGS] != 0 || *mu_over != 0 ||
+               (no_far && walk_ctr[ph::WC_M2L_LOCAL] + walk_ctr[ph::WC_M2L_IMAGE] > 0);
 }
 
 }  // namespace
@@ -1238,7 +1287,8 @@ static int capture_kdk(photons_ctx *c, const photons_params *q, int n, double *p
     if (!rc) rc = ph_enqueue_drift_dev(n, pos, vel, c->kdk_f + 1, q->boxsize, st);
     if (!rc) rc = ph_enqueue_pass(c, q, pos, acc, levels, mask);
     if (!rc) {
-        ph::note_launch(), k_pass_failed<<<1, 1, 0, st>>>(c->b.cnt, c->w.ctr, c->mu_over, c->kdk_skip);
+        ph::note_launch(), k_pass_failed<<<1, 1, 0, st>>>(
+            c->b.cnt, c->w.ctr, c->mu_over, !(q->flags & PHOTONS_F_NO_FARFIELD) && !capture_far(c, q), c->kdk_skip);
         if (cudaGetLastError() != cudaSuccess) rc = ph_set_error(PH_ERR_CUDA, "k_pass_failed launch");
     }
     if (!rc) rc = ph_enqueue_kick_dev(n, vel, acc, c->kdk_f, c->kdk_skip, st);
@@ -1318,7 +1368,9 @@ int ph_kdk_graph_step(photons_ctx *c, const photons_params *q, int n, double *po
     int grow = 0;
     PH_TRY(ph_check_build(c, h[ph::BC_FLAGS], levels, &grow));
     const unsigned long long fl = c->ws.c[ph::WC_FLAGS];
-    if (grow || fl) {
+    const bool lacks_far = !k.far && !(q->flags & PHOTONS_F_NO_FARFIELD) && walk_made_m2l(c);
+    if (lacks_far) c->far_idle = 0;
+    if (grow || fl || lacks_far) {
         // the caller's pass grows what did not fit (its own checks repeat these)
         *done = KDK_PASS_AGAIN;
         return 0;
@@ -1334,7 +1386,8 @@ int ph_kdk_graph_step(photons_ctx *c, const photons_params *q, int n, double *po
     c->info.depth_off.resize(c->info.depth + 2);
     c->have_lists = true;
     c->mask = mask;
-    const bool any_m2l = c->ws.c[ph::WC_M2L_LOCAL] + c->ws.c[ph::WC_M2L_IMAGE] > 0;
+    const bool any_m2l = walk_made_m2l(c);
+    note_far(c);
     c->have_multipoles = (!(q->flags & PHOTONS_F_NO_FARFIELD) && any_m2l) || (q->flags & PHOTONS_F_MULTIPOLES);
     c->last_flags = q->flags;
     c->precision = q->precision;

@@ -30,7 +30,7 @@ enum {
 // Everything a captured pass bakes in; a pass with a different key is
 // captured anew.  Zero-filled before use so it compares with memcmp.
 struct PassKey {
-    int n, nbox, levels, top, maxleaf, precision, flags, dio, variant, nwarps, stage_extra;
+    int n, nbox, levels, top, maxleaf, precision, flags, dio, variant, nwarps, stage_extra, far;
     unsigned mask;
     double boxsize, theta, rs, rcut, eps, mass;
     const void *pos, *acc;
@@ -120,6 +120,7 @@ struct photons_ctx {
     // the captured pass
     bool capturing = false, have_key = false;
     cudaGraphExec_t gexec = nullptr;
+    int far_idle = 0;  // captured passes in a row without an M2L task
     unsigned long long graph_kernels = 0;  // kernel nodes of gexec
     PassKey key{};
     // the captured kick-drift-kick step: the pass's key, velocity array and

@@ -436,3 +436,66 @@ def test_fp32_long_lists_split_over_a_block(ph, fp, ics, workload, nside, maxlea
     assert np.median(e) <= 1e-5, np.median(e)
     assert np.percentile(e, 99) <= 1e-4, np.percentile(e, 99)
     assert np.array_equal(a32, fp.run(pos, p, precision=ph.FP32_SPLIT, flags=ph.F_ONE_WAY))
+
+
+@pytest.mark.parametrize("device_io", [False, True])
+def test_far_field_comes_back_after_passes_without_it(ph, ics, device_io):
+    """A context leaves the far field out of its captured pass after passes
+    without an M2L task; a pass with such tasks then gives the same forces,
+    bit for bit, as on a fresh context, and so do the passes after it."""
+    torch = pytest.importorskip("torch")
+    quiet, pq = ics.make("zeldovich256", nside=24, maxleaf=16)
+    halos, p = ics.make("nfw128", nside=24, maxleaf=16)
+    halos = halos * (pq["boxsize"] / p["boxsize"])  # one box and parameter set for both
+
+    def run(f, pos):
+        if not device_io:
+            return f.run(pos, pq)
+        d.copy_(torch.from_numpy(pos))
+        torch.cuda.synchronize()
+        f.run_device(d.data_ptr(), a.data_ptr(), len(pos), pq)
+        torch.cuda.synchronize()
+        return a.cpu().numpy()
+
+    d = torch.empty((24 ** 3, 3), dtype=torch.float64, device="cuda")
+    a = torch.empty_like(d)
+    fresh, used = ph.ForcePass(0), ph.ForcePass(0)
+    want = run(fresh, halos)
+    assert fresh.counters()["n_m2l"] > 0
+    for _ in range(5):
+        run(used, quiet)
+        assert used.counters()["n_m2l"] + used.counters()["n_m2l_ext"] == 0
+    for _ in range(3):
+        assert np.array_equal(run(used, halos), want)
+
+
+def test_kdk_step_that_needs_the_far_field_again(ph, ics):
+    """The captured kick-drift-kick step after passes without the far field:
+    a step whose pass makes M2L tasks equals the step composed of single
+    calls, bit for bit."""
+    torch = pytest.importorskip("torch")
+    quiet, p = ics.make("zeldovich256", nside=24, maxleaf=16)
+    halos, ph_p = ics.make("nfw128", nside=24, maxleaf=16)
+    halos = halos * (p["boxsize"] / ph_p["boxsize"])
+    n = len(quiet)
+    pos = torch.from_numpy(quiet).cuda()
+    vel, acc = torch.zeros_like(pos), torch.zeros_like(pos)
+    step, single = ph.ForcePass(0), ph.ForcePass(0)
+    stream = torch.cuda.current_stream()
+    single.set_stream(stream.cuda_stream)
+    torch.cuda.synchronize()
+    for _ in range(6):
+        step.kdk_step_device(pos.data_ptr(), vel.data_ptr(), acc.data_ptr(), n, p, 1e-12, 0.0)
+    for _ in range(3):
+        pos.copy_(torch.from_numpy(halos))
+        q = [t.clone() for t in (pos, vel, acc)]
+        torch.cuda.synchronize()
+        step.kdk_step_device(pos.data_ptr(), vel.data_ptr(), acc.data_ptr(), n, p, 1e-9, 1e-3)
+        assert step.counters()["n_m2l"] > 0
+        ph.kick(n, q[1].data_ptr(), q[2].data_ptr(), 1e-9, stream.cuda_stream)
+        ph.drift(n, q[0].data_ptr(), q[1].data_ptr(), 1e-3, p["boxsize"], stream.cuda_stream)
+        single.run_device(q[0].data_ptr(), q[2].data_ptr(), n, p)
+        ph.kick(n, q[1].data_ptr(), q[2].data_ptr(), 1e-9, stream.cuda_stream)
+        torch.cuda.synchronize()
+        for x, y in zip((pos, vel, acc), q):
+            assert torch.equal(x, y)
