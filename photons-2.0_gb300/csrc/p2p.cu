@@ -1031,6 +1031,7 @@ __global__ void k_mu_pair(const int *tree_cnt, const unsigned long long *walk_fl
 // is evaluated one way.  The entries a target evaluates (all but the
 // received) are packed in list order into ev[off + k] = (entry, slot),
 // nev[t] of them.
+template <bool F64>
 __global__ void k_mu_slots(const int *tree_cnt, const unsigned long long *walk_flags, const uint32_t *pool,
                            const long long *off, const int *cnt, const long long *total, long long cap,
                            const int *pq, int *slot, int2 *ev, int *nev, int *over, int seg, int2 *items,
@@ -1063,7 +1064,7 @@ __global__ void k_mu_slots(const int *tree_cnt, const unsigned long long *walk_f
         }
         if (!fits && repeats) kept = 0;  // the caller repeats the pass with more room
         if (lane == 0) nev[t] = kept;
-        if (seg) {
+        if (F64) {
             // FP64: the leaf's work items, seg evaluated entries each (all in one
             // when there is no room for their slots)
             const int ni = !fits ? kept > 0 : (kept + seg - 1) / seg;
@@ -1989,9 +1990,10 @@ int launch_p2p_mutual(const P2PArgs &a, const MutualBufs &m, int fp64, cudaStrea
     PH_CUDA_CHECK(cudaMemsetAsync(a.work_counter, 0, sizeof(int), st));
     const int sms = device_sm_count();
     const int seg = fp64 ? mu64_seg(m.maxleaf) : 0;
-    ph::note_launch(), k_mu_slots<<<sms * 8, 256, 0, st>>>(a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt,
-                                                            m.total, m.buf_cap, m.pq, m.slot, m.ev, m.nev, m.over, seg,
-                                                            m.items, m.nitems, m.repeats);
+    auto slots = fp64 ? k_mu_slots<true> : k_mu_slots<false>;
+    ph::note_launch(), slots<<<sms * 8, 256, 0, st>>>(a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt, m.total,
+                                                       m.buf_cap, m.pq, m.slot, m.ev, m.nev, m.over, seg, m.items,
+                                                       m.nitems, m.repeats);
     if (fp64) {
         double *rbuf = reinterpret_cast<double *>(m.buf);
         ph::note_launch(), k_p2p_mutual64<<<sms, MU64_TB, MU64_SMEM, st>>>(a, m.ev, m.nev, m.rbase, m.nrecv, rbuf, seg,
