@@ -861,19 +861,20 @@ __device__ __forceinline__ void mu_sort_regs(uint32_t *lst, int L, int lane)
         if (32 * r + lane < L) lst[32 * r + lane] = v[r];
 }
 
+// A warp per list, in registers up to MU_SORT_MAX entries.  (Lists of 257 to
+// 1,024 sorted in shared memory, 32 KB a block, took 227 against 44 us in an
+// FP64 pass over 110,591 particles, half in halos, and 80 against 14 us at
+// 32^3 particles, leaf 16: two list reads and writes a step and few warps.)
 __global__ void __launch_bounds__(256) k_mu_sort(const int *tree_cnt, const unsigned long long *walk_flags,
                                                   uint32_t *pool, const long long *off, const int *cnt, int *sorted)
 {
-    __shared__ uint32_t s_buf[8][MU_SORT_MAX];
-    const int lane = warp_lane(), wib = threadIdx.x >> 5;
+    const int lane = warp_lane();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int nleaf = *walk_flags ? 0 : tree_cnt[BC_LEAVES];
-    uint32_t *buf = s_buf[wib];
     for (int t = gw; t < nleaf; t += nw) {
         const int L = cnt[t];
         uint32_t *lst = pool + off[t];
         const int ok = L <= MU_SORT_MAX;
-        // lists of up to 256 entries (most of them) are sorted in registers
         if (L > 1 && L <= 32) {
             mu_sort_regs<1>(lst, L, lane);
         } else if (L > 32 && L <= 64) {
@@ -882,27 +883,10 @@ __global__ void __launch_bounds__(256) k_mu_sort(const int *tree_cnt, const unsi
             mu_sort_regs<4>(lst, L, lane);
         } else if (L > 128 && L <= 256) {
             mu_sort_regs<8>(lst, L, lane);
-        } else if (ok && L > 1) {
-            int P = 2;
-            while (P < L) P <<= 1;
-            for (int i = lane; i < P; i += 32) buf[i] = i < L ? lst[i] : 0xffffffffu;
-            for (int k = 2; k <= P; k <<= 1)
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    __syncwarp();
-                    for (int i = lane; i < P; i += 32) {
-                        const int ixj = i ^ j;
-                        if (ixj > i) {
-                            const uint32_t a = buf[i], b = buf[ixj];
-                            if ((a > b) == ((i & k) == 0)) {
-                                buf[i] = b;
-                                buf[ixj] = a;
-                            }
-                        }
-                    }
-                }
-            __syncwarp();
-            for (int i = lane; i < L; i += 32) lst[i] = buf[i];
-            __syncwarp();
+        } else if (L > 256 && L <= 512) {
+            mu_sort_regs<16>(lst, L, lane);
+        } else if (L > 512 && ok) {
+            mu_sort_regs<32>(lst, L, lane);
         }
         if (lane == 0) sorted[t] = ok;
     }
@@ -1790,28 +1774,35 @@ __global__ void __launch_bounds__(MU64_TB, 1) k_p2p_mutual64(P2PArgs A, const in
 
 // Each leaf adds the partial sums of its own work items, then the reactions
 // its owners left in its slots, in order: received entry k at
-// rbase + 3 k r, item i at rbase + 3 (nrecv + i) r.  With the reaction
-// buffer too small (over) the items added their sums themselves.
-__global__ void k_mu_gather64(P2PArgs A, const int *over, const int *nrecv, const int *nev, int seg,
-                              const long long *rbase, const double *rbuf)
+// rbase + 3 k r, item i at rbase + 3 (nrecv + i) r.  A block per leaf, its
+// warps contiguous parts of the slots, combined in order (halo leaves have
+// thousands: a warp per leaf took 1.29 ms of a pass over 110,591 particles,
+// half in halos, a block 0.67 ms).  With the reaction buffer too small (over) the items added
+// their sums themselves.
+#define GATHER64_TB 256
+__global__ void __launch_bounds__(GATHER64_TB) k_mu_gather64(P2PArgs A, const int *over, const int *nrecv,
+                                                             const int *nev, int seg, const long long *rbase,
+                                                             const double *rbuf)
 {
-    const int lane = warp_lane();
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    constexpr int NW = GATHER64_TB / 32;
+    __shared__ double s_sum[NW][3][32];
+    const int lane = warp_lane(), warp = threadIdx.x >> 5;
     const int nleaf = *over ? 0 : p2p_targets(A);
-    for (int t = gw; t < nleaf; t += nw) {
+    for (int t = blockIdx.x; t < nleaf; t += gridDim.x) {
         const int nt = A.npart[t], it = A.ipart[t], nr = nrecv[t], all = nr + (nev[t] + seg - 1) / seg;
-        if (all == 0 || nt == 0) continue;
+        if (all == 0 || nt == 0) continue;  // the same for the whole block
         const int rl = mu_row_g(nt, MU64_ROW);
         const double *base = rbuf + rbase[t];
         // rows of at most 16 doubles: two or more slots at a time, a subset of lanes each
-        const int wide = nt <= 8 ? 8 : (nt <= 16 ? 16 : 32), ways = 32 / wide;
-        const int way = lane / wide;
+        const int wide = nt <= 4 ? 4 : (nt <= 8 ? 8 : (nt <= 16 ? 16 : 32)), ways = 32 / wide;
+        const int way = lane / wide, per = (all + NW - 1) / NW;
+        const int first = min(all, warp * per), last = min(all, first + per);
         for (int j0 = 0; j0 < nt; j0 += wide) {
             const int j = j0 + lane % wide;
             double v0 = 0.0, v1 = 0.0, v2 = 0.0;
             if (j < nt) {
 #pragma unroll 4
-                for (int i = way; i < all; i += ways) {
+                for (int i = first + way; i < last; i += ways) {
                     const int k = i + nr < all ? i + nr : i + nr - all;  // own items first
                     const double *src = base + (long long)k * 3 * rl + j;
                     v0 += src[0];
@@ -1824,10 +1815,18 @@ __global__ void k_mu_gather64(P2PArgs A, const int *over, const int *nrecv, cons
                 v1 += shfl_xor_d(v1, o);
                 v2 += shfl_xor_d(v2, o);
             }
-            if (way == 0 && j < nt) {
-                A.ax[it + j] += v0;
-                A.ay[it + j] += v1;
-                A.az[it + j] += v2;
+            __syncthreads();  // the sums before have been read
+            if (way == 0) {
+                s_sum[warp][0][lane] = v0;
+                s_sum[warp][1][lane] = v1;
+                s_sum[warp][2][lane] = v2;
+            }
+            __syncthreads();
+            if (warp < 3 && lane < wide && j0 + lane < nt) {
+                double v = 0.0;
+#pragma unroll
+                for (int w = 0; w < NW; w++) v += s_sum[w][warp][lane];
+                (warp == 0 ? A.ax : (warp == 1 ? A.ay : A.az))[it + j0 + lane] += v;
             }
         }
     }
@@ -1943,11 +1942,12 @@ static int launch_mutual_build(const P2PArgs &a, const MutualBufs &m, int shape,
 // entries per FP64 work item: about 32k pairs of full leaves (a scheduler's
 // FP64 pipe takes ~0.2 ms for them), so that no item is long against the
 // kernel and a leaf of a halo, with thousands of entries, spreads over the
-// chip; at most 256
+// chip; at most 64 (32^3 particles, leaf 16, a periodic box and its images:
+// 1.56 ms in the pair kernel at 128 entries, 1.21 ms at 64)
 int mu64_seg(int maxleaf)
 {
     const int s = 32768 / (maxleaf * maxleaf);
-    return s < 2 ? 2 : (s > 256 ? 256 : s);
+    return s < 2 ? 2 : (s > 64 ? 64 : s);
 }
 
 // shared memory above the 48 KB default, allowed once per device
@@ -1998,7 +1998,7 @@ int launch_p2p_mutual(const P2PArgs &a, const MutualBufs &m, int fp64, cudaStrea
         double *rbuf = reinterpret_cast<double *>(m.buf);
         ph::note_launch(), k_p2p_mutual64<<<sms, MU64_TB, MU64_SMEM, st>>>(a, m.ev, m.nev, m.rbase, m.nrecv, rbuf, seg,
                                                                            m.items, m.nitems, m.over);
-        ph::note_launch(), k_mu_gather64<<<sms * 4, 256, 0, st>>>(a, m.over, m.nrecv, m.nev, seg, m.rbase, rbuf);
+        ph::note_launch(), k_mu_gather64<<<sms * 8, GATHER64_TB, 0, st>>>(a, m.over, m.nrecv, m.nev, seg, m.rbase, rbuf);
         PH_CUDA_CHECK(cudaGetLastError());
         return 0;
     }
