@@ -242,6 +242,8 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
     const int parity = A.depth & 1;
     const int nleaf = A.tree_cnt[BC_LEAVES];
     const int list_begin = A.depth_off[A.depth], list_end = A.depth_off[A.depth + 1];
+    if (list_begin >= list_end) return;  // below the tree
+    bool any = false;                    // whether this warp had a target
     unsigned long long c_p2p_loc = 0, c_p2p_img = 0, c_m2l_loc = 0, c_m2l_img = 0, c_pl = 0, c_pi = 0;
     unsigned flags = 0;
     int max_stack = 0, max_stage = 0;
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         if (lane == 0) tk = atomicAdd(&W.ctr[WC_WORK0 + parity], 1ULL);
         const long long ti = list_begin + (long long)__shfl_sync(0xffffffffu, tk, 0);
         if (ti >= list_end) break;
+        any = true;
         const int a = A.depth_list[ti];
         const bool leaf_a = a < nleaf;
         // the target's box: its root (the receiving domain of the image
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         }
         __syncwarp();
     }
+    if (!any) return;
     // per-warp counters
     c_p2p_loc = warp_sum_ll(c_p2p_loc);
     c_p2p_img = warp_sum_ll(c_p2p_img);
