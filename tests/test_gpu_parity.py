@@ -499,3 +499,26 @@ def test_kdk_step_that_needs_the_far_field_again(ph, ics):
         torch.cuda.synchronize()
         for x, y in zip((pos, vel, acc), q):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n,maxleaf", [(1024, 8), (1025, 1), (2049, 8), (7168, 16), (7169, 16), (14337, 4),
+                                       (30011, 1), (60000, 40)])
+def test_tree_around_the_split_sizes_matches_oracle(ph, fp, port, n, maxleaf):
+    """Trees whose upper nodes lie around the sizes at which a node is split
+    by one block (1,024 and 7,168 particles): permutation, numbering and lists
+    exactly the oracle's."""
+    rng = np.random.default_rng(n)
+    p = dict(boxsize=100.0, theta=0.5, rs=4.0, rcut=18.0, eps=0.1, mass=1.0, maxleaf=maxleaf)
+    pos = rng.uniform(0.0, 100.0, (n, 3))
+    pos[: n // 2] = np.mod(rng.normal(37.0, 4.0, (n // 2, 3)), 100.0)  # half in one clump
+    r = port.run(pos, p, capture=True, tree=True, nthreads=8)
+    fp.run(pos, p, precision=ph.FP64, flags=ph.F_TREE_ORDER | ph.F_KEEP_LISTS)
+    c = fp.counters()
+    for k in COUNTERS[:10]:
+        assert c[k] == r["counters"][k], k
+    assert np.array_equal(fp.positions(), r["pos"])
+    for kind, (t, s, im) in fp.lists().items():
+        assert digest(t, s, im) == digest(*(np.asarray(x) for x in r["lists"][kind])), kind
+    tr = fp.tree()
+    for k in ("leaf_ipart", "leaf_npart", "node_npart", "node_son"):
+        assert np.array_equal(tr[k], r["tree"][k]), k

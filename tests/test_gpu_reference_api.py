@@ -213,3 +213,14 @@ def test_direct_sum_filter_keeps_every_source(ph, n, rmax, eps, reach):
         want = (f[:, None] * d[on]).sum(0)
         scale = (np.abs(f)[:, None] * np.abs(d[on])).sum() + 1e-300
         assert np.abs(got[k] - want).max() <= 1e-13 * scale, (n, t)
+
+
+@pytest.mark.parametrize("ntarget", [1, 9, 4096, 4097])
+def test_direct_sum_slices_and_bins_match_oracle(ph, port, ics, ntarget):
+    """The direct sum with the sources in several slices (few targets) and
+    over binned sources (more than 4,096): the bar of the direct sum above."""
+    pos, p = ics.make("nfw128", nside=32)
+    targets = np.random.default_rng(5).choice(pos.shape[0], ntarget, replace=False).astype(np.int32)
+    got = ph.direct_sum(pos, p, targets)
+    want = port.direct_sum(pos, p, targets, nthreads=8)
+    assert rel_err(got, want, p).max() <= 1e-10
