@@ -133,6 +133,39 @@ inline void note_launch()
     else g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+// Kernels of a chain (tree levels, walk levels, far-field depths: dozens of
+// launches of a few microseconds each) are launched with programmatic stream
+// serialization: a kernel's blocks may be set up while the kernel before it
+// in the stream runs, and chain_begin(), the first statement of every such
+// kernel, waits until that kernel has finished and its writes are visible.
+// Each kernel of a chain waits for the one before it, so all earlier work is
+// done too.  Kernels with const __restrict__ or __ldg loads, which the
+// compiler may move above the wait, are launched with <<<>>>.
+__device__ __forceinline__ void chain_begin()
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
+template <class... P, class... A>
+inline void chain(void (*kernel)(P...), int grid, int block, size_t shared, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    note_launch();
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // checked by the callers' cudaGetLastError
+}
+
 // exclusive scan of n int32 values (n read on the device from n_ptr, at most
 // cap elements); writes total to *total (device) if total != nullptr.
 void scan_exclusive_i32(const int *in, int *out, const int *n_ptr, int cap, int *total, int *scratch,

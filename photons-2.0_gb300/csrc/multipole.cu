@@ -222,6 +222,7 @@ __global__ void k_m2m_depth(const int *list, const int *depth_off, int d, const 
                             const int *son1, const double *cx, const double *cy, const double *cz, double *M,
                             const int *gate)
 {
+    ph::chain_begin();
     if (gate && !*gate) return;
     const int begin = depth_off[d], end = depth_off[d + 1], nleaf = tree_cnt[BC_LEAVES];
     if (begin == end) return;
@@ -383,6 +384,7 @@ __global__ void __launch_bounds__(MP_TB) k_m2l(const int *tree_cnt, const unsign
 __global__ void k_l2l_depth(const int *list, const int *depth_off, int d, const int *parent, const double *cx,
                             const double *cy, const double *cz, double *L, const int *gate)
 {
+    ph::chain_begin();
     if (gate && !*gate) return;
     const int begin = depth_off[d], end = depth_off[d + 1];
     if (begin == end) return;
@@ -657,6 +659,7 @@ __global__ void k_l2p_f32(const float4 *pos4, const int *ipart, const int *npart
 // zero the local expansions of every unified id
 __global__ void k_zero_L(double *L, const int *tree_cnt, const int *gate)
 {
+    ph::chain_begin();
     if (gate && !*gate) return;
     const long long n = (long long)(tree_cnt[BC_LEAVES] + tree_cnt[BC_NODES]) * PH_NMULTI;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -700,7 +703,7 @@ int run_m2l(const MultipoleArgs &a, cudaStream_t st)
 static void launch_l2l(const MultipoleArgs &a, cudaStream_t st)
 {
     for (int d = 1; d < a.ndepth; d++)
-        ph::note_launch(), k_l2l_depth<<<device_sm_count() * 8, MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.parent, a.cx, a.cy,
+        ph::chain(k_l2l_depth, device_sm_count() * 8, MP_TB, 0, st, a.depth_list, a.depth_off, d, a.parent, a.cx, a.cy,
                                                                        a.cz, a.L, a.gate_l);
 }
 
@@ -741,9 +744,9 @@ int run_p2m_m2m(const MultipoleArgs &a, cudaStream_t st)
     ph::note_launch(), k_p2m<<<grid_cap(), MP_TB, 0, st>>>(a.px, a.py, a.pz, a.ipart, a.npart, a.cx, a.cy, a.cz,
                                                              a.tree_cnt, a.boxid, a.boxes, a.M, a.gate_m);
     for (int d = a.ndepth - 1; d >= 0; d--)
-        ph::note_launch(), k_m2m_depth<<<device_sm_count() * 8, MP_TB, 0, st>>>(a.depth_list, a.depth_off, d, a.tree_cnt, a.son0,
+        ph::chain(k_m2m_depth, device_sm_count() * 8, MP_TB, 0, st, a.depth_list, a.depth_off, d, a.tree_cnt, a.son0,
                                                                        a.son1, a.cx, a.cy, a.cz, a.M, a.gate_m);
-    ph::note_launch(), k_zero_L<<<grid_cap(), 256, 0, st>>>(a.L, a.tree_cnt, a.gate_m);
+    ph::chain(k_zero_L, grid_cap(), 256, 0, st, a.L, a.tree_cnt, a.gate_m);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

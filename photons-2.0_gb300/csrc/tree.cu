@@ -96,6 +96,7 @@ __device__ __forceinline__ int open_mode(const BuildBufs &b, int len)
 
 __global__ void k_init_roots(BuildBufs b, int n, int top)
 {
+    ph::chain_begin();
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < b.nbox; t += gridDim.x * blockDim.x) {
         const BoxParams &B = b.boxes[t];
         b.tn_start[t] = B.first;
@@ -147,6 +148,7 @@ __device__ __forceinline__ void level_nch_node(BuildBufs &b, int lb, int i)
 
 __global__ void k_level_nch(BuildBufs b)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN], C = b.cnt[BC_LEVEL_COUNT];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) level_nch_node(b, lb, i);
 }
@@ -160,6 +162,7 @@ __device__ __forceinline__ void chunk_map_node(BuildBufs &b, int i, int lane)
 
 __global__ void k_chunk_map(BuildBufs b)
 {
+    ph::chain_begin();
     const int C = b.cnt[BC_LEVEL_COUNT];
     int lane = warp_lane();
     int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -171,6 +174,7 @@ __global__ void k_chunk_map(BuildBufs b)
 // of the adds, which keep their order.
 __global__ void k_chunk_sum(BuildBufs b, int D)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN];
     const double *coord = axis_ptr(b.x, b.y, b.z, D);
     int W = b.cnt[BC_W];
@@ -202,6 +206,7 @@ __global__ void k_chunk_sum(BuildBufs b, int D)
 // warp reduction (fixed order)
 __global__ void k_node_mean(BuildBufs b, int D)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN], C = b.cnt[BC_LEVEL_COUNT];
     int lane = warp_lane();
     int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -219,6 +224,7 @@ __global__ void k_node_mean(BuildBufs b, int D)
 
 __global__ void k_chunk_count(BuildBufs b, int D)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN];
     const double *coord = axis_ptr(b.x, b.y, b.z, D);
     int W = b.cnt[BC_W];
@@ -298,6 +304,7 @@ __device__ __forceinline__ void node_split_node(BuildBufs &b, int lb, int i, int
 
 __global__ void k_node_split(BuildBufs b, int maxleaf)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN], C = b.cnt[BC_LEVEL_COUNT];
     int lane = warp_lane();
     int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -375,6 +382,7 @@ __device__ __forceinline__ void make_children_node(BuildBufs &b, int lb, int C, 
 
 __global__ void k_make_children(BuildBufs b, int maxleaf, int D)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN], C = b.cnt[BC_LEVEL_COUNT];
     const int leaves_before = b.cnt[BC_LEAVES];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x)
@@ -409,6 +417,7 @@ __device__ void level_finish(BuildBufs &b, int d, int top)
 
 __global__ void k_level_finish(BuildBufs b, int d, int top)
 {
+    ph::chain_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) level_finish(b, d, top);
 }
 
@@ -448,6 +457,7 @@ __device__ int block_scan_excl(const int *in, int *out, int n, int *s_warp)
 
 __global__ void __launch_bounds__(SMALL_TB) k_level_plan(BuildBufs b, int finish_prev, int top)
 {
+    ph::chain_begin();
     __shared__ int s_warp[33];
     if (finish_prev >= 0 && threadIdx.x == 0) level_finish(b, finish_prev, top);
     __syncthreads();
@@ -462,6 +472,7 @@ __global__ void __launch_bounds__(SMALL_TB) k_level_plan(BuildBufs b, int finish
 
 __global__ void __launch_bounds__(SMALL_TB) k_level_close(BuildBufs b, int maxleaf, int D)
 {
+    ph::chain_begin();
     __shared__ int s_warp[33];
     const int lb = b.cnt[BC_LEVEL_BEGIN], C = b.cnt[BC_LEVEL_COUNT];
     const int lane = warp_lane();
@@ -483,6 +494,7 @@ __global__ void __launch_bounds__(SMALL_TB) k_level_close(BuildBufs b, int maxle
 // no work and reads nothing stale.
 __global__ void k_tree_totals(BuildBufs b)
 {
+    ph::chain_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (b.cnt[BC_LEVEL_COUNT] > 0) b.cnt[BC_FLAGS] |= PH_FLAG_TOP;
         b.cnt[BC_NODES] = b.cnt[BC_LEVEL_BEGIN] + b.cnt[BC_MID_NODES] + b.cnt[BC_SUB_NODES];
@@ -508,6 +520,7 @@ __global__ void k_tree_totals(BuildBufs b)
 // per chunk.
 __global__ void k_rank(BuildBufs b, int D)
 {
+    ph::chain_begin();
     const int lb = b.cnt[BC_LEVEL_BEGIN];
     const double *coord = axis_ptr(b.x, b.y, b.z, D);
     int W = b.cnt[BC_W];
@@ -566,6 +579,7 @@ __global__ void k_rank(BuildBufs b, int D)
 // stores any.
 __global__ void k_swap(BuildBufs b, int D)
 {
+    ph::chain_begin();
     int W = b.cnt[BC_W];
     int lane = warp_lane();
     int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -628,6 +642,7 @@ static_assert(PH_MID / CHUNK <= 8 && PH_MID / MID_SEG <= 32, "one warp holds a n
 
 __global__ void __launch_bounds__(MID_TB, 1) k_mid_build(BuildBufs b, int axis0, int maxleaf, int levels)
 {
+    ph::chain_begin();
     extern __shared__ __align__(16) unsigned char mid_smem[];
     MidTree &s = *reinterpret_cast<MidTree *>(mid_smem);
     if (b.cnt[BC_LEVEL_COUNT] > 0 || (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY))) return;
@@ -919,6 +934,7 @@ __device__ void sub_split_node(SubTree &s, int i, int depth, int L, int lend, in
 // during level L.  So one barrier per level.
 __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0, int maxleaf, int levels)
 {
+    ph::chain_begin();
     extern __shared__ __align__(16) unsigned char sub_smem[];
     SubTree &s = *reinterpret_cast<SubTree *>(sub_smem);
     if (b.cnt[BC_LEVEL_COUNT] > 0 || (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY))) return;
@@ -1066,6 +1082,7 @@ __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0
 // src/fmm.c:101-118.)
 __global__ void k_mark_leaves(BuildBufs b)
 {
+    ph::chain_begin();
     const int nleaves = b.cnt[BC_LEAVES];
     for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nleaves; l += gridDim.x * blockDim.x) {
         const int p = b.tl_start[l];
@@ -1087,6 +1104,7 @@ __device__ __forceinline__ int scan_value(const int *w, const int *d, const int 
 
 __global__ void k_scan_input(const int *n_ptr, const int *w, const int *d, const int *t, int *out)
 {
+    ph::chain_begin();
     const int n = *n_ptr;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         out[i] = scan_value(w, d, t, i);
@@ -1098,6 +1116,7 @@ __global__ void k_scan_input(const int *n_ptr, const int *w, const int *d, const
 __global__ void __launch_bounds__(ONE_SCAN_TB) k_scan_one(const int *n_ptr, const int *w, const int *d, const int *t,
                                                           int *out)
 {
+    ph::chain_begin();
     __shared__ int s_warp[33];
     const int lane = warp_lane(), warp = threadIdx.x >> 5, n = *n_ptr;
     int carry = 0;
@@ -1133,6 +1152,7 @@ __global__ void __launch_bounds__(ONE_SCAN_TB) k_scan_one(const int *n_ptr, cons
 // node or leaf that starts where it does
 __global__ void k_leaf_ranks(BuildBufs b)
 {
+    ph::chain_begin();
     const int nleaves = b.cnt[BC_LEAVES], nnodes = b.cnt[BC_NODES];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nleaves + nnodes; i += gridDim.x * blockDim.x) {
         const bool leaf = i < nleaves;
@@ -1173,6 +1193,7 @@ __device__ __forceinline__ int child_id(const BuildBufs &b, int code, int nleave
 // temp nodes and leaves into the unified index space
 __global__ void k_scatter_tree(BuildBufs b, TreeBufs T)
 {
+    ph::chain_begin();
     const int nnodes = b.cnt[BC_NODES], nleaves = b.cnt[BC_LEAVES];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nleaves + nnodes; i += gridDim.x * blockDim.x) {
         if (i < nleaves) {
@@ -1210,6 +1231,7 @@ __global__ void k_scatter_tree(BuildBufs b, TreeBufs T)
 // per depth.
 __global__ void __launch_bounds__(32) k_depth_count(BuildBufs b, TreeBufs T, int ndepth)
 {
+    ph::chain_begin();
     __shared__ int h[PH_MAX_DEPTH_CAP + 2];
     const int nu = b.cnt[BC_NODES] + b.cnt[BC_LEAVES], nblk = gridDim.x, k = blockIdx.x, lane = threadIdx.x;
     for (int d = lane; d < ndepth; d += 32) h[d] = 0;
@@ -1227,6 +1249,7 @@ __global__ void __launch_bounds__(32) k_depth_count(BuildBufs b, TreeBufs T, int
 
 __global__ void __launch_bounds__(32) k_depth_place(BuildBufs b, TreeBufs T, int ndepth)
 {
+    ph::chain_begin();
     __shared__ int cur[PH_MAX_DEPTH_CAP + 2];
     const int nu = b.cnt[BC_NODES] + b.cnt[BC_LEAVES], nblk = gridDim.x, k = blockIdx.x, lane = threadIdx.x;
     const unsigned lt = (1u << lane) - 1u;
@@ -1305,7 +1328,8 @@ int build_tree(BuildBufs &b, TreeBufs &T, const PassParams &p, int n, int levels
                                            (int)sizeof(MidTree)));
         if (dev >= 0 && dev < 64) done[dev].store(true);
     }
-    ph::note_launch(), k_init_roots<<<(b.nbox + TB - 1) / TB, TB, 0, st>>>(b, n, top);
+    PH_CUDA_CHECK(cudaMemsetAsync(b.words, 0, sizeof(int) * (size_t)((n + 31) / 32), st));
+    ph::chain(k_init_roots, (b.nbox + TB - 1) / TB, TB, 0, st, b, n, top);
     // a level has at most nbox 2^d nodes: the first levels are small enough for
     // single-block bookkeeping (7 launches a level instead of 19)
     bool pending = false;  // a small level whose k_level_finish is still to come
@@ -1317,66 +1341,65 @@ int build_tree(BuildBufs &b, TreeBufs &T, const PassParams &p, int n, int levels
         const int D = (p.axis0 + d) % 3;  // from direct_local_start; the axis cycles (src/fmm.c:99)
         const bool small = d < 24 && ((long long)b.nbox << d) <= SMALL_LEVEL;
         if (small) {
-            ph::note_launch(), k_level_plan<<<1, SMALL_TB, 0, st>>>(b, pending ? d - 1 : -1, top);
+            ph::chain(k_level_plan, 1, SMALL_TB, 0, st, b, pending ? d - 1 : -1, top);
         } else {
-            if (pending) ph::note_launch(), k_level_finish<<<1, 1, 0, st>>>(b, d - 1, top);
-            ph::note_launch(), k_level_nch<<<maxb, TB, 0, st>>>(b);
+            if (pending) ph::chain(k_level_finish, 1, 1, 0, st, b, d - 1, top);
+            ph::chain(k_level_nch, maxb, TB, 0, st, b);
             scan_exclusive_i32_bounded(b.tn_nch, b.tn_chunk_base, b.cnt + BC_LEVEL_COUNT, b.cap_nodes, lvl_max,
                                        b.cnt + BC_W, b.scan_scratch, b.scan_scratch_elems, st);
-            ph::note_launch(), k_chunk_map<<<maxb, TB, 0, st>>>(b);
+            ph::chain(k_chunk_map, maxb, TB, 0, st, b);
         }
-        ph::note_launch(), k_chunk_sum<<<maxb, TB, 0, st>>>(b, D);
-        ph::note_launch(), k_node_mean<<<maxb, TB, 0, st>>>(b, D);
-        ph::note_launch(), k_chunk_count<<<maxb, TB, 0, st>>>(b, D);
+        ph::chain(k_chunk_sum, maxb, TB, 0, st, b, D);
+        ph::chain(k_node_mean, maxb, TB, 0, st, b, D);
+        ph::chain(k_chunk_count, maxb, TB, 0, st, b, D);
         if (small) {
-            ph::note_launch(), k_level_close<<<1, SMALL_TB, 0, st>>>(b, p.maxleaf, D);
+            ph::chain(k_level_close, 1, SMALL_TB, 0, st, b, p.maxleaf, D);
         } else {
-            ph::note_launch(), k_node_split<<<maxb, TB, 0, st>>>(b, p.maxleaf);
+            ph::chain(k_node_split, maxb, TB, 0, st, b, p.maxleaf);
             scan_exclusive_i32_bounded(b.tn_nodeflag, b.tn_nodebase, b.cnt + BC_LEVEL_COUNT, b.cap_nodes, lvl_max,
                                        b.cnt + BC_NEXT_NODES, b.scan_scratch, b.scan_scratch_elems, st);
             scan_exclusive_i32_bounded(b.tn_leafflag, b.tn_leafbase, b.cnt + BC_LEVEL_COUNT, b.cap_nodes, lvl_max,
                                        b.cnt + BC_NEW_LEAVES, b.scan_scratch, b.scan_scratch_elems, st);
-            ph::note_launch(), k_make_children<<<maxb, TB, 0, st>>>(b, p.maxleaf, D);
+            ph::chain(k_make_children, maxb, TB, 0, st, b, p.maxleaf, D);
         }
-        ph::note_launch(), k_rank<<<maxb, TB, 0, st>>>(b, D);
-        ph::note_launch(), k_swap<<<maxb, TB, 0, st>>>(b, D);
+        ph::chain(k_rank, maxb, TB, 0, st, b, D);
+        ph::chain(k_swap, maxb, TB, 0, st, b, D);
         if (small) {
             pending = true;
         } else {
-            ph::note_launch(), k_level_finish<<<1, 1, 0, st>>>(b, d, top);
+            ph::chain(k_level_finish, 1, 1, 0, st, b, d, top);
             pending = false;
         }
     }
-    if (pending) ph::note_launch(), k_level_finish<<<1, 1, 0, st>>>(b, top - 1, top);
+    if (pending) ph::chain(k_level_finish, 1, 1, 0, st, b, top - 1, top);
     if (b.mid > CHUNK)
-        ph::note_launch(), k_mid_build<<<device_sm_count(), MID_TB, sizeof(MidTree), st>>>(b, p.axis0, p.maxleaf, levels);
-    ph::note_launch(), k_subtree_build<<<device_sm_count() * 4, SUB_TB, sizeof(SubTree), st>>>(b, p.axis0, p.maxleaf,
+        ph::chain(k_mid_build, device_sm_count(), MID_TB, sizeof(MidTree), st, b, p.axis0, p.maxleaf, levels);
+    ph::chain(k_subtree_build, device_sm_count() * 4, SUB_TB, sizeof(SubTree), st, b, p.axis0, p.maxleaf,
                                                                                                 levels);
-    PH_CUDA_CHECK(cudaMemsetAsync(b.words, 0, sizeof(int) * (size_t)((n + 31) / 32), st));
-    ph::note_launch(), k_tree_totals<<<1, 1, 0, st>>>(b);
-    ph::note_launch(), k_mark_leaves<<<maxb, TB, 0, st>>>(b);
+    ph::chain(k_tree_totals, 1, 1, 0, st, b);
+    ph::chain(k_mark_leaves, maxb, TB, 0, st, b);
     // leaf starts before each word of 32 positions, then nodes before each leaf
     const int nwords = (n + 31) / 32;
     if (nwords <= ONE_SCAN_MAX) {
-        ph::note_launch(), k_scan_one<<<1, ONE_SCAN_TB, 0, st>>>(b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.wordpre);
+        ph::chain(k_scan_one, 1, ONE_SCAN_TB, 0, st, b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.wordpre);
     } else {
-        ph::note_launch(), k_scan_input<<<maxb, TB, 0, st>>>(b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.bigpos);
+        ph::chain(k_scan_input, maxb, TB, 0, st, b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.bigpos);
         scan_exclusive_i32(b.bigpos, b.wordpre, b.cnt + BC_WORDS, nwords, b.cnt + BC_SCAN_TOTAL, b.scan_scratch,
                            b.scan_scratch_elems, st);
     }
-    ph::note_launch(), k_leaf_ranks<<<maxb, TB, 0, st>>>(b);
+    ph::chain(k_leaf_ranks, maxb, TB, 0, st, b);
     if (b.rule_cap <= ONE_SCAN_MAX) {
-        ph::note_launch(), k_scan_one<<<1, ONE_SCAN_TB, 0, st>>>(b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.lf_base);
+        ph::chain(k_scan_one, 1, ONE_SCAN_TB, 0, st, b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.lf_base);
     } else {
-        ph::note_launch(), k_scan_input<<<maxb, TB, 0, st>>>(b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.bigpos);
+        ph::chain(k_scan_input, maxb, TB, 0, st, b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.bigpos);
         scan_exclusive_i32(b.bigpos, b.lf_base, b.cnt + BC_LEAVES, b.rule_cap, b.cnt + BC_SCAN_TOTAL, b.scan_scratch,
                            b.scan_scratch_elems, st);
     }
-    ph::note_launch(), k_scatter_tree<<<maxb, TB, 0, st>>>(b, T);
-    ph::note_launch(), k_depth_count<<<nblk, 32, 0, st>>>(b, T, ndepth);
+    ph::chain(k_scatter_tree, maxb, TB, 0, st, b, T);
+    ph::chain(k_depth_count, nblk, 32, 0, st, b, T, ndepth);
     scan_exclusive_i32(T.depth_blk, T.depth_blk + (size_t)ndepth * nblk, b.cnt + BC_DEPTH_CELLS, ndepth * nblk,
                        b.cnt + BC_DEPTH_TOTAL, b.scan_scratch, b.scan_scratch_elems, st);
-    ph::note_launch(), k_depth_place<<<nblk, 32, 0, st>>>(b, T, ndepth);
+    ph::chain(k_depth_place, nblk, 32, 0, st, b, T, ndepth);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

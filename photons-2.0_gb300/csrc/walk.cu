@@ -214,6 +214,7 @@ __device__ __forceinline__ uint32_t get2(const uint32_t *s, int scap, const uint
 template <int MINB>
 __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
 {
+    ph::chain_begin();
     const Geo &g = A.g;
     WalkBufs &W = A.w;
     const int lane = warp_lane();
@@ -514,6 +515,7 @@ __global__ void k_geom32(const double *cx, const double *cy, const double *cz, c
                          const double *wz, const double *wsum, const int *son0, const int *son1, const int *tree_cnt, float4 *chi,
                          float4 *clo, float4 *w32, int2 *son2)
 {
+    ph::chain_begin();
     const int nu = tree_cnt[BC_LEAVES] + tree_cnt[BC_NODES];
     for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += gridDim.x * blockDim.x) {
         son2[u] = make_int2(son0[u], son1[u]);
@@ -530,7 +532,7 @@ __global__ void k_geom32(const double *cx, const double *cy, const double *cz, c
 int launch_geom32(const TreeBufs &t, const int *tree_cnt, cudaStream_t st)
 {
     const int blocks = device_sm_count() * 8;
-    ph::note_launch(), k_geom32<<<blocks, 256, 0, st>>>(t.cx, t.cy, t.cz, t.wx, t.wy, t.wz, t.wsum, t.son0, t.son1, tree_cnt,
+    ph::chain(k_geom32, blocks, 256, 0, st, t.cx, t.cy, t.cz, t.wx, t.wy, t.wz, t.wsum, t.son0, t.son1, tree_cnt,
                                                     t.chi, t.clo, t.w32, t.son2);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
@@ -566,9 +568,9 @@ int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxPar
     for (int d = 0; d < ndepth; d++) {
         A.depth = d;
         if (w.nwarps == device_sm_count() * 3 * 8)
-            ph::note_launch(), k_walk_level<3><<<blocks, WALK_TB, 0, st>>>(A);
+            ph::chain(k_walk_level<3>, blocks, WALK_TB, 0, st, A);
         else
-            ph::note_launch(), k_walk_level<2><<<blocks, WALK_TB, 0, st>>>(A);
+            ph::chain(k_walk_level<2>, blocks, WALK_TB, 0, st, A);
     }
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
