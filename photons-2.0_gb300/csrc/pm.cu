@@ -10,27 +10,24 @@
 //   3. a 4-point finite-difference gradient of psi per mesh cell
 //      (src/partmesh.c:524-735) and its CIC interpolation to the particles:
 //      acc_pm = grad psi (src/partmesh.c:574-587).
-// The mesh arithmetic is FP64 in the reference's order, every product and
-// sum rounded on its own except the interpolation sums (fused multiply-adds);
-// the constant pi is the reference's: conv.f90 declares
-// `real*8, parameter :: M_PI = 3.1415926`, a default (single-precision)
-// real literal, so its value is 3.1415926 rounded to FP32 (3.141592502593994).
+// The Green's function and the transforms are FP64; the weights, the gradient
+// and the interpolation sums are 64-bit integers that resolve more than a
+// double's 53 bits of what they are added to.  The constant pi is the
+// reference's: conv.f90 declares `real*8, parameter :: M_PI = 3.1415926`, a
+// default (single-precision) real literal, so its value is 3.1415926 rounded
+// to FP32 (3.141592502593994).
 // The deposit adds with FP64 atomics, so its summation order (and the last
 // bits of the density) varies from run to run.
 #include <cufft.h>
 
 #include <cmath>
+#include <cstring>
 
 #include "api_internal.cuh"
 
 namespace {
 
 constexpr double PM_PI = (double)3.1415926f;  // src/conv.f90:171
-
-struct Cic {
-    int i, j, k, ii, jj, kk;
-    double wi, wj, wk, win, wjn, wkn;
-};
 
 __device__ __forceinline__ int wrap(int a, int N) { return a < 0 ? a + N : (a >= N ? a - N : a); }
 
@@ -52,42 +49,135 @@ __device__ __forceinline__ void cic_axis(double x, double norm, double delta, in
     cn = wrap(cn, N);
 }
 
-__device__ __forceinline__ Cic cic(const double *pos, int p, double norm, double delta, int N)
-{
-    Cic s;
-    cic_axis(pos[3 * (size_t)p], norm, delta, N, s.i, s.ii, s.wi, s.win);
-    cic_axis(pos[3 * (size_t)p + 1], norm, delta, N, s.j, s.jj, s.wj, s.wjn);
-    cic_axis(pos[3 * (size_t)p + 2], norm, delta, N, s.k, s.kk, s.wk, s.wkn);
-    return s;
-}
-
 __device__ __forceinline__ size_t cell(int i, int j, int k, int N) { return ((size_t)i * N + j) * N + k; }
 
 
-__global__ void k_pm_deposit(const double *__restrict__ pos, int n, int N, double norm, double delta, double mass,
-                             double *rho)
+// The same in 64-bit integers.  GB300 issues one warp instruction on doubles
+// in the time of about 35 on integers, and the deposit and the interpolation
+// were bound by them.  Weights in units of 2^-63.  The cell's centre is the
+// reference's (c + 1/2) delta rounded to a double; the distance to it and its
+// product with N / L are held to 2^-53 of a cell, a product of weights to
+// 2^-62.  (The exact centre instead took 8 us less and halved the error
+// against extended precision, but left the reference's rounding: 2.2e-15
+// against 1.4e-15 of the FP64 evaluation's forces.)
+struct CicFix {
+    int i, j, k, ii, jj, kk;
+    unsigned long long wi, wj, wk, win, wjn, wkn;
+    bool finite;
+};
+
+// N / L and its inverse: mantissas (64 bits with the top one set, 53 bits)
+// and exponent fields; ok: both are ordinary doubles
+struct Norm64 {
+    unsigned long long mant, dmant;
+    int expo, dexpo;
+    double norm, delta;
+    bool ok;
+};
+
+__device__ __forceinline__ void cic_axis_fix(double x, const Norm64 &q, int N, int &c, int &cn, unsigned long long &w,
+                                             unsigned long long &wn, bool &finite)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const Cic s = cic(pos, p, norm, delta, N);
-        // ((m wx) wy) wz with the shared leading products formed once
-        const double mn = __dmul_rn(mass, s.win), mi = __dmul_rn(mass, s.wi);
-        const double nn = __dmul_rn(mn, s.wjn), in = __dmul_rn(mi, s.wjn);
-        const double nj = __dmul_rn(mn, s.wj), ij = __dmul_rn(mi, s.wj);
-        atomicAdd(rho + cell(s.i, s.j, s.k, N), __dmul_rn(nn, s.wkn));
-        atomicAdd(rho + cell(s.ii, s.j, s.k, N), __dmul_rn(in, s.wkn));
-        atomicAdd(rho + cell(s.i, s.jj, s.k, N), __dmul_rn(nj, s.wkn));
-        atomicAdd(rho + cell(s.i, s.j, s.kk, N), __dmul_rn(nn, s.wk));
-        atomicAdd(rho + cell(s.ii, s.jj, s.k, N), __dmul_rn(ij, s.wkn));
-        atomicAdd(rho + cell(s.ii, s.j, s.kk, N), __dmul_rn(in, s.wk));
-        atomicAdd(rho + cell(s.i, s.jj, s.kk, N), __dmul_rn(nj, s.wk));
-        atomicAdd(rho + cell(s.ii, s.jj, s.kk, N), __dmul_rn(ij, s.wk));
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int ex = (int)(b >> 52);  // with the sign: negative x has ex >= 2048
+    const int sh = 2056 - ex - q.expo;
+    const unsigned long long mx = (b & ((1ULL << 52) - 1)) | (ex ? 1ULL << 52 : 0);
+    // u = x N / L in units of 2^-52, rounded
+    const unsigned long long hi = __umul64hi(mx << 11, q.mant);
+    const unsigned long long half = sh > 0 && sh <= 64 ? (hi >> ((sh - 1) & 63)) & 1 : 0;
+    const unsigned long long u = (sh >= 0 && sh < 64 ? hi >> sh : 0) + half;
+    c = (int)(u >> 52);
+    if (q.ok && ex < 2047 && sh >= 0 && c < 1024) {
+        // (2 c + 1) delta in units of half delta's last place, rounded to 53
+        // bits, half to even
+        unsigned long long m = (unsigned long long)(2 * c + 1) * q.dmant;
+        const int cut = 11 - __clzll((long long)m);
+        if (cut > 0) m = (m + ((1ULL << (cut - 1)) - 1) + ((m >> cut) & 1)) & ~((1ULL << cut) - 1);
+        // x in the same units: below delta its last bits may be cut off
+        const int up = ex - q.dexpo + 1;
+        const unsigned long long xm = up >= 0 ? mx << up : (up > -64 ? mx >> -up : 0);
+        const long long t = (long long)(xm - m);
+        const unsigned long long d = (unsigned long long)(t > 0 ? t : -t);
+        cn = t > 0 ? c + 1 : c - 1;
+        w = __umul64hi(d << 10, q.mant) << (q.expo + q.dexpo - 2045);
+        w = min(w, 1ULL << 63);
+        wn = (1ULL << 63) - w;
+        c = wrap(c, N);
+        cn = wrap(cn, N);
+    } else if (isfinite(x)) {  // below the box, or many cells above its lower edge
+        double v, vn;
+        cic_axis(x, q.norm, q.delta, N, c, cn, v, vn);
+        w = __double2ull_rn(v * 9223372036854775808.0);  // 2^63
+        wn = __double2ull_rn(vn * 9223372036854775808.0);
+    } else {
+        c = cn = 0;
+        w = wn = 0;
+        finite = false;
     }
 }
 
-__global__ void k_pm_scale(double *a, size_t m, double s)
+__device__ __forceinline__ CicFix cic_fix(const double *pos, int p, const Norm64 &q, int N)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x)
-        a[i] = __dmul_rn(a[i], s);
+    CicFix s;
+    s.finite = true;
+    cic_axis_fix(pos[3 * (size_t)p], q, N, s.i, s.ii, s.wi, s.win, s.finite);
+    cic_axis_fix(pos[3 * (size_t)p + 1], q, N, s.j, s.jj, s.wj, s.wjn, s.finite);
+    cic_axis_fix(pos[3 * (size_t)p + 2], q, N, s.k, s.kk, s.wk, s.wkn, s.finite);
+    return s;
+}
+
+// product of two weights
+__device__ __forceinline__ unsigned long long wmul(unsigned long long a, unsigned long long b)
+{
+    return __umul64hi(a, b) << 1;
+}
+
+// a weight (2^-63 units, at most 2^63) as a double, rounded to nearest
+__device__ __forceinline__ double weight_d(unsigned long long v)
+{
+    const int lz = __clzll((long long)v);
+    const unsigned long long m = v << (lz & 63);
+    const unsigned long long r = (m >> 11) + ((m >> 10) & 1);  // with the leading bit
+    return v ? __longlong_as_double((long long)(((unsigned long long)(1022 - lz) << 52) + r)) : 0.0;
+}
+
+// A warp takes 32 particles; two lanes then add one particle's corners, one
+// lane the four at its nearest plane in z and one those at the next, so that
+// the two addresses of a pair lie in one 32-byte sector three times in four.
+// Bound by the atomics now: 10^6 clustered particles, 128 cells a side,
+// 136 -> 90 us (a lane per particle and FP64 weights before).
+__global__ void k_pm_deposit(const double *__restrict__ pos, int n, int N, Norm64 q, double *rho)
+{
+    const int lane = warp_lane(), odd = lane & 1;
+    const int step = gridDim.x * blockDim.x;
+    for (int p0 = blockIdx.x * blockDim.x + threadIdx.x - lane; p0 < n; p0 += step) {
+        const int p = p0 + lane;
+        CicFix s{};
+        s.finite = true;
+        if (p < n) s = cic_fix(pos, p, q, N);
+        const unsigned long long nn = wmul(s.win, s.wjn), in = wmul(s.wi, s.wjn), nj = wmul(s.win, s.wj),
+                                 ij = wmul(s.wi, s.wj);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int src = (lane & ~1) | h;
+            const int pi = __shfl_sync(0xffffffffu, s.i, src), pii = __shfl_sync(0xffffffffu, s.ii, src);
+            const int pj = __shfl_sync(0xffffffffu, s.j, src), pjj = __shfl_sync(0xffffffffu, s.jj, src);
+            // each lane of the pair needs its plane of the source particle
+            const int k0 = __shfl_sync(0xffffffffu, s.k, src), k1 = __shfl_sync(0xffffffffu, s.kk, src);
+            const unsigned long long z0 = __shfl_sync(0xffffffffu, s.wkn, src), z1 = __shfl_sync(0xffffffffu, s.wk, src);
+            const unsigned long long a = __shfl_sync(0xffffffffu, nn, src), b = __shfl_sync(0xffffffffu, in, src);
+            const unsigned long long c = __shfl_sync(0xffffffffu, nj, src), d = __shfl_sync(0xffffffffu, ij, src);
+            const bool ok = __shfl_sync(0xffffffffu, (int)s.finite, src);
+            if (p0 + src >= n) continue;
+            const int k = odd ? k1 : k0;
+            const unsigned long long z = odd ? z1 : z0;
+            const double nan = __longlong_as_double(0x7ff8000000000000LL);
+            atomicAdd(rho + cell(pi, pj, k, N), ok ? weight_d(wmul(a, z)) : nan);
+            atomicAdd(rho + cell(pii, pj, k, N), ok ? weight_d(wmul(b, z)) : nan);
+            atomicAdd(rho + cell(pi, pjj, k, N), ok ? weight_d(wmul(c, z)) : nan);
+            atomicAdd(rho + cell(pii, pjj, k, N), ok ? weight_d(wmul(d, z)) : nan);
+        }
+    }
 }
 
 // sinc(pi q / N), 1 at q = 0, as the reference forms it
@@ -124,11 +214,12 @@ __global__ void k_pm_green_table(double *G, int N, double pref, double ismth2)
     }
 }
 
-// the half spectrum times the Green's function
-__global__ void k_pm_green(cufftDoubleComplex *rk, const double *__restrict__ G, size_t m)
+// the half spectrum times the Green's function and the density of one
+// particle's mass in one cell, m (N/L)^3 (the deposit adds weights)
+__global__ void k_pm_green(cufftDoubleComplex *rk, const double *__restrict__ G, size_t m, double mass_density)
 {
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < m; t += (size_t)gridDim.x * blockDim.x) {
-        const double gf = G[t];
+        const double gf = __dmul_rn(G[t], mass_density);
         rk[t].x = __dmul_rn(rk[t].x, gf);
         rk[t].y = __dmul_rn(rk[t].y, gf);
     }
@@ -136,62 +227,90 @@ __global__ void k_pm_green(cufftDoubleComplex *rk, const double *__restrict__ G,
 
 // 4-point derivative along each axis (src/partmesh.c:524-531):
 // f1 invx (psi+1 - psi-1) - f2 invx (psi+2 - psi-2), f1 = 4/3, f2 = 1/6, invx = N / (2 L)
-// (x, y, z, 0) per cell, one 32-byte record, so that the interpolation's
-// eight corners are eight sector loads
-__global__ void k_pm_gradient(const double *__restrict__ psi, int N, double invx, double4_32a *g4)
+// = invx / 6 (8 (psi+1 - psi-1) - (psi+2 - psi-2)).
+// The bracket is formed in 64-bit integers from the twelve potentials, in
+// units of 2^-58 of the power of two above the largest of them (exact where
+// they are within a factor of 32 of it, and better than one rounded
+// difference elsewhere); the interpolation multiplies by invx / 6.
+// (x, y, z, exponent) per cell, one 32-byte record, so that the
+// interpolation's eight corners are eight sector loads.  128 cells a side:
+// 65 -> 42 us.
+using GradCell = longlong4_32a;  // w: exponent field of the largest potential, 2047 if one is not finite
+
+__device__ __forceinline__ int d_expo(double v) { return (int)((__double_as_longlong(v) >> 52) & 2047); }
+
+// v in units of 2^(e - 1023 - 57), e the largest exponent field around
+__device__ __forceinline__ long long d_fix(double v, int e)
 {
-    const double f1 = 4.0 / 3.0, f2 = 1.0 / 6.0;
-    const double c1 = __dmul_rn(f1, invx), c2 = __dmul_rn(f2, invx);
-    const size_t m = (size_t)N * N * N;
+    const long long b = __double_as_longlong(v);
+    const int ev = (int)((b >> 52) & 2047);
+    const long long m = ((b & ((1LL << 52) - 1)) | (ev ? 1LL << 52 : 0)) << 5;
+    const int sh = e - (ev ? ev : 1);
+    const long long r = sh < 64 ? m >> sh : 0;
+    return b < 0 ? -r : r;
+}
+
+__global__ void k_pm_gradient(const double *__restrict__ psi, int N, GradCell *__restrict__ g)
+{
+    const unsigned m2 = (unsigned)N * N;
+    const size_t m = (size_t)m2 * N;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < m; t += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(t / ((size_t)N * N)), j = (int)((t / N) % N), k = (int)(t % N);
-        double d, gx, gy, gz;
-        d = __dmul_rn(c1, __dsub_rn(psi[cell(wrap(i + 1, N), j, k, N)], psi[cell(wrap(i - 1, N), j, k, N)]));
-        gx = __dsub_rn(d, __dmul_rn(c2, __dsub_rn(psi[cell(wrap(i + 2, N), j, k, N)], psi[cell(wrap(i - 2, N), j, k, N)])));
-        d = __dmul_rn(c1, __dsub_rn(psi[cell(i, wrap(j + 1, N), k, N)], psi[cell(i, wrap(j - 1, N), k, N)]));
-        gy = __dsub_rn(d, __dmul_rn(c2, __dsub_rn(psi[cell(i, wrap(j + 2, N), k, N)], psi[cell(i, wrap(j - 2, N), k, N)])));
-        d = __dmul_rn(c1, __dsub_rn(psi[cell(i, j, wrap(k + 1, N), N)], psi[cell(i, j, wrap(k - 1, N), N)]));
-        gz = __dsub_rn(d, __dmul_rn(c2, __dsub_rn(psi[cell(i, j, wrap(k + 2, N), N)], psi[cell(i, j, wrap(k - 2, N), N)])));
-        g4[t] = make_double4_32a(gx, gy, gz, 0.0);
+        const int i = (int)(t / m2);
+        const unsigned r = (unsigned)(t - (size_t)i * m2);
+        const int j = (int)(r / (unsigned)N), k = (int)(r % (unsigned)N);
+        double v[12];  // +1, -1, +2, -2 along x, y, z
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+            const int d = (o & 1) ? -(o / 2 + 1) : o / 2 + 1;
+            v[o] = psi[cell(wrap(i + d, N), j, k, N)];
+            v[4 + o] = psi[cell(i, wrap(j + d, N), k, N)];
+            v[8 + o] = psi[cell(i, j, wrap(k + d, N), N)];
+        }
+        int e = 1;
+#pragma unroll
+        for (int o = 0; o < 12; o++) e = max(e, d_expo(v[o]));
+        long long d[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            d[a] = 8 * (d_fix(v[4 * a], e) - d_fix(v[4 * a + 1], e)) - (d_fix(v[4 * a + 2], e) - d_fix(v[4 * a + 3], e));
+        g[t] = make_longlong4_32a(d[0], d[1], d[2], e);
     }
 }
 
-// one corner's weighted gradient added to the three running sums.  The
-// adds are fused multiply-adds (one rounding instead of two): the kernel is
-// bound by GB300's FP64 pipe, and this halves its work in the sums.
-__device__ __forceinline__ void corner(double3 &a, double w, const double4_32a &g, bool first)
-{
-    if (first) {
-        a = make_double3(__dmul_rn(w, g.x), __dmul_rn(w, g.y), __dmul_rn(w, g.z));
-    } else {
-        a.x = __fma_rn(w, g.x, a.x);
-        a.y = __fma_rn(w, g.y, a.y);
-        a.z = __fma_rn(w, g.z, a.z);
-    }
-}
-
-// the eight weighted cell values summed in the reference's order, for the
-// three components at once
-__global__ void k_pm_interp(const double *__restrict__ pos, int n, int N, double norm, double delta,
-                            const double4_32a *__restrict__ g4, double *acc)
+// the eight weighted cell values, the three components at once: 64-bit
+// integer products summed at the largest corner's exponent, to 2^-56 of the
+// largest potential around it (the potential itself is known to 2^-53).
+// 10^6 particles, 128 cells a side: 132 -> 68 us.
+__global__ void k_pm_interp(const double *__restrict__ pos, int n, int N, Norm64 q, double invx6,
+                            const GradCell *__restrict__ g, double *acc)
 {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const Cic s = cic(pos, p, norm, delta, N);
-        // (wx wy) wz with the four leading products formed once
-        const double nn = __dmul_rn(s.win, s.wjn), in = __dmul_rn(s.wi, s.wjn);
-        const double nj = __dmul_rn(s.win, s.wj), ij = __dmul_rn(s.wi, s.wj);
-        double3 a;
-        corner(a, __dmul_rn(nn, s.wkn), g4[cell(s.i, s.j, s.k, N)], true);
-        corner(a, __dmul_rn(in, s.wkn), g4[cell(s.ii, s.j, s.k, N)], false);
-        corner(a, __dmul_rn(nj, s.wkn), g4[cell(s.i, s.jj, s.k, N)], false);
-        corner(a, __dmul_rn(ij, s.wkn), g4[cell(s.ii, s.jj, s.k, N)], false);
-        corner(a, __dmul_rn(nn, s.wk), g4[cell(s.i, s.j, s.kk, N)], false);
-        corner(a, __dmul_rn(in, s.wk), g4[cell(s.ii, s.j, s.kk, N)], false);
-        corner(a, __dmul_rn(nj, s.wk), g4[cell(s.i, s.jj, s.kk, N)], false);
-        corner(a, __dmul_rn(ij, s.wk), g4[cell(s.ii, s.jj, s.kk, N)], false);
-        acc[3 * (size_t)p] = a.x;
-        acc[3 * (size_t)p + 1] = a.y;
-        acc[3 * (size_t)p + 2] = a.z;
+        const CicFix s = cic_fix(pos, p, q, N);
+        GradCell c[8];
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            c[o] = g[cell((o & 1) ? s.ii : s.i, (o & 2) ? s.jj : s.j, (o & 4) ? s.kk : s.k, N)];
+        int e = 1;
+#pragma unroll
+        for (int o = 0; o < 8; o++) e = max(e, (int)c[o].w);
+        const unsigned long long xy[4] = {wmul(s.win, s.wjn), wmul(s.wi, s.wjn), wmul(s.win, s.wj), wmul(s.wi, s.wj)};
+        long long ax = 4, ay = 4, az = 4;  // eight products are cut off below: half a unit each
+#pragma unroll
+        for (int o = 0; o < 8; o++) {
+            const long long w = (long long)__umul64hi(xy[o & 3], (o & 4) ? s.wk : s.wkn);  // 2^-62 units
+            const int sh = min(63, e - (int)c[o].w);
+            ax += __mul64hi(c[o].x, w) >> sh;
+            ay += __mul64hi(c[o].y, w) >> sh;
+            az += __mul64hi(c[o].z, w) >> sh;
+        }
+        // sums are in units of 2^(e - 1078); two factors stay inside the range of doubles
+        const int h = (e - 1078) >> 1, h2 = e - 1078 - h;
+        const double f2 = __longlong_as_double((long long)(h2 + 1023) << 52);
+        const double f = s.finite && e < 2047 ? invx6 * __longlong_as_double((long long)(h + 1023) << 52)
+                                              : __longlong_as_double(0x7ff8000000000000LL);
+        acc[3 * (size_t)p] = (double)ax * f * f2;
+        acc[3 * (size_t)p + 1] = (double)ay * f * f2;
+        acc[3 * (size_t)p + 2] = (double)az * f * f2;
     }
 }
 
@@ -251,10 +370,20 @@ int ph_pm_enqueue(photons_ctx *c, const photons_params *p, int N, int n, const d
     const double L = p->boxsize;
     const double norm = (double)N / L, delta = 1.0 / norm;  // src/partmesh.c:85-86
     PH_CUDA_CHECK(cudaMemsetAsync(c->pm_rho, 0, sizeof(double) * m, st));
-    ph::note_launch(), k_pm_deposit<<<blocks, 256, 0, st>>>(pos, n, N, norm, delta, p->mass, c->pm_rho);
+    Norm64 q;
+    q.norm = norm;
+    q.delta = delta;
+    unsigned long long nb, db;
+    memcpy(&nb, &norm, sizeof nb);
+    memcpy(&db, &delta, sizeof db);
+    q.mant = ((nb & ((1ULL << 52) - 1)) | 1ULL << 52) << 11;
+    q.dmant = (db & ((1ULL << 52) - 1)) | 1ULL << 52;
+    q.expo = (int)(nb >> 52);
+    q.dexpo = (int)(db >> 52);
+    q.ok = std::isnormal(norm) && std::isnormal(delta);  // otherwise weights are formed in FP64
+    ph::note_launch(), k_pm_deposit<<<blocks, 256, 0, st>>>(pos, n, N, q, c->pm_rho);
     double renormal = (double)N / L;
     renormal = renormal * renormal * renormal;
-    ph::note_launch(), k_pm_scale<<<blocks, 256, 0, st>>>(c->pm_rho, m, renormal);
     cufftResult r = cufftSetStream(c->pm_plan_r2c, st);
     if (r == CUFFT_SUCCESS) r = cufftSetStream(c->pm_plan_c2r, st);
     if (r == CUFFT_SUCCESS) r = cufftExecD2Z(c->pm_plan_r2c, c->pm_rho, c->pm_rk);
@@ -268,13 +397,13 @@ int ph_pm_enqueue(photons_ctx *c, const photons_params *p, int N, int n, const d
         c->pm_green_pref = pref;
         c->pm_green_ismth2 = ismth2;
     }
-    ph::note_launch(), k_pm_green<<<blocks, 256, 0, st>>>(c->pm_rk, c->pm_green, mk);
+    ph::note_launch(), k_pm_green<<<blocks, 256, 0, st>>>(c->pm_rk, c->pm_green, mk, p->mass * renormal);
     r = cufftExecZ2D(c->pm_plan_c2r, c->pm_rk, c->pm_rho);
     if (r != CUFFT_SUCCESS) return cufft_error(r, "cufftExecZ2D");
     const double invx = 0.5 * N / L;  // src/partmesh.c:458
-    double4_32a *g4 = reinterpret_cast<double4_32a *>(c->pm_grad);
-    ph::note_launch(), k_pm_gradient<<<blocks, 256, 0, st>>>(c->pm_rho, N, invx, g4);
-    ph::note_launch(), k_pm_interp<<<blocks, 256, 0, st>>>(pos, n, N, norm, delta, g4, acc_pm);
+    GradCell *g = reinterpret_cast<GradCell *>(c->pm_grad);
+    ph::note_launch(), k_pm_gradient<<<blocks, 256, 0, st>>>(c->pm_rho, N, g);
+    ph::note_launch(), k_pm_interp<<<blocks, 256, 0, st>>>(pos, n, N, q, invx / 6.0, g, acc_pm);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

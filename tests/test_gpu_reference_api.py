@@ -1,6 +1,7 @@
 """The reference-named entry points (fmm_construct ... fmm_ext) driven
 through the reference's globals, as src/photoNs.c:97-116 drives them, and
 the batched operators and the FP64 direct sum against the oracle."""
+import contextlib
 import numpy as np
 import pytest
 
@@ -224,3 +225,32 @@ def test_direct_sum_slices_and_bins_match_oracle(ph, port, ics, ntarget):
     got = ph.direct_sum(pos, p, targets)
     want = port.direct_sum(pos, p, targets, nthreads=8)
     assert rel_err(got, want, p).max() <= 1e-10
+
+
+@pytest.mark.parametrize("nside,L", [(4, 1.0), (37, 10.0), (64, 64.0), (64, 3.0e-7), (50, 1.0e9)])
+def test_pm_weights_at_cell_edges_match_oracle(ph, nside, L):
+    """The PM where the integer weights meet their edges: positions at cell
+    boundaries and centres, the box's two faces, just below zero, one last
+    place to either side, tiny ones, and random ones.  The bar of the golden
+    PM test."""
+    import pm_oracle
+    rng = np.random.default_rng(nside)
+    h = L / nside
+    edge = np.concatenate([np.arange(nside + 1) * h, (np.arange(nside) + 0.5) * h])
+    edge = np.concatenate([edge, np.nextafter(edge, 0.0), np.nextafter(edge, 2 * L),
+                           [0.0, -0.0, -0.25 * h, -1e-9 * h, 1e-300, 1e-20 * L, L]])
+    pos = np.concatenate([rng.choice(edge, (400, 3)), rng.uniform(0.0, L, (400, 3)),
+                          np.mod(rng.normal(0.3 * L, 0.01 * L, (400, 3)), L)])
+    p = dict(boxsize=L, theta=0.5, rs=1.25 * h, rcut=6.0 * h, eps=0.0, mass=2.5, maxleaf=16)
+    with contextlib.closing(ph.ForcePass(0)) as fp:
+        got = fp.pm_force(pos, p, nside)
+    want = pm_oracle.pm_force(pos, L, nside, p["rs"], p["mass"])
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
+
+
+def test_pm_of_a_position_that_is_not_finite_is_nan(ph):
+    pos = np.random.default_rng(0).uniform(0.0, 8.0, (50, 3))
+    pos[7, 1] = np.nan
+    p = dict(boxsize=8.0, theta=0.5, rs=1.0, rcut=4.0, eps=0.0, mass=1.0, maxleaf=16)
+    with contextlib.closing(ph.ForcePass(0)) as fp:
+        assert np.isnan(fp.pm_force(pos, p, 8)).all()
