@@ -1601,6 +1601,15 @@ int ph_download_tree(photons_ctx *c, HostTree &h, bool with_expansions)
     return 0;
 }
 
+// the local expansions alone, in unified order (zero without multipoles)
+int ph_download_locals(photons_ctx *c, std::vector<double> &L)
+{
+    const size_t m = (size_t)PH_NMULTI * (c->info.nleaf + c->info.nnode);
+    L.assign(m, 0.0);
+    if (c->have_multipoles) PH_CUDA_CHECK(cudaMemcpy(L.data(), c->L, sizeof(double) * m, cudaMemcpyDeviceToHost));
+    return 0;
+}
+
 // unified id -> the reference's index space
 static inline int ref_id(const photons_ctx *c, int u)
 {

@@ -176,6 +176,7 @@ int ph_stage_m2l(photons_ctx *c, int precision);
 int ph_stage_downward(photons_ctx *c, int precision);
 int ph_stage_output(photons_ctx *c, double *acc, int device_io, int tree_order);
 int ph_download_tree(photons_ctx *c, HostTree &h, bool with_expansions);
+int ph_download_locals(photons_ctx *c, std::vector<double> &L);
 int ph_pm_enqueue(photons_ctx *c, const photons_params *p, int nside, int n, const double *pos, double *acc_pm);
 void ph_pm_release(photons_ctx *c);
 

@@ -228,12 +228,14 @@ static void interact(unsigned mask, bool downward)
         for (int d = 0; d < 3; d++) part[i].acc[d] += g_stage[3 * (size_t)i + d];
     if (nm2l || downward) {
         // local expansions back into the host tree, as the reference keeps them
-        HostTree h;
-        if (ph_download_tree(c, h, true)) fatal("download");
-        for (int u = 0; u < h.nleaf; u++)
-            for (int m = 0; m < REF_NMULTI; m++) g_leaf_base[u].L[m] = h.L[(size_t)u * PH_NMULTI + m];
-        for (int k = 0; k < h.nnode; k++)
-            for (int m = 0; m < REF_NMULTI; m++) g_node_base[k].L[m] = h.L[(size_t)(h.nleaf + k) * PH_NMULTI + m];
+        // (only they changed: the whole tree took fourteen copies)
+        std::vector<double> L;
+        if (ph_download_locals(c, L)) fatal("download");
+        const int nleaf = c->info.nleaf, nnode = c->info.nnode;
+        for (int u = 0; u < nleaf; u++)
+            for (int m = 0; m < REF_NMULTI; m++) g_leaf_base[u].L[m] = L[(size_t)u * PH_NMULTI + m];
+        for (int k = 0; k < nnode; k++)
+            for (int m = 0; m < REF_NMULTI; m++) g_node_base[k].L[m] = L[(size_t)(nleaf + k) * PH_NMULTI + m];
     }
 }
 
