@@ -198,7 +198,8 @@ static int alloc_tree(photons_ctx *c, int n, int cap)
         t.cap_u = cu;
         // per-unified walk bookkeeping and expansions
         ph::WalkBufs &w = c->w;
-        PH_TRY(dalloc(w.pd_off, cu)); PH_TRY(dalloc(w.pd_cnt, cu));
+        PH_TRY(dalloc(w.queue, cu));
+        w.queue_cap = cu;
         PH_TRY(dalloc(w.p2p_off, cu)); PH_TRY(dalloc(w.p2p_cnt, cu));
         PH_TRY(dalloc(w.m2l_off, cu)); PH_TRY(dalloc(w.m2l_cnt, cu));
         PH_TRY(dalloc(t.chi, cu)); PH_TRY(dalloc(t.clo, cu)); PH_TRY(dalloc(t.w32, cu)); PH_TRY(dalloc(t.son2, cu));
@@ -249,8 +250,7 @@ static int alloc_walk(photons_ctx *c, long long p2p_cap, long long pd_cap, long 
     if (pd_cap > w.pd_cap) {
         w.pd_cap = 0;
         c->epoch++;
-        PH_TRY(dalloc(w.pd_pool[0], pd_cap));
-        PH_TRY(dalloc(w.pd_pool[1], pd_cap));
+        PH_TRY(dalloc(w.pd_pool, pd_cap));
         w.pd_cap = pd_cap;
         c->epoch++;
     }
@@ -286,8 +286,8 @@ static void free_all(photons_ctx *c)
                     b.lf_base, b.words, b.wordpre, b.tl_start, b.tl_len, b.tl_depth, b.tl_parent, b.tl_box,
                     b.ch_partial, b.ch_cnt, b.ch_small_base, b.ch_node, b.cnt, b.scan_scratch, c->t.ipart, c->t.npart,
                     c->t.depth, c->t.parent, c->t.son0, c->t.son1, c->t.cx, c->t.cy, c->t.cz, c->t.wx, c->t.wy,
-                    c->t.wz, c->t.wsum, c->t.split, c->t.depth_list, c->t.depth_off, c->w.pd_pool[0],
-                    c->w.pd_pool[1], c->w.pd_off, c->w.pd_cnt, c->w.p2p_pool, c->w.p2p_off, c->w.p2p_cnt,
+                    c->t.wz, c->t.wsum, c->t.split, c->t.depth_list, c->t.depth_off, c->w.queue,
+                    c->w.pd_pool, c->w.p2p_pool, c->w.p2p_off, c->w.p2p_cnt,
                     c->w.m2l_pool, c->w.m2l_off, c->w.m2l_cnt, c->w.scratch, c->w.ctr, c->pos4, c->ax, c->ay,
                     c->az, c->M, c->L, c->io, c->work_counter, c->t.chi, c->t.clo, c->t.w32, c->t.son2, c->M32,
                     c->t.depth_cnt, b.tn_boxid, b.tl_boxid,
@@ -863,10 +863,7 @@ static void grow_walk_caps(photons_ctx *c, unsigned long long fl, long long &p2p
     if (fl & PH_FLAG_POOL_OVERFLOW) {
         long long need = (long long)w[ph::WC_P2P_FILL];
         if (need > c->w.p2p_cap) p2p_cap = need + need / 8 + 4096;
-        need = (long long)w[ph::WC_PD_MAX];
-        long long cur = (long long)w[ph::WC_PD_FILL0];
-        if ((long long)w[ph::WC_PD_FILL1] > cur) cur = (long long)w[ph::WC_PD_FILL1];
-        if (cur > need) need = cur;
+        need = (long long)w[ph::WC_PD_FILL];
         if (need > c->w.pd_cap) pd_cap = need + need / 8 + 4096;
         need = (long long)w[ph::WC_M2L_FILL];
         if (need > c->w.m2l_cap) m2l_cap = need + need / 8 + 4096;
@@ -886,7 +883,7 @@ static void walk_caps(photons_ctx *c, long long &p2p_cap, long long &pd_cap, lon
     // 130 list entries per target leaf at leaf 16-64); an overflow grows them
     const long long per = c->pp.maxleaf > 16 ? c->pp.maxleaf : 16;
     p2p_cap = c->hint_p2p ? c->hint_p2p : n * 32 * 16 / per + 4096;
-    pd_cap = c->hint_pd ? c->hint_pd : n * 16 * 16 / per + 4096;
+    pd_cap = c->hint_pd ? c->hint_pd : n * 32 * 16 / per + 4096;
     m2l_cap = c->hint_m2l ? c->hint_m2l : n * 2 + 4096;
     stack_cap = c->w.stack_cap ? c->w.stack_cap : 4096;
     stage_cap = c->w.stage_cap ? c->w.stage_cap : 16384;
@@ -907,7 +904,7 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
     walk_caps(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
     for (int attempt = 0; attempt < 6; attempt++) {
         PH_TRY(alloc_walk(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap));
-        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->ndepth, c->pp, mask, c->stream, c->walk_imp));
+        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream, c->walk_imp));
         PH_CUDA_CHECK(cudaMemcpyAsync(c->ws.c, c->w.ctr, sizeof(c->ws.c), cudaMemcpyDeviceToHost, c->stream));
         PH_CUDA_CHECK(cudaStreamSynchronize(c->stream));
         unsigned long long fl = c->ws.c[ph::WC_FLAGS];
@@ -917,6 +914,7 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
             keep_walk_hints(c, p2p_cap, pd_cap, m2l_cap);  // a repeated pass allocates once
             return ph_record(c, EV_WALK);
         }
+        if (fl & PH_FLAG_WALK_WAIT) return ph_set_error(PH_ERR_STATE, "the walk did not finish in time");
         grow_walk_caps(c, fl, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
     }
     return ph_set_error(PH_ERR_CAPACITY, "interaction lists did not fit after repeated growth");
@@ -1137,7 +1135,7 @@ static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double
                            unsigned mask)
 {
     PH_TRY(ph_enqueue_tree(c, src, levels));
-    PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->ndepth, c->pp, mask, c->stream));
+    PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream));
     PH_TRY(ph_record(c, EV_WALK));
     PH_TRY(ph_stage_p2p(c, p->precision, 1));
     const bool far = capture_far(c, p);
@@ -1231,6 +1229,7 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
         ph_tree_info_from(c, h, levels);
         c->have_tree = true;
         unsigned long long fl = c->ws.c[ph::WC_FLAGS];
+        if (fl & PH_FLAG_WALK_WAIT) return ph_set_error(PH_ERR_STATE, "the walk did not finish in time");
         if (fl) {
             grow_walk_caps(c, fl, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
             continue;
@@ -1533,7 +1532,7 @@ extern "C" int photons_get_counters(photons_ctx *c, long long *out, int n)
     v[18] = c->info.depth;
     v[19] = (long long)w[ph::WC_MAX_STACK];
     v[20] = (long long)w[ph::WC_MAX_STAGE];
-    v[21] = (long long)std::max(w[ph::WC_PD_MAX], std::max(w[ph::WC_PD_FILL0], w[ph::WC_PD_FILL1]));
+    v[21] = (long long)w[ph::WC_PD_FILL];
     v[22] = (long long)w[ph::WC_P2P_FILL];
     v[23] = (long long)w[ph::WC_M2L_FILL];
     for (int i = 0; i < n && i < 32; i++) out[i] = v[i];

@@ -109,21 +109,20 @@ struct TreeInfo {
 };
 
 enum WalkCounter {
-    WC_PD_FILL0 = 0, WC_PD_FILL1, WC_P2P_FILL, WC_M2L_FILL,
+    WC_PD_FILL = 0, WC_P2P_FILL, WC_M2L_FILL,
     WC_P2P_LOCAL, WC_P2P_IMAGE, WC_M2L_LOCAL, WC_M2L_IMAGE,
-    WC_PAIRS_LOCAL, WC_PAIRS_IMAGE, WC_FLAGS, WC_MAX_STACK, WC_MAX_STAGE, WC_PD_MAX,
-    WC_WORK0, WC_WORK1,  // next target of the depth being walked (depth parity)
+    WC_PAIRS_LOCAL, WC_PAIRS_IMAGE, WC_FLAGS, WC_MAX_STACK, WC_MAX_STAGE,
+    WC_HEAD, WC_TAIL,  // places of the target queue taken, and made beyond the roots'
     WC_N
 };
 
 // Interaction lists.  P2P lists are per target leaf, M2L lists per target
-// (leaf or node), push-down lists per node (consumed by its children at the
-// next depth; two pools alternate by depth parity).
+// (leaf or node), push-down lists per node (inherited by its children).
 struct WalkBufs {
-    uint32_t *pd_pool[2] = {nullptr, nullptr};
+    int4 *queue = nullptr;  // targets in the order their parents were done: id and inherited list
+    int queue_cap = 0;
+    uint32_t *pd_pool = nullptr;
     long long pd_cap = 0;
-    long long *pd_off = nullptr;
-    int *pd_cnt = nullptr;
     uint32_t *p2p_pool = nullptr;
     long long p2p_cap = 0;
     long long *p2p_off = nullptr;
@@ -157,7 +156,7 @@ struct WalkImports {
 
 // image_mask: bit 0 the local tree, bit k the k-th periodic image;
 // ndepth = depths to launch (at least the tree's deepest + 1)
-int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int ndepth,
+int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
                const PassParams &p, unsigned image_mask, cudaStream_t st, const WalkImports &imp = WalkImports());
 
 // top: launched levels of wide nodes (<= levels); levels: depth bound

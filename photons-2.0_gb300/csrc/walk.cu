@@ -16,10 +16,21 @@
 // opens the target a (pairs (a0, b), (a1, b)).  Pairs that open the target
 // go to a's push-down list, which both children inherit; the self pair
 // (a, a) of a node pushes down (a0, a) and (a1, a) in the form of its two
-// children.  So the whole walk is: for each depth, for each target at that
-// depth, expand the inherited list with a warp-wide stack until only
-// records and push-downs remain.  The multiset of recorded pairs is the
-// reference's; only their order differs.
+// children.  So the whole walk is: for each target, expand the inherited
+// list with a warp-wide stack until only records and push-downs remain.
+// The multiset of recorded pairs is the reference's; only their order
+// differs.
+//
+// One launch, ordered by the data: a target is expanded as soon as its
+// parent's list is complete.  A launch per depth left most of the chip idle
+// most of the time: the upper depths have fewer targets than warps, and from
+// there on each depth waited for its longest target (a shallow leaf that
+// opens a halo's nodes takes 130 us).  Depth by depth -> one launch, ncu: 16^3
+// grid 179 -> 124 us, 32^3 238 -> 169 us, 63^3 NFW leaf 24 1.37 -> 0.73 ms,
+// 128^3 NFW leaf 24 4.62 -> 3.77 ms, 128^3 Zel'dovich leaf 48 0.80 -> 0.67 ms.
+// (Polling with acquire loads, which drop the L1 each time, took 248 us at
+// 16^3; lists of long targets cut in parts, or leaves in a launch of their
+// own after the nodes, gained on halos what they lost on grids.)
 //
 // Acceptance is evaluated in FP64 with explicit round-to-nearest operations
 // (no contraction) so that every decision equals the reference's.
@@ -119,10 +130,8 @@ __device__ __forceinline__ int acceptance_fp32(float wi0, float wi1, float wi2, 
 struct WalkArgs {
     Geo g;
     WalkBufs w;
-    const int *depth_list;
-    const int *depth_off;  // device [depth+2]: this depth's slice of depth_list
     const int *tree_cnt;   // device build counters: leaves at BC_LEAVES (the root is unified id nleaf)
-    int depth;
+    int nbox;
     int nroot;               // entries of the root's list: (root, img) for the selected images
     int root_img[PH_NIMG];
     const int *boxid;        // box of each unified id
@@ -211,8 +220,36 @@ __device__ __forceinline__ uint32_t get2(const uint32_t *s, int scap, const uint
     return pos < scap ? s[pos] : g[pos];
 }
 
+// The target at place t of the queue and its list (entries, offset in the
+// pool as 31 low bits and the rest), waited for until the warp that expands
+// its parent puts it there; id -1 if that takes more than two seconds.  The
+// wait ends: places are taken in order, so the warps that hold earlier ones
+// run, and what they do needs nothing of the waiting warp.
+__device__ __forceinline__ int4 queue_wait(const int4 *queue, long long t)
+{
+    unsigned long long t0 = 0;
+    for (unsigned i = 0;; i++) {
+        int4 v;
+        asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "l"(queue + t)
+                     : "memory");
+        if ((v.x | v.y | v.z | v.w) >= 0) {  // every word is written once, none negative
+            __threadfence();
+            return v;
+        }
+        __nanosleep(20);
+        if ((i & 63u) == 63u) {
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > 2000000000ull) return make_int4(-1, 0, 0, 0);
+        }
+    }
+}
+
 template <int MINB>
-__global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
+__global__ void __launch_bounds__(WALK_TB, MINB) k_walk(WalkArgs A)
 {
     ph::chain_begin();
     const Geo &g = A.g;
@@ -220,16 +257,6 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
     const int lane = warp_lane();
     const unsigned lt = (1u << lane) - 1u;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    // this depth counts in the counters of its parity; the other parity's,
-    // last used by the depth before, are reset for the next depth (which
-    // starts after this kernel), its pool fill kept in WC_PD_MAX
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int o = (A.depth + 1) & 1;
-        const unsigned long long f = W.ctr[WC_PD_FILL0 + o];
-        if (f > W.ctr[WC_PD_MAX]) W.ctr[WC_PD_MAX] = f;
-        W.ctr[WC_PD_FILL0 + o] = 0;
-        W.ctr[WC_WORK0 + o] = 0;
-    }
     if (gw >= W.nwarps) return;
     uint32_t *stack = W.scratch + (size_t)gw * (W.stack_cap + 3 * W.stage_cap);
     uint32_t *st_p2p = stack + W.stack_cap;
@@ -240,24 +267,31 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
     uint32_t *sh_p2p = sh_stack + WS_STACK;
     uint32_t *sh_pd = sh_p2p + WS_P2P;
     uint32_t *sh_m2l = sh_pd + WS_PD;
-    const int parity = A.depth & 1;
     const int nleaf = A.tree_cnt[BC_LEAVES];
-    const int list_begin = A.depth_off[A.depth], list_end = A.depth_off[A.depth + 1];
-    if (list_begin >= list_end) return;  // below the tree
-    bool any = false;                    // whether this warp had a target
+    const long long ntarget = nleaf + A.tree_cnt[BC_NODES];
+    bool any = false;  // whether this warp had a target
     unsigned long long c_p2p_loc = 0, c_p2p_img = 0, c_m2l_loc = 0, c_m2l_img = 0, c_pl = 0, c_pi = 0;
     unsigned flags = 0;
     int max_stack = 0, max_stage = 0;
 
-    // targets are handed out one at a time (their lists differ in length by
-    // more than tenfold on clustered input); each is expanded by one warp
+    // the queue's places are taken one at a time; the first ones are the boxes' roots
     for (;;) {
-        unsigned long long tk = 0;
-        if (lane == 0) tk = atomicAdd(&W.ctr[WC_WORK0 + parity], 1ULL);
-        const long long ti = list_begin + (long long)__shfl_sync(0xffffffffu, tk, 0);
-        if (ti >= list_end) break;
+        long long tk = 0;
+        int4 item = make_int4(0, 0, 0, 0);
+        if (lane == 0) {
+            tk = (long long)atomicAdd(&W.ctr[WC_HEAD], 1ULL);
+            if (tk >= ntarget) item.x = -2;
+            else if (tk < A.nbox) item = make_int4(A.boxes[tk].root, -1, 0, 0);
+            else item = queue_wait(W.queue, tk);
+            if (item.x == -1) flags |= PH_FLAG_WALK_WAIT;
+        }
+        const int a = __shfl_sync(0xffffffffu, item.x, 0);
+        int n_in = __shfl_sync(0xffffffffu, item.y, 0);
+        const unsigned in_lo = __shfl_sync(0xffffffffu, item.z, 0), in_hi = __shfl_sync(0xffffffffu, item.w, 0);
+        __syncwarp();
+        if (a == -2) break;
         any = true;
-        const int a = A.depth_list[ti];
+        if (a < 0) break;
         const bool leaf_a = a < nleaf;
         // the target's box: its root (the receiving domain of the image
         // pruning), side and cutoff
@@ -270,15 +304,9 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         const float4 ah = g.chi[a], al = g.clo[a], aw = g.w32[a];
         const int na = g.npart[a];
         const int a0 = leaf_a ? -1 : g.son0[a], a1 = leaf_a ? -1 : g.son1[a];
-        const int par = g.parent[a];
         const uint32_t *input = nullptr;
-        int n_in;
-        if (par < 0) {
-            n_in = A.nroot + A.imp.nroot;
-        } else {
-            input = W.pd_pool[parity ^ 1] + W.pd_off[par];
-            n_in = W.pd_cnt[par];
-        }
+        if (n_in < 0) n_in = A.nroot + A.imp.nroot;
+        else input = W.pd_pool + (((long long)in_hi << 31) | in_lo);
         int top = 0, in_pos = 0;
         int n_p2p = 0, n_m2l = 0, n_pd = 0;
         for (;;) {
@@ -295,7 +323,7 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
                     e[s2] = get2(sh_stack, WS_STACK, stack, top + j);
                 } else if (j < k) {
                     // the root's list: itself under each selected image, then the received trees
-                    if (input) e[s2] = input[i];
+                    if (input) e[s2] = __ldcg(input + i);
                     else if (i < A.nroot) e[s2] = PH_ENTRY(a, A.root_img[i]);
                     else e[s2] = PH_ENTRY(A.imp.root[i - A.nroot], PH_IMG_IMPORT);
                 }
@@ -454,37 +482,41 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk_level(WalkArgs A)
         int stage_hi = max(n_p2p, max(n_m2l, n_pd));
         max_stage = max(max_stage, stage_hi);
         if (stage_hi > W.stage_cap) flags |= PH_FLAG_STAGE_OVERFLOW;
-        // commit staged lists
-        long long off = 0;
+        // commit staged lists: the places in the pools, and a node's two places in
+        // the queue, taken by three lanes at once
+        const int n_out = leaf_a ? n_p2p : n_pd;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&W.ctr[leaf_a ? WC_P2P_FILL : WC_PD_FILL], (unsigned long long)n_out);
+        else if (lane == 1 && n_m2l) at = atomicAdd(&W.ctr[WC_M2L_FILL], (unsigned long long)n_m2l);
+        else if (lane == 2 && !leaf_a) at = atomicAdd(&W.ctr[WC_TAIL], 2ULL);
+        const long long off = (long long)__shfl_sync(0xffffffffu, at, 0), off_m = (long long)__shfl_sync(0xffffffffu, at, 1);
+        const long long place = (long long)__shfl_sync(0xffffffffu, at, 2);
+        const bool ok = off + n_out <= (leaf_a ? W.p2p_cap : W.pd_cap) && n_out <= W.stage_cap;
+        const bool ok_m = off_m + n_m2l <= W.m2l_cap && n_m2l <= W.stage_cap;
+        if (!ok || !ok_m) flags |= PH_FLAG_POOL_OVERFLOW;
         if (leaf_a) {
-            if (lane == 0) off = (long long)atomicAdd((unsigned long long *)&W.ctr[WC_P2P_FILL], (unsigned long long)n_p2p);
-            off = __shfl_sync(0xffffffffu, off, 0);
-            bool ok = off + n_p2p <= W.p2p_cap && n_p2p <= W.stage_cap;
-            if (!ok) flags |= PH_FLAG_POOL_OVERFLOW;
-            else
+            if (ok)
 #pragma unroll 4
                 for (int i = lane; i < n_p2p; i += 32) W.p2p_pool[off + i] = get2(sh_p2p, WS_P2P, st_p2p, i);
             if (lane == 0) { W.p2p_off[a] = ok ? off : 0; W.p2p_cnt[a] = ok ? n_p2p : 0; }
         } else {
-            if (lane == 0) off = (long long)atomicAdd((unsigned long long *)&W.ctr[WC_PD_FILL0 + parity], (unsigned long long)n_pd);
-            off = __shfl_sync(0xffffffffu, off, 0);
-            bool ok = off + n_pd <= W.pd_cap && n_pd <= W.stage_cap;
-            if (!ok) flags |= PH_FLAG_POOL_OVERFLOW;
-            else
+            if (ok)
 #pragma unroll 4
-                for (int i = lane; i < n_pd; i += 32) W.pd_pool[parity][off + i] = get2(sh_pd, WS_PD, st_pd, i);
-            if (lane == 0) { W.pd_off[a] = ok ? off : 0; W.pd_cnt[a] = ok ? n_pd : 0; }
+                for (int i = lane; i < n_pd; i += 32) W.pd_pool[off + i] = get2(sh_pd, WS_PD, st_pd, i);
+            // the list is complete: both children can be expanded
+            __threadfence();
+            __syncwarp();
+            if (lane < 2) {
+                const long long o = ok ? off : 0;
+                asm volatile("st.relaxed.gpu.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(W.queue + A.nbox + place + lane),
+                             "r"(lane ? a1 : a0), "r"(ok ? n_pd : 0), "r"((int)(o & 0x7fffffff)), "r"((int)(o >> 31))
+                             : "memory");
+            }
         }
-        if (lane == 0) off = (long long)atomicAdd((unsigned long long *)&W.ctr[WC_M2L_FILL], (unsigned long long)n_m2l);
-        off = __shfl_sync(0xffffffffu, off, 0);
-        {
-            bool ok = off + n_m2l <= W.m2l_cap && n_m2l <= W.stage_cap;
-            if (!ok) flags |= PH_FLAG_POOL_OVERFLOW;
-            else
+        if (ok_m)
 #pragma unroll 4
-                for (int i = lane; i < n_m2l; i += 32) W.m2l_pool[off + i] = get2(sh_m2l, WS_M2L, st_m2l, i);
-            if (lane == 0) { W.m2l_off[a] = ok ? off : 0; W.m2l_cnt[a] = ok ? n_m2l : 0; }
-        }
+            for (int i = lane; i < n_m2l; i += 32) W.m2l_pool[off_m + i] = get2(sh_m2l, WS_M2L, st_m2l, i);
+        if (lane == 0) { W.m2l_off[a] = ok_m ? off_m : 0; W.m2l_cnt[a] = ok_m ? n_m2l : 0; }
         __syncwarp();
     }
     if (!any) return;
@@ -538,12 +570,12 @@ int launch_geom32(const TreeBufs &t, const int *tree_cnt, cudaStream_t st)
     return 0;
 }
 
-// Enqueue the walk of depths 0..ndepth-1; depths past the tree's deepest
-// exit at once.  Counters and flags stay on the device (w.ctr).
-int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int ndepth,
+// Enqueue the walk.  Counters and flags stay on the device (w.ctr).
+int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
                const PassParams &p, unsigned image_mask, cudaStream_t st, const WalkImports &imp)
 {
     PH_CUDA_CHECK(cudaMemsetAsync(w.ctr, 0, sizeof(unsigned long long) * WC_N, st));
+    PH_CUDA_CHECK(cudaMemsetAsync(w.queue, 0xff, sizeof(int4) * (size_t)w.queue_cap, st));
     WalkArgs A{};
     A.g.cx = t.cx; A.g.cy = t.cy; A.g.cz = t.cz;
     A.g.wx = t.wx; A.g.wy = t.wy; A.g.wz = t.wz; A.g.wsum = t.wsum;
@@ -553,9 +585,8 @@ int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxPar
     A.prune_k2f = (float)((0.95 * p.theta) * (0.95 * p.theta));
     A.boxid = t.boxid;
     A.boxes = boxes;
+    A.nbox = nbox;
     A.w = w;
-    A.depth_list = t.depth_list;
-    A.depth_off = t.depth_off;
     A.tree_cnt = tree_cnt;
     A.nroot = 0;
     for (int img = 0; img < PH_NIMG; img++)
@@ -565,13 +596,10 @@ int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxPar
     A.imp = imp;
     A.maxleaf = p.maxleaf;
     const int blocks = (w.nwarps * 32 + WALK_TB - 1) / WALK_TB;
-    for (int d = 0; d < ndepth; d++) {
-        A.depth = d;
-        if (w.nwarps == device_sm_count() * 3 * 8)
-            ph::chain(k_walk_level<3>, blocks, WALK_TB, 0, st, A);
-        else
-            ph::chain(k_walk_level<2>, blocks, WALK_TB, 0, st, A);
-    }
+    if (w.nwarps == device_sm_count() * 3 * 8)
+        ph::chain(k_walk<3>, blocks, WALK_TB, 0, st, A);
+    else
+        ph::chain(k_walk<2>, blocks, WALK_TB, 0, st, A);
     PH_CUDA_CHECK(cudaGetLastError());
     return 0;
 }
