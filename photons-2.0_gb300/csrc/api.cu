@@ -883,7 +883,9 @@ static void walk_caps(photons_ctx *c, long long &p2p_cap, long long &pd_cap, lon
     // 130 list entries per target leaf at leaf 16-64); an overflow grows them
     const long long per = c->pp.maxleaf > 16 ? c->pp.maxleaf : 16;
     p2p_cap = c->hint_p2p ? c->hint_p2p : n * 32 * 16 / per + 4096;
-    pd_cap = c->hint_pd ? c->hint_pd : n * 32 * 16 / per + 4096;
+    // push-down entries: up to 51 16 / leaf a particle in halos (leaf 16), 4.7 16 / leaf
+    // in a 256^3 Zel'dovich box (leaf 64); cut short, they also hide the P2P need
+    pd_cap = c->hint_pd ? c->hint_pd : n * (per < 48 ? 64 : 32) * 16 / per + 4096;
     m2l_cap = c->hint_m2l ? c->hint_m2l : n * 2 + 4096;
     stack_cap = c->w.stack_cap ? c->w.stack_cap : 4096;
     stage_cap = c->w.stage_cap ? c->w.stage_cap : 16384;
