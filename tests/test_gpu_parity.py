@@ -522,3 +522,22 @@ def test_tree_around_the_split_sizes_matches_oracle(ph, fp, port, n, maxleaf):
     tr = fp.tree()
     for k in ("leaf_ipart", "leaf_npart", "node_npart", "node_son"):
         assert np.array_equal(tr[k], r["tree"][k]), k
+
+
+@pytest.mark.parametrize("n,maxleaf,spread", [(17, 16, 1.0), (2, 1, 1.0), (40, 1, 1.0), (300, 16, 0.02), (5000, 1, 0.001)])
+def test_walk_of_small_and_deep_trees_matches_oracle(ph, fp, port, n, maxleaf, spread):
+    """The walk's queue at its ends: two leaves under one root, fewer targets
+    than warps, and a deep chain of nodes (a tight clump in an empty box):
+    lists exactly the oracle's, twice from one context."""
+    rng = np.random.default_rng(n)
+    p = dict(boxsize=100.0, theta=0.5, rs=4.0, rcut=18.0, eps=0.1, mass=1.0, maxleaf=maxleaf)
+    pos = np.mod(50.0 + spread * rng.uniform(-50.0, 50.0, (n, 3)), 100.0)
+    pos[-1] = (3.0, 4.0, 95.0)
+    r = port.run(pos, p, capture=True, tree=False, nthreads=4)
+    for _ in range(2):
+        fp.run(pos, p, precision=ph.FP64, flags=ph.F_TREE_ORDER | ph.F_KEEP_LISTS)
+        c = fp.counters()
+        for k in COUNTERS[:4]:
+            assert c[k] == r["counters"][k], k
+        for kind, (t, s, im) in fp.lists().items():
+            assert digest(t, s, im) == digest(*(np.asarray(x) for x in r["lists"][kind])), kind
