@@ -134,7 +134,7 @@ inline void note_launch()
     else g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-// Kernels of a chain (tree levels, walk levels, far-field depths: dozens of
+// Kernels of a chain (tree levels, far-field depths, the walk after them: dozens of
 // launches of a few microseconds each) are launched with programmatic stream
 // serialization: a kernel's blocks may be set up while the kernel before it
 // in the stream runs, and chain_begin(), the first statement of every such
