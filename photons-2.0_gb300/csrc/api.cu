@@ -157,7 +157,9 @@ static int alloc_tree(photons_ctx *c, int n, int cap)
         PH_TRY(dalloc(b.tn_split, cap)); PH_TRY(dalloc(b.tn_nch, cap)); PH_TRY(dalloc(b.tn_chunk_base, cap));
         PH_TRY(dalloc(b.tn_nodeflag, cap)); PH_TRY(dalloc(b.tn_leafflag, cap)); PH_TRY(dalloc(b.tn_nodebase, cap));
         PH_TRY(dalloc(b.tn_leafbase, cap));
-        PH_TRY(dalloc(b.lf_depth, cap)); PH_TRY(dalloc(b.lf_top, cap)); PH_TRY(dalloc(b.lf_base, cap));
+        PH_TRY(dalloc(b.lf_depth, cap)); PH_TRY(dalloc(b.lf_top, cap)); PH_TRY(dalloc(b.lf_empty, cap));
+        PH_TRY(dalloc(b.lf_base, cap)); PH_TRY(dalloc(b.lf_in, cap));
+        PH_TRY(dalloc(b.lf_scan, ph::scan_scratch_elems(cap) + 8));
         PH_TRY(dalloc(b.tl_start, cap)); PH_TRY(dalloc(b.tl_len, cap)); PH_TRY(dalloc(b.tl_depth, cap));
         PH_TRY(dalloc(b.tl_parent, cap)); PH_TRY(dalloc(b.tl_box, (size_t)6 * cap));
         PH_TRY(dalloc(b.tn_boxid, cap)); PH_TRY(dalloc(b.tl_boxid, cap));
@@ -283,7 +285,7 @@ static void free_all(photons_ctx *c)
     void *ptrs[] = {b.x, b.y, b.z, b.perm, b.smallpos, b.bigpos, b.tn_start, b.tn_len, b.tn_depth, b.tn_parent,
                     b.tn_child0, b.tn_child1, b.tn_mode, b.tn_S, b.tn_box, b.tn_split, b.tn_nch, b.tn_chunk_base,
                     b.tn_nodeflag, b.tn_leafflag, b.tn_nodebase, b.tn_leafbase, b.lf_depth, b.lf_top,
-                    b.lf_base, b.words, b.wordpre, b.tl_start, b.tl_len, b.tl_depth, b.tl_parent, b.tl_box,
+                    b.lf_empty, b.lf_base, b.lf_in, b.lf_scan, b.words, b.wordpre, b.tl_start, b.tl_len, b.tl_depth, b.tl_parent, b.tl_box,
                     b.ch_partial, b.ch_cnt, b.ch_small_base, b.ch_node, b.cnt, b.scan_scratch, c->t.ipart, c->t.npart,
                     c->t.depth, c->t.parent, c->t.son0, c->t.son1, c->t.cx, c->t.cy, c->t.cz, c->t.wx, c->t.wy,
                     c->t.wz, c->t.wsum, c->t.split, c->t.depth_list, c->t.depth_off, c->w.queue,

@@ -26,12 +26,14 @@ struct BuildBufs {
     int *tn_nodeflag = nullptr, *tn_leafflag = nullptr, *tn_nodebase = nullptr, *tn_leafbase = nullptr;
     // temp leaves
     int *tl_start = nullptr, *tl_len = nullptr, *tl_depth = nullptr, *tl_parent = nullptr;
-    // numbering: bit i of word w: a leaf starts at particle 32 w + i; leaf
-    // starts before each word; per leaf in depth-first order: its depth, the
-    // depth of the topmost node or leaf starting where it does, and the nodes
-    // before it in preorder
+    // numbering: bit i of word w: a leaf with particles starts at particle
+    // 32 w + i; such starts before each word; per start: that leaf's depth,
+    // the depth of the topmost node or leaf starting there, the empty leaves
+    // there, and the nodes (low half) and empty leaves (high half) of all the
+    // starts before; that scan's input and scratch
     int *words = nullptr, *wordpre = nullptr;
-    int *lf_depth = nullptr, *lf_top = nullptr, *lf_base = nullptr;
+    int *lf_depth = nullptr, *lf_top = nullptr, *lf_empty = nullptr;
+    long long *lf_base = nullptr, *lf_in = nullptr, *lf_scan = nullptr;
     double *tl_box = nullptr;  // [6][cap_leaves]
     // chunks
     double *ch_partial = nullptr;
@@ -71,7 +73,9 @@ enum BuildCounter {
     BC_MID_LEAVES = 16,
     BC_WORDS = 17,        // words of the leaf-start bit mask
     BC_SCAN_TOTAL = 18,
-    BC_NCOUNTERS = 20
+    BC_EMPTY = 19,        // empty leaves
+    BC_STARTS = 20,       // leaves with particles
+    BC_NCOUNTERS = 22
 };
 
 // nodes of at most this many particles are split in shared memory (30 bytes a

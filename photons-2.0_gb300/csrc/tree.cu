@@ -1073,71 +1073,97 @@ __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0
 
 // ---------------- numbering ----------------
 // Leaves partition the particles in depth-first order, so a leaf's number is
-// the number of leaf starts before its own: a bit per particle, counted by
-// words.  Nodes that start where a leaf does are its ancestors from the
+// the number of leaves before its own start: a bit per particle where a leaf
+// with particles starts, counted by words, plus the empty leaves before.
+// Nodes that start where such a leaf does are its ancestors from the
 // topmost one starting there (a right child or a root) down to its parent,
 // and nodes in preorder are those of the first leaf, those of the second and
 // so on: a node's number is the nodes of the leaves before plus its depth
 // below that topmost one.  (The reference numbers them while it recurses,
 // src/fmm.c:101-118.)
+// An empty leaf is a left child: where the mean of equal coordinates rounds
+// below them, the lower half of the split holds nothing (sheets, lines and
+// lattices; a right child always holds something).  It starts where its
+// sibling does and comes before what the sibling holds, so the empty leaves
+// of one start are ordered by depth and precede the leaf with particles.
 __global__ void k_mark_leaves(BuildBufs b)
 {
     ph::chain_begin();
     const int nleaves = b.cnt[BC_LEAVES];
     for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nleaves; l += gridDim.x * blockDim.x) {
-        const int p = b.tl_start[l];
-        atomicOr(reinterpret_cast<unsigned *>(b.words) + (p >> 5), 1u << (p & 31));
+        b.lf_empty[l] = 0;
+        if (b.tl_len[l] > 0) {
+            const int p = b.tl_start[l];
+            atomicOr(reinterpret_cast<unsigned *>(b.words) + (p >> 5), 1u << (p & 31));
+        } else {
+            atomicAdd(&b.cnt[BC_EMPTY], 1);
+        }
     }
 }
 
-// leaf starts before particle p
-__device__ __forceinline__ int leaf_rank(const BuildBufs &b, int p)
+// starts before particle p
+__device__ __forceinline__ int start_rank(const BuildBufs &b, int p)
 {
     return b.wordpre[p >> 5] + __popc((unsigned)b.words[p >> 5] & ((1u << (p & 31)) - 1u));
 }
 
-// scan inputs: bits set of w[i], or d[i] - t[i]
-__device__ __forceinline__ int scan_value(const int *w, const int *d, const int *t, int i)
+// scan inputs: the starts of word i; per start, the nodes there and, in the
+// upper half, the empty leaves
+__device__ __forceinline__ void scan_value(const BuildBufs &b, int i, int &v) { v = __popc((unsigned)b.words[i]); }
+__device__ __forceinline__ void scan_value(const BuildBufs &b, int i, long long &v)
 {
-    return w ? __popc((unsigned)w[i]) : d[i] - t[i];
+    v = (b.lf_depth[i] - b.lf_top[i]) | ((long long)b.lf_empty[i] << 32);
 }
 
-__global__ void k_scan_input(const int *n_ptr, const int *w, const int *d, const int *t, int *out)
+template <class V>
+__global__ void k_scan_input(BuildBufs b, const int *n_ptr, V *out)
 {
     ph::chain_begin();
     const int n = *n_ptr;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = scan_value(w, d, t, i);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) scan_value(b, i, out[i]);
+}
+
+template <class V>
+__device__ __forceinline__ V warp_incl(V v)
+{
+    const int lane = warp_lane();
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const V t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
 }
 
 // the exclusive scan of up to ONE_SCAN_MAX of them in one block
 #define ONE_SCAN_TB 1024
 #define ONE_SCAN_MAX (1 << 16)
-__global__ void __launch_bounds__(ONE_SCAN_TB) k_scan_one(const int *n_ptr, const int *w, const int *d, const int *t,
-                                                          int *out)
+template <class V>
+__global__ void __launch_bounds__(ONE_SCAN_TB) k_scan_one(BuildBufs b, const int *n_ptr, V *out)
 {
     ph::chain_begin();
-    __shared__ int s_warp[33];
+    __shared__ V s_warp[33];
     const int lane = warp_lane(), warp = threadIdx.x >> 5, n = *n_ptr;
-    int carry = 0;
+    V carry = 0;
     for (int base = 0; base < n; base += 4 * ONE_SCAN_TB) {
         const int i0 = base + 4 * (int)threadIdx.x;
-        int v[4], sum = 0;
+        V v[4], sum = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            v[k] = i0 + k < n ? scan_value(w, d, t, i0 + k) : 0;
+            v[k] = 0;
+            if (i0 + k < n) scan_value(b, i0 + k, v[k]);
             sum += v[k];
         }
-        const int incl = warp_incl_scan(sum);
+        const V incl = warp_incl(sum);
         if (lane == 31) s_warp[warp] = incl;
         __syncthreads();
         if (warp == 0) {
-            const int x = s_warp[lane], xi = warp_incl_scan(x);
+            const V x = s_warp[lane], xi = warp_incl(x);
             s_warp[lane] = xi - x;
             if (lane == 31) s_warp[32] = xi;
         }
         __syncthreads();
-        int at = carry + s_warp[warp] + incl - sum;
+        V at = carry + s_warp[warp] + incl - sum;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             if (i0 + k < n) out[i0 + k] = at;
@@ -1148,18 +1174,23 @@ __global__ void __launch_bounds__(ONE_SCAN_TB) k_scan_one(const int *n_ptr, cons
     }
 }
 
-// per leaf in depth-first order: its depth, and the depth of the topmost
-// node or leaf that starts where it does
+// per start: the depth of the leaf with particles, the depth of the topmost
+// node or leaf that starts there, and the empty leaves
 __global__ void k_leaf_ranks(BuildBufs b)
 {
     ph::chain_begin();
     const int nleaves = b.cnt[BC_LEAVES], nnodes = b.cnt[BC_NODES];
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.cnt[BC_STARTS] = nleaves - b.cnt[BC_EMPTY];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nleaves + nnodes; i += gridDim.x * blockDim.x) {
         const bool leaf = i < nleaves;
         const int t = leaf ? i : i - nleaves;
         const int start = leaf ? b.tl_start[t] : b.tn_start[t], parent = leaf ? b.tl_parent[t] : b.tn_parent[t],
                   depth = leaf ? b.tl_depth[t] : b.tn_depth[t];
-        const int r = leaf_rank(b, start);
+        const int r = start_rank(b, start);
+        if (leaf && b.tl_len[t] == 0) {
+            atomicAdd(&b.lf_empty[r], 1);
+            continue;
+        }
         if (leaf) b.lf_depth[r] = depth;
         if (parent < 0 || b.tn_start[parent] != start) b.lf_top[r] = depth;
     }
@@ -1179,14 +1210,30 @@ __device__ __forceinline__ void write_geom(TreeBufs &T, int u, const double *box
 // preorder number of the node of depth `depth` that starts at particle p
 __device__ __forceinline__ int node_number(const BuildBufs &b, int p, int depth)
 {
-    const int r = leaf_rank(b, p);
-    return b.lf_base[r] + depth - b.lf_top[r];
+    const int r = start_rank(b, p);
+    return (int)b.lf_base[r] + depth - b.lf_top[r];
 }
 
-// a child's unified id: a leaf's rank, or a node's preorder number after the leaves
+// depth-first number of temp leaf l
+__device__ __forceinline__ int leaf_number(const BuildBufs &b, int l)
+{
+    const int start = b.tl_start[l], r = start_rank(b, start), empty = b.lf_empty[r];
+    int id = r + (int)(b.lf_base[r] >> 32);
+    if (empty == 0) return id;
+    if (b.tl_len[l] > 0) return id + empty;
+    // after the empty leaves of the nodes above its parent that start here too
+    for (int t = b.tl_parent[l];;) {
+        t = b.tn_parent[t];
+        if (t < 0 || b.tn_start[t] != start) return id;
+        const int c = b.tn_child0[t];
+        id += PH_IS_LEAF_CODE(c) && b.tl_len[~c] == 0;
+    }
+}
+
+// a child's unified id: a leaf's number, or a node's preorder number after the leaves
 __device__ __forceinline__ int child_id(const BuildBufs &b, int code, int nleaves)
 {
-    return PH_IS_LEAF_CODE(code) ? leaf_rank(b, b.tl_start[~code])
+    return PH_IS_LEAF_CODE(code) ? leaf_number(b, ~code)
                                  : nleaves + node_number(b, b.tn_start[code], b.tn_depth[code]);
 }
 
@@ -1197,7 +1244,7 @@ __global__ void k_scatter_tree(BuildBufs b, TreeBufs T)
     const int nnodes = b.cnt[BC_NODES], nleaves = b.cnt[BC_LEAVES];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nleaves + nnodes; i += gridDim.x * blockDim.x) {
         if (i < nleaves) {
-            const int l = i, u = leaf_rank(b, b.tl_start[l]), par = b.tl_parent[l];
+            const int l = i, u = leaf_number(b, l), par = b.tl_parent[l];
             T.ipart[u] = b.tl_start[l];
             T.npart[u] = b.tl_len[l];
             T.depth[u] = b.tl_depth[l];
@@ -1378,22 +1425,21 @@ int build_tree(BuildBufs &b, TreeBufs &T, const PassParams &p, int n, int levels
                                                                                                 levels);
     ph::chain(k_tree_totals, 1, 1, 0, st, b);
     ph::chain(k_mark_leaves, maxb, TB, 0, st, b);
-    // leaf starts before each word of 32 positions, then nodes before each leaf
+    // starts before each word of 32 positions, then nodes and empty leaves before each start
     const int nwords = (n + 31) / 32;
     if (nwords <= ONE_SCAN_MAX) {
-        ph::chain(k_scan_one, 1, ONE_SCAN_TB, 0, st, b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.wordpre);
+        ph::chain(k_scan_one<int>, 1, ONE_SCAN_TB, 0, st, b, b.cnt + BC_WORDS, b.wordpre);
     } else {
-        ph::chain(k_scan_input, maxb, TB, 0, st, b.cnt + BC_WORDS, b.words, nullptr, nullptr, b.bigpos);
+        ph::chain(k_scan_input<int>, maxb, TB, 0, st, b, b.cnt + BC_WORDS, b.bigpos);
         scan_exclusive_i32(b.bigpos, b.wordpre, b.cnt + BC_WORDS, nwords, b.cnt + BC_SCAN_TOTAL, b.scan_scratch,
                            b.scan_scratch_elems, st);
     }
     ph::chain(k_leaf_ranks, maxb, TB, 0, st, b);
     if (b.rule_cap <= ONE_SCAN_MAX) {
-        ph::chain(k_scan_one, 1, ONE_SCAN_TB, 0, st, b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.lf_base);
+        ph::chain(k_scan_one<long long>, 1, ONE_SCAN_TB, 0, st, b, b.cnt + BC_STARTS, b.lf_base);
     } else {
-        ph::chain(k_scan_input, maxb, TB, 0, st, b.cnt + BC_LEAVES, nullptr, b.lf_depth, b.lf_top, b.bigpos);
-        scan_exclusive_i32(b.bigpos, b.lf_base, b.cnt + BC_LEAVES, b.rule_cap, b.cnt + BC_SCAN_TOTAL, b.scan_scratch,
-                           b.scan_scratch_elems, st);
+        ph::chain(k_scan_input<long long>, maxb, TB, 0, st, b, b.cnt + BC_STARTS, b.lf_in);
+        scan_exclusive_i64(b.lf_in, b.lf_base, b.cnt + BC_STARTS, b.rule_cap, nullptr, b.lf_scan, st);
     }
     ph::chain(k_scatter_tree, maxb, TB, 0, st, b, T);
     ph::chain(k_depth_count, nblk, 32, 0, st, b, T, ndepth);
