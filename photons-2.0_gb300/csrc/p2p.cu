@@ -506,16 +506,18 @@ __device__ __forceinline__ void comp_streams(float2 *v, int m)
 __device__ __forceinline__ int ow_limit(const BoxParams &B, int maxleaf) { return max(32, B.count / (100 * maxleaf)); }
 
 // the long leaves (ctl[0]: their number; ctl[1], ctl[2]: the kernel's
-// counters of the long and of all leaves)
-__global__ void k_ow_long(const int *tree_cnt, const unsigned long long *walk_flags, const int *cnt, const int *boxid,
-                          const BoxParams *boxes, int maxleaf, int *ctl, int *longs)
+// counters of the long and of all leaves).  A leaf without particles is not
+// among them: it would reach none of the barriers that a leaf of the block
+// kernel ends with.
+__global__ void k_ow_long(const int *tree_cnt, const unsigned long long *walk_flags, const int *npart, const int *cnt,
+                          const int *boxid, const BoxParams *boxes, int maxleaf, int *ctl, int *longs)
 {
     const int nleaf = *walk_flags ? 0 : tree_cnt[BC_LEAVES];
     const int lane = warp_lane();
     const int stride = gridDim.x * blockDim.x;
     for (int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; t0 < nleaf; t0 += stride) {
         const int t = t0 + lane;
-        const bool is = t < nleaf && cnt[t] > ow_limit(boxes[boxid[t]], maxleaf);
+        const bool is = t < nleaf && npart[t] > 0 && cnt[t] > ow_limit(boxes[boxid[t]], maxleaf);
         const unsigned m = __ballot_sync(0xffffffffu, is);
         int at = 0;
         if (lane == 0 && m) at = atomicAdd(ctl, __popc(m));
@@ -1760,6 +1762,7 @@ __global__ void __launch_bounds__(MU64_TB, 1) k_p2p_mutual64(P2PArgs A, const in
         const int2 item = items[i];
         const int t = item.x, e0 = item.y * seg;
         const int nt = A.npart[t], it = A.ipart[t];
+        if (nt == 0) continue;
         const int ne = fits ? min(seg, nev[t] - e0) : nev[t], prow = mu_row_g(nt, MU64_ROW);
         const int2 *evt = ev + A.p2p_off[t] + e0;
         double *part = fits ? rbuf + rbase[t] + (long long)(nrecv[t] + item.y) * 3 * prow : nullptr;
@@ -2038,7 +2041,7 @@ int launch_p2p(const P2PArgs &a, int fp64, cudaStream_t st)
     } else {
         const int resident = device_sm_count() * P2P_MINB;
         PH_CUDA_CHECK(cudaMemsetAsync(a.ow_ctl, 0, 3 * sizeof(int), st));
-        ph::note_launch(), k_ow_long<<<device_sm_count(), 256, 0, st>>>(a.tree_cnt, a.walk_flags, a.p2p_cnt, a.boxid,
+        ph::note_launch(), k_ow_long<<<device_sm_count(), 256, 0, st>>>(a.tree_cnt, a.walk_flags, a.npart, a.p2p_cnt, a.boxid,
                                                                          a.boxes, a.maxleaf, a.ow_ctl, a.ow_long);
         ph::note_launch(), k_p2p_split_packed<P2P_WARPS><<<resident, P2P_TB, 0, st>>>(a);
         ph::note_launch(), k_p2p_split_packed<1><<<resident, P2P_TB, 0, st>>>(a);
