@@ -867,8 +867,12 @@ __device__ __forceinline__ void mu_sort_regs(uint32_t *lst, int L, int lane)
 // 1,024 sorted in shared memory, 32 KB a block, took 227 against 44 us in an
 // FP64 pass over 110,591 particles, half in halos, and 80 against 14 us at
 // 32^3 particles, leaf 16: two list reads and writes a step and few warps.)
+// sorted[t]: the list is sorted and the leaf's pairs may be evaluated once.
+// Not so for a leaf without particles: it evaluates nothing, and slots that
+// wait for its reactions would never be written.
 __global__ void __launch_bounds__(256) k_mu_sort(const int *tree_cnt, const unsigned long long *walk_flags,
-                                                  uint32_t *pool, const long long *off, const int *cnt, int *sorted)
+                                                  uint32_t *pool, const long long *off, const int *cnt,
+                                                  const int *npart, int *sorted)
 {
     const int lane = warp_lane();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -890,7 +894,7 @@ __global__ void __launch_bounds__(256) k_mu_sort(const int *tree_cnt, const unsi
         } else if (L > 512 && ok) {
             mu_sort_regs<32>(lst, L, lane);
         }
-        if (lane == 0) sorted[t] = ok;
+        if (lane == 0) sorted[t] = ok && npart[t] > 0;
     }
 }
 
@@ -902,13 +906,13 @@ __global__ void __launch_bounds__(256) k_mu_sort(const int *tree_cnt, const unsi
 #define MU_SORT_TB 512
 __global__ void __launch_bounds__(MU_SORT_TB) k_mu_sort_long(const int *tree_cnt, const unsigned long long *walk_flags,
                                                              uint32_t *pool, const long long *off, const int *cnt,
-                                                             int *sorted)
+                                                             const int *npart, int *sorted)
 {
     extern __shared__ __align__(16) uint32_t sort_buf[];
     const int nleaf = *walk_flags ? 0 : tree_cnt[BC_LEAVES];
     for (int t = blockIdx.x; t < nleaf; t += gridDim.x) {
         const int L = cnt[t];
-        if (L <= MU_SORT_MAX || L > MU_SORT_LONG) continue;  // the same for the whole block
+        if (L <= MU_SORT_MAX || L > MU_SORT_LONG || npart[t] == 0) continue;  // the same for the whole block
         uint32_t *lst = pool + off[t];
         int P = 2 * MU_SORT_MAX;
         while (P < L) P <<= 1;
@@ -1972,13 +1976,13 @@ int launch_mutual_pairing(const P2PArgs &a, const MutualBufs &m, int fp64, cudaS
     const int sms = device_sm_count();
     const int seg = fp64 ? mu64_seg(m.maxleaf) : 0;
     ph::note_launch(), k_mu_sort<<<sms * 4, 256, 0, st>>>(a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt,
-                                                           m.sorted);
+                                                           a.npart, m.sorted);
     if (fp64) {
         if (int rc = mu64_attributes()) return rc;
         PH_CUDA_CHECK(cudaMemsetAsync(m.nitems, 0, sizeof(int), st));
         if (m.sort_long)
             ph::note_launch(), k_mu_sort_long<<<sms * 3, MU_SORT_TB, MU_SORT_LONG * sizeof(uint32_t), st>>>(
-                a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt, m.sorted);
+                a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt, a.npart, m.sorted);
     }
     ph::note_launch(), k_mu_pair<<<sms * 8, 256, 0, st>>>(a.tree_cnt, a.walk_flags, m.pool, a.p2p_off, a.p2p_cnt,
                                                            a.npart, m.sorted, m.slot, m.pq, m.nrecv, m.size,

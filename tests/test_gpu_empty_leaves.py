@@ -158,15 +158,23 @@ def test_tree_and_forces_with_empty_leaves(ph, fp, case):
 
 
 @pytest.mark.parametrize("case", range(len(SMALL)))
-@pytest.mark.parametrize("flags", ["F_ONE_WAY"])
+def test_fp64_mutual_pairs_with_empty_leaves(ph, fp, case):
+    pos, maxleaf = SMALL[case]
+    p = direct_params(maxleaf)
+    check_forces(fp.run(pos, p, precision=ph.FP64), pos, p)
+
+
+@pytest.mark.parametrize("case", range(len(SMALL)))
+@pytest.mark.parametrize("flags", [None, "F_ONE_WAY"])
 def test_fp32_pairs_with_empty_leaves(ph, fp, case, flags):
-    """One way, long lists by a block, against the FP64 pass.  The bars of the clustered inputs (median 1e-5, 99th
+    """Mutual pairs (leaf 64) or one way, long lists by a block, against the
+    FP64 pass.  The bars of the clustered inputs (median 1e-5, 99th
     percentile 1e-4), and for lattices, whose forces cancel, that of the
     golden lattice: 1e-5 of one nearest-neighbour pair force."""
     pos, maxleaf = SMALL[case]
     p = direct_params(maxleaf)
     a64 = fp.run(pos, p, precision=ph.FP64, flags=ph.F_ONE_WAY)
-    a32 = fp.run(pos, p, precision=ph.FP32_SPLIT, flags=getattr(ph, flags))
+    a32 = fp.run(pos, p, precision=ph.FP32_SPLIT, flags=getattr(ph, flags) if flags else 0)
     if case >= 5:
         r = np.linalg.norm(pos[1:] - pos[0], axis=1).min()
         assert np.abs(a32 - a64).max() <= 1e-5 * p["mass"] / r ** 2
