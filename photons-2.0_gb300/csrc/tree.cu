@@ -640,12 +640,27 @@ struct MidTree {
 };
 static_assert(PH_MID / CHUNK <= 8 && PH_MID / MID_SEG <= 32, "one warp holds a node's chunk sums and segment counts");
 
+// Whether the build has failed so far (wide nodes left, too little room or
+// too few levels): node numbers may then have been taken without a record
+// written, so no block goes on from them.  One thread reads, since blocks
+// of the same launch may raise a flag meanwhile, and the block returns as a
+// whole.
+__device__ __forceinline__ bool build_failed(const BuildBufs &b)
+{
+    __shared__ int s_failed;
+    if (threadIdx.x == 0)
+        s_failed = b.cnt[BC_LEVEL_COUNT] > 0 ||
+                   (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH));
+    __syncthreads();
+    return s_failed != 0;
+}
+
 __global__ void __launch_bounds__(MID_TB, 1) k_mid_build(BuildBufs b, int axis0, int maxleaf, int levels)
 {
     ph::chain_begin();
     extern __shared__ __align__(16) unsigned char mid_smem[];
     MidTree &s = *reinterpret_cast<MidTree *>(mid_smem);
-    if (b.cnt[BC_LEVEL_COUNT] > 0 || (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY))) return;
+    if (build_failed(b)) return;
     const int T0 = b.cnt[BC_LEVEL_BEGIN], L0 = b.cnt[BC_LEAVES];
     const int tid = threadIdx.x, lane = warp_lane(), warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -937,7 +952,7 @@ __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0
     ph::chain_begin();
     extern __shared__ __align__(16) unsigned char sub_smem[];
     SubTree &s = *reinterpret_cast<SubTree *>(sub_smem);
-    if (b.cnt[BC_LEVEL_COUNT] > 0 || (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY))) return;
+    if (build_failed(b)) return;
     const int T0 = b.cnt[BC_LEVEL_BEGIN] + b.cnt[BC_MID_NODES], L0 = b.cnt[BC_LEAVES] + b.cnt[BC_MID_LEAVES];
     const int tid = threadIdx.x, warp = tid >> 5;
     int *operm = reinterpret_cast<int *>(s.x);

@@ -524,6 +524,28 @@ def test_tree_around_the_split_sizes_matches_oracle(ph, fp, port, n, maxleaf):
         assert np.array_equal(tr[k], r["tree"][k]), k
 
 
+@pytest.mark.parametrize("n,maxleaf,steps", [(3000, 16, 25), (7000, 8, 40)])
+def test_tree_deeper_than_the_bound_in_a_used_context_matches_oracle(ph, port, n, maxleaf, steps):
+    """A tree whose nodes of more than 1,024 particles go below the depth
+    bound, in a context whose node records are those of a larger tree: the
+    build is repeated with a deeper bound, and its tree is the oracle's."""
+    rng = np.random.default_rng(n)
+    p = dict(boxsize=100.0, theta=0.5, rs=4.0, rcut=18.0, eps=0.1, mass=1.0, maxleaf=maxleaf)
+    fp = ph.ForcePass(0)
+    fp.run(rng.uniform(0.0, 100.0, (7100, 3)), p, precision=ph.FP64)
+    # each split takes one outlier off a tight clump
+    pos = rng.uniform(0.0, 4096.0 ** -(steps + 1.0), (n, 3))
+    pos[:steps] = 90.0 * 4096.0 ** -np.arange(steps)[:, None]
+    r = port.run(pos, p, capture=False, tree=True, nthreads=8)
+    fp.run(pos, p, precision=ph.FP64, flags=ph.F_TREE_ORDER)
+    assert fp.counters()["depth"] > 20
+    assert np.array_equal(fp.positions(), r["pos"])
+    tr = fp.tree()
+    for k in ("leaf_ipart", "leaf_npart", "node_npart", "node_son"):
+        assert np.array_equal(tr[k], r["tree"][k]), k
+    fp.close()
+
+
 @pytest.mark.parametrize("n,maxleaf,spread", [(17, 16, 1.0), (2, 1, 1.0), (40, 1, 1.0), (300, 16, 0.02), (5000, 1, 0.001)])
 def test_walk_of_small_and_deep_trees_matches_oracle(ph, fp, port, n, maxleaf, spread):
     """The walk's queue at its ends: two leaves under one root, fewer targets
