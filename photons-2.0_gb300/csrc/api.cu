@@ -615,7 +615,7 @@ static int estimate_levels(int n, int maxleaf)
     return lv < MAX_DEPTH_CAP - 1 ? lv : MAX_DEPTH_CAP - 1;
 }
 
-// levels of wide nodes (more than PH_MID particles) to launch: none if every
+// levels of wide nodes (more than b.mid particles) to launch: none if every
 // box is smaller, else the last build's need with a margin, else an estimate
 // from the largest; never above the depth bound
 static int tree_top(const photons_ctx *c, int levels)
@@ -726,6 +726,8 @@ static int ph_prepare_boxes(photons_ctx *c, int nbox, const photons_params *p, c
     // (build, 2,097,152 near-uniform particles: 1.08 ms either way; 250,047
     // half in halos 0.83 -> 0.70; 256^3 5.05 -> 5.32)
     c->b.mid = n <= (1 << 21) ? PH_MID : CHUNK_ELEMS;
+    c->b.sub = CHUNK_ELEMS;
+    if (c->sub_n == (int)n && c->sub_leaf == p->maxleaf) c->b.mid = c->b.sub = PH_SUB_SMALL;
     c->pp.boxsize = p->boxsize;
     c->pp.theta = p->theta;
     c->pp.rs = p->rs;
@@ -772,7 +774,7 @@ static int ph_enqueue_tree(photons_ctx *c, const double *src, int levels)
 }
 
 // build flags after the stream has finished: capacity overflow is an error
-// of the reference's rule; PH_FLAG_TOP asks for more levels of wide nodes,
+// of the reference's rule; PH_FLAG_SUBTREE asks for smaller subtrees; PH_FLAG_TOP asks for more levels of wide nodes,
 // PH_FLAG_DEPTH for a deeper bound (*grow: the bound to build again with)
 static int ph_check_build(photons_ctx *c, int flags, int levels, int *grow)
 {
@@ -781,6 +783,16 @@ static int ph_check_build(photons_ctx *c, int flags, int levels, int *grow)
         return ph_set_error(PH_ERR_CAPACITY, "leaf capacity 2N/MAXLEAF=%d exceeded by the mean-split tree", c->b.rule_cap);
     if (flags & PH_FLAG_NODE_CAPACITY)
         return ph_set_error(PH_ERR_CAPACITY, "node capacity 2N/MAXLEAF=%d exceeded by the mean-split tree", c->b.rule_cap);
+    if (flags & PH_FLAG_SUBTREE) {
+        if (c->b.sub == PH_SUB_SMALL)
+            return ph_set_error(PH_ERR_DEPTH, "more than %d nodes over %d particles", CHUNK_ELEMS, PH_SUB_SMALL);
+        c->sub_n = c->n;
+        c->sub_leaf = c->pp.maxleaf;
+        c->b.mid = c->b.sub = PH_SUB_SMALL;
+        c->hint_top = 0;
+        *grow = levels;
+        return 0;
+    }
     if (flags & (PH_FLAG_DEPTH | PH_FLAG_TOP)) {
         const int top = tree_top(c, levels);
         if (flags & PH_FLAG_TOP) c->hint_top = top * 2 > top + 4 ? top * 2 : top + 4;
@@ -1105,6 +1117,7 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
     k.dio = dio; k.variant = p2p_variant(); k.nwarps = c->w.nwarps; k.mask = mask;
     k.stage_extra = stage_shortfall();
     k.far = capture_far(c, p);
+    k.sub = c->b.sub;
     k.boxsize = p->boxsize; k.theta = p->theta; k.rs = p->rs; k.rcut = p->rcut; k.eps = p->eps; k.mass = p->mass;
     k.pos = dio ? (const void *)pos : nullptr;
     k.acc = dio ? (const void *)acc : nullptr;
@@ -1268,7 +1281,7 @@ __global__ void k_pass_failed(const int *tree_cnt, const unsigned long long *wal
                               int *out)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0)
-        *out = (tree_cnt[ph::BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH | PH_FLAG_TOP)) ||
+        *out = (tree_cnt[ph::BC_FLAGS] & PH_FLAGS_TREE) ||
                walk_ctr[ph::WC_FLAGS] != 0 || *mu_over != 0 ||
                (no_far && walk_ctr[ph::WC_M2L_LOCAL] + walk_ctr[ph::WC_M2L_IMAGE] > 0);
 }

@@ -30,7 +30,7 @@ enum {
 // Everything a captured pass bakes in; a pass with a different key is
 // captured anew.  Zero-filled before use so it compares with memcmp.
 struct PassKey {
-    int n, nbox, levels, top, maxleaf, precision, flags, dio, variant, nwarps, stage_extra, far;
+    int n, nbox, levels, top, maxleaf, precision, flags, dio, variant, nwarps, stage_extra, far, sub;
     unsigned mask;
     double boxsize, theta, rs, rcut, eps, mass;
     const void *pos, *acc;
@@ -120,6 +120,7 @@ struct photons_ctx {
     // the captured pass
     bool capturing = false, have_key = false;
     cudaGraphExec_t gexec = nullptr;
+    int sub_n = 0, sub_leaf = 0;  // the pass (particles, MAXLEAF) that last took small subtrees
     int far_idle = 0;  // captured passes in a row without an M2L task
     unsigned long long graph_kernels = 0;  // kernel nodes of gexec
     PassKey key{};

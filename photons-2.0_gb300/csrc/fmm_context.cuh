@@ -45,6 +45,7 @@ struct BuildBufs {
     size_t scan_scratch_elems = 0;
     int cap_nodes = 0, cap_leaves = 0, cap_chunks = 0, cap_n = 0;
     int mid = 0;       // this build: nodes of at most this many particles are not split by the levels
+    int sub = 0;       // this build: nodes of at most this many particles root a block's subtree (<= mid)
     int rule_cap = 0;  // this pass's 2N/MAXLEAF capacity (src/fmm.c:203-209), <= cap_nodes
     int *level_begin_h = nullptr;  // host copy, per level
     // boxes: temp node / leaf -> box, and the per-box table
@@ -81,6 +82,10 @@ enum BuildCounter {
 // nodes of at most this many particles are split in shared memory (30 bytes a
 // particle, 210 KB)
 #define PH_MID 7168
+
+// subtrees of a build that is repeated because one of 1,024 particles had
+// too many nodes: at most three nodes a particle fit
+#define PH_SUB_SMALL 256
 
 // deepest tree the depth lists hold (depths 0..PH_MAX_DEPTH_CAP-1)
 #define PH_MAX_DEPTH_CAP 2048

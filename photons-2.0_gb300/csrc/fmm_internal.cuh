@@ -39,7 +39,11 @@
 #define PH_FLAG_NODE_CAPACITY 16u
 #define PH_FLAG_DEPTH 32u
 #define PH_FLAG_WALK_WAIT 128u  // a walk warp gave up waiting for its target
+#define PH_FLAG_SUBTREE 256u  // a subtree of more nodes or leaves than one block holds
 #define PH_FLAG_TOP 64u  // wide nodes left after the launched levels of the tree build
+// a tree that was not built
+#define PH_FLAGS_TREE \
+    (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH | PH_FLAG_SUBTREE | PH_FLAG_TOP)
 
 struct PassParams {
     double boxsize, theta, rs, rcut, eps, mass;

@@ -19,8 +19,9 @@
 //      of the next level; child boxes come from the split plane.
 // A node of at most mid particles (PH_MID, or CHUNK in large builds) is not
 // split by the levels: one block holds its particles in shared memory and
-// splits it down to nodes of at most CHUNK (k_mid_build), and each of those roots a subtree that one block
-// builds whole (k_subtree_build), every node of it split by one warp.  Both
+// splits it down to nodes of at most sub, CHUNK (k_mid_build), and each of
+// those roots a subtree that one block builds whole (k_subtree_build), every
+// node of it split by one warp.  Both
 // use the arithmetic of the levels (sums over chunks of CHUNK in the same
 // order), so the tree is the one a build that splits every depth level by
 // level makes.
@@ -91,7 +92,7 @@ __device__ __forceinline__ long long order_key(double x)
 // the state of a node of len particles not yet split
 __device__ __forceinline__ int open_mode(const BuildBufs &b, int len)
 {
-    return len <= CHUNK ? MODE_DEFERRED : (len <= b.mid ? MODE_MID : MODE_PENDING);
+    return len <= b.sub ? MODE_DEFERRED : (len <= b.mid ? MODE_MID : MODE_PENDING);
 }
 
 __global__ void k_init_roots(BuildBufs b, int n, int top)
@@ -499,7 +500,7 @@ __global__ void k_tree_totals(BuildBufs b)
         if (b.cnt[BC_LEVEL_COUNT] > 0) b.cnt[BC_FLAGS] |= PH_FLAG_TOP;
         b.cnt[BC_NODES] = b.cnt[BC_LEVEL_BEGIN] + b.cnt[BC_MID_NODES] + b.cnt[BC_SUB_NODES];
         b.cnt[BC_LEAVES] += b.cnt[BC_MID_LEAVES] + b.cnt[BC_SUB_LEAVES];
-        if (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH | PH_FLAG_TOP)) {
+        if (b.cnt[BC_FLAGS] & PH_FLAGS_TREE) {
             b.cnt[BC_NODES] = 0;
             b.cnt[BC_LEAVES] = 0;
             b.cnt[BC_NLEVELS] = 0;
@@ -650,7 +651,7 @@ __device__ __forceinline__ bool build_failed(const BuildBufs &b)
     __shared__ int s_failed;
     if (threadIdx.x == 0)
         s_failed = b.cnt[BC_LEVEL_COUNT] > 0 ||
-                   (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH));
+                   (b.cnt[BC_FLAGS] & (PH_FLAG_LEAF_CAPACITY | PH_FLAG_NODE_CAPACITY | PH_FLAG_DEPTH | PH_FLAG_SUBTREE));
     __syncthreads();
     return s_failed != 0;
 }
@@ -830,7 +831,11 @@ __global__ void __launch_bounds__(MID_TB, 1) k_mid_build(BuildBufs b, int axis0,
 }
 
 // ---------------- subtrees of at most CHUNK particles ----------------
-// Shared memory of one subtree block, 53.3 KB: four blocks per SM.
+// Shared memory of one subtree block, 53.3 KB: four blocks per SM.  The
+// arrays hold CHUNK nodes and leaves.  Subtrees with empty leaves can have
+// more (a line of particles: up to three nodes a particle, two of the three
+// axes splitting nothing off); the build is then repeated with subtrees of
+// at most PH_SUB_SMALL particles, the rest split by the levels.
 struct SubTree {
     // the subtree's particles; once written back, the region holds the
     // original permutation (bytes 0-4095) and the parents
@@ -849,6 +854,7 @@ struct SubTree {
     // k_subtree_build)
     int nalloc[3];
     int nleaves, fail, nbase, lbase;
+    int large;  // more nodes or leaves than the arrays hold
 };
 
 __device__ __forceinline__ void sub_swap(SubTree &s, int i, int j)
@@ -917,18 +923,29 @@ __device__ void sub_split_node(SubTree &s, int i, int depth, int L, int lend, in
         int off = ns;
         for (int ch = 0; ch < 2; ch++) {
             int code;
+            // a node below the launched depths fails the subtree, and so does
+            // a node or leaf beyond the arrays
             if (sizes[ch] <= maxleaf) {
                 const int j = atomicAdd(&s.nleaves, 1);
-                s.l_start[j] = (unsigned short)off;
-                s.l_len[j] = (unsigned short)sizes[ch];
                 code = ~j;
+                if (j < CHUNK) {
+                    s.l_start[j] = (unsigned short)off;
+                    s.l_len[j] = (unsigned short)sizes[ch];
+                } else {
+                    atomicAdd(&s.nalloc[(L + 1) % 3], SUB_FAIL);
+                    s.large = 1;
+                }
             } else {
-                // a node below the launched depths fails the subtree
-                const int j = lend + (atomicAdd(&s.nalloc[(L + 1) % 3], depth + 1 >= levels ? SUB_FAIL + 1 : 1) &
-                                      (SUB_FAIL - 1));
-                s.n_start[j] = (unsigned short)off;
-                s.n_len[j] = (unsigned short)sizes[ch];
+                const bool deep = depth + 1 >= levels;
+                const int j = lend + (atomicAdd(&s.nalloc[(L + 1) % 3], deep ? SUB_FAIL + 1 : 1) & (SUB_FAIL - 1));
                 code = j;
+                if (j < CHUNK) {
+                    s.n_start[j] = (unsigned short)off;
+                    s.n_len[j] = (unsigned short)sizes[ch];
+                } else {
+                    atomicAdd(&s.nalloc[(L + 1) % 3], SUB_FAIL);
+                    s.large = 1;
+                }
             }
             if (ch == 0) s.n_c0[i] = (short)code;
             else s.n_c1[i] = (short)code;
@@ -973,6 +990,7 @@ __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0
             s.n_len[0] = (unsigned short)len;
             s.lev[0] = 0;
             s.fail = 0;
+            s.large = 0;
         }
         __syncthreads();
         int failed = rd >= levels;
@@ -991,7 +1009,7 @@ __global__ void __launch_bounds__(SUB_TB) k_subtree_build(BuildBufs b, int axis0
         }
         __syncthreads();  // lev[] complete
         if (failed) {
-            if (tid == 0) atomicOr(&b.cnt[BC_FLAGS], PH_FLAG_DEPTH);
+            if (tid == 0) atomicOr(&b.cnt[BC_FLAGS], s.large ? PH_FLAG_SUBTREE : PH_FLAG_DEPTH);
             continue;  // the next subtree's first writes follow a barrier all threads passed
         }
         for (int k = tid; k < len; k += SUB_TB) {

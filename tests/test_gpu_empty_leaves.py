@@ -191,3 +191,23 @@ def test_numbering_of_large_trees_with_empty_leaves(ph, fp, n, z, background, ma
     p = dict(boxsize=L, theta=0.5, rs=0.5, rcut=2.25, eps=0.01, mass=1.0, maxleaf=maxleaf)
     fp.run(pos, p, precision=ph.FP64, flags=ph.F_ONE_WAY)
     check_tree(fp, pos, maxleaf)
+
+
+@pytest.mark.parametrize("graph", ["1", "0"])
+def test_subtree_with_more_leaves_than_one_block_holds(ph, graph, monkeypatch):
+    """A line of 1,000 particles whose y and z splits are empty, beside 1,500
+    others: 1,240 leaves under a node of 1,000 particles.  Also the pass
+    after it (which starts from the small subtrees) and an ordinary one."""
+    monkeypatch.setenv("PHOTONS_GRAPH", graph)
+    rng = np.random.default_rng(5)
+    pos = rng.uniform(0.0, 50.0, (2500, 3)) * (1.0, 2.0, 2.0)
+    pos[1500:] = (0.0, 54.723, 56.247)
+    pos[1500:, 0] = rng.uniform(90.0, 100.0, 1000)
+    p = dict(boxsize=L, theta=0.5, rs=2.0, rcut=9.0, eps=0.1, mass=1.0, maxleaf=2)
+    fp = ph.ForcePass(0)
+    for _ in range(2):
+        fp.run(pos, p, precision=ph.FP64)
+        check_tree(fp, pos, 2)
+    fp.run(sheet(3000, 1.3), dict(p, maxleaf=16), precision=ph.FP64)
+    check_tree(fp, sheet(3000, 1.3), 16)
+    fp.close()
