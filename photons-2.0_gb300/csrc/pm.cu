@@ -60,10 +60,16 @@ __device__ __forceinline__ size_t cell(int i, int j, int k, int N) { return ((si
 // 2^-62.  (The exact centre instead took 8 us less and halved the error
 // against extended precision, but left the reference's rounding: 2.2e-15
 // against 1.4e-15 of the FP64 evaluation's forces.)
+// A particle more than half a cell below the box has weights the reference
+// leaves outside [0, 1] (its cell index is truncated towards zero, so the
+// distance to the centre is up to 1.5 cells and the neighbour's weight
+// negative): its weights are doubles, held as bit patterns.
+enum { CIC_FIXED = 0, CIC_SIGNED = 1, CIC_NAN = 2 };
+
 struct CicFix {
     int i, j, k, ii, jj, kk;
     unsigned long long wi, wj, wk, win, wjn, wkn;
-    bool finite;
+    int kind;
 };
 
 // N / L and its inverse: mantissas (64 bits with the top one set, 53 bits)
@@ -76,7 +82,7 @@ struct Norm64 {
 };
 
 __device__ __forceinline__ void cic_axis_fix(double x, const Norm64 &q, int N, int &c, int &cn, unsigned long long &w,
-                                             unsigned long long &wn, bool &finite)
+                                             unsigned long long &wn, int &kind)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const int ex = (int)(b >> 52);  // with the sign: negative x has ex >= 2048
@@ -107,22 +113,36 @@ __device__ __forceinline__ void cic_axis_fix(double x, const Norm64 &q, int N, i
     } else if (isfinite(x)) {  // below the box, or many cells above its lower edge
         double v, vn;
         cic_axis(x, q.norm, q.delta, N, c, cn, v, vn);
+        if (vn < 0.0) kind = max(kind, (int)CIC_SIGNED);
         w = __double2ull_rn(v * 9223372036854775808.0);  // 2^63
         wn = __double2ull_rn(vn * 9223372036854775808.0);
     } else {
         c = cn = 0;
         w = wn = 0;
-        finite = false;
+        kind = CIC_NAN;
     }
 }
 
 __device__ __forceinline__ CicFix cic_fix(const double *pos, int p, const Norm64 &q, int N)
 {
     CicFix s;
-    s.finite = true;
-    cic_axis_fix(pos[3 * (size_t)p], q, N, s.i, s.ii, s.wi, s.win, s.finite);
-    cic_axis_fix(pos[3 * (size_t)p + 1], q, N, s.j, s.jj, s.wj, s.wjn, s.finite);
-    cic_axis_fix(pos[3 * (size_t)p + 2], q, N, s.k, s.kk, s.wk, s.wkn, s.finite);
+    s.kind = CIC_FIXED;
+    const double x = pos[3 * (size_t)p], y = pos[3 * (size_t)p + 1], z = pos[3 * (size_t)p + 2];
+    cic_axis_fix(x, q, N, s.i, s.ii, s.wi, s.win, s.kind);
+    cic_axis_fix(y, q, N, s.j, s.jj, s.wj, s.wjn, s.kind);
+    cic_axis_fix(z, q, N, s.k, s.kk, s.wk, s.wkn, s.kind);
+    if (s.kind == CIC_SIGNED) {
+        double w[3], wn[3];
+        cic_axis(x, q.norm, q.delta, N, s.i, s.ii, w[0], wn[0]);
+        cic_axis(y, q.norm, q.delta, N, s.j, s.jj, w[1], wn[1]);
+        cic_axis(z, q.norm, q.delta, N, s.k, s.kk, w[2], wn[2]);
+        s.wi = __double_as_longlong(w[0]);
+        s.wj = __double_as_longlong(w[1]);
+        s.wk = __double_as_longlong(w[2]);
+        s.win = __double_as_longlong(wn[0]);
+        s.wjn = __double_as_longlong(wn[1]);
+        s.wkn = __double_as_longlong(wn[2]);
+    }
     return s;
 }
 
@@ -132,6 +152,12 @@ __device__ __forceinline__ unsigned long long wmul(unsigned long long a, unsigne
     return __umul64hi(a, b) << 1;
 }
 
+// of two weights of a CIC_SIGNED particle
+__device__ __forceinline__ unsigned long long wmul_signed(unsigned long long a, unsigned long long b)
+{
+    return __double_as_longlong(__dmul_rn(__longlong_as_double(a), __longlong_as_double(b)));
+}
+
 // a weight (2^-63 units, at most 2^63) as a double, rounded to nearest
 __device__ __forceinline__ double weight_d(unsigned long long v)
 {
@@ -139,6 +165,13 @@ __device__ __forceinline__ double weight_d(unsigned long long v)
     const unsigned long long m = v << (lz & 63);
     const unsigned long long r = (m >> 11) + ((m >> 10) & 1);  // with the leading bit
     return v ? __longlong_as_double((long long)(((unsigned long long)(1022 - lz) << 52) + r)) : 0.0;
+}
+
+// a corner's weight from its xy and z parts
+__device__ __forceinline__ double corner_d(unsigned long long xy, unsigned long long z, int kind)
+{
+    if (kind == CIC_FIXED) return weight_d(wmul(xy, z));
+    return kind == CIC_SIGNED ? __longlong_as_double(wmul_signed(xy, z)) : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // A warp takes 32 particles; two lanes then add one particle's corners, one
@@ -153,10 +186,14 @@ __global__ void k_pm_deposit(const double *__restrict__ pos, int n, int N, Norm6
     for (int p0 = blockIdx.x * blockDim.x + threadIdx.x - lane; p0 < n; p0 += step) {
         const int p = p0 + lane;
         CicFix s{};
-        s.finite = true;
         if (p < n) s = cic_fix(pos, p, q, N);
-        const unsigned long long nn = wmul(s.win, s.wjn), in = wmul(s.wi, s.wjn), nj = wmul(s.win, s.wj),
-                                 ij = wmul(s.wi, s.wj);
+        unsigned long long nn = wmul(s.win, s.wjn), in = wmul(s.wi, s.wjn), nj = wmul(s.win, s.wj), ij = wmul(s.wi, s.wj);
+        if (s.kind == CIC_SIGNED) {
+            nn = wmul_signed(s.win, s.wjn);
+            in = wmul_signed(s.wi, s.wjn);
+            nj = wmul_signed(s.win, s.wj);
+            ij = wmul_signed(s.wi, s.wj);
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int src = (lane & ~1) | h;
@@ -167,15 +204,14 @@ __global__ void k_pm_deposit(const double *__restrict__ pos, int n, int N, Norm6
             const unsigned long long z0 = __shfl_sync(0xffffffffu, s.wkn, src), z1 = __shfl_sync(0xffffffffu, s.wk, src);
             const unsigned long long a = __shfl_sync(0xffffffffu, nn, src), b = __shfl_sync(0xffffffffu, in, src);
             const unsigned long long c = __shfl_sync(0xffffffffu, nj, src), d = __shfl_sync(0xffffffffu, ij, src);
-            const bool ok = __shfl_sync(0xffffffffu, (int)s.finite, src);
+            const int kind = __shfl_sync(0xffffffffu, s.kind, src);
             if (p0 + src >= n) continue;
             const int k = odd ? k1 : k0;
             const unsigned long long z = odd ? z1 : z0;
-            const double nan = __longlong_as_double(0x7ff8000000000000LL);
-            atomicAdd(rho + cell(pi, pj, k, N), ok ? weight_d(wmul(a, z)) : nan);
-            atomicAdd(rho + cell(pii, pj, k, N), ok ? weight_d(wmul(b, z)) : nan);
-            atomicAdd(rho + cell(pi, pjj, k, N), ok ? weight_d(wmul(c, z)) : nan);
-            atomicAdd(rho + cell(pii, pjj, k, N), ok ? weight_d(wmul(d, z)) : nan);
+            atomicAdd(rho + cell(pi, pj, k, N), corner_d(a, z, kind));
+            atomicAdd(rho + cell(pii, pj, k, N), corner_d(b, z, kind));
+            atomicAdd(rho + cell(pi, pjj, k, N), corner_d(c, z, kind));
+            atomicAdd(rho + cell(pii, pjj, k, N), corner_d(d, z, kind));
         }
     }
 }
@@ -293,6 +329,25 @@ __global__ void k_pm_interp(const double *__restrict__ pos, int n, int N, Norm64
         int e = 1;
 #pragma unroll
         for (int o = 0; o < 8; o++) e = max(e, (int)c[o].w);
+        // sums are in units of 2^(e - 1078); two factors stay inside the range of doubles
+        const int h = (e - 1078) >> 1, h2 = e - 1078 - h;
+        const double f2 = __longlong_as_double((long long)(h2 + 1023) << 52);
+        const double f = s.kind != CIC_NAN && e < 2047 ? invx6 * __longlong_as_double((long long)(h + 1023) << 52)
+                                                       : __longlong_as_double(0x7ff8000000000000LL);
+        if (s.kind == CIC_SIGNED) {
+            double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int o = 0; o < 8; o++) {
+                const unsigned long long xy = wmul_signed((o & 1) ? s.wi : s.win, (o & 2) ? s.wj : s.wjn);
+                const double w = __longlong_as_double(wmul_signed(xy, (o & 4) ? s.wk : s.wkn));
+                const int up = (int)c[o].w - e - 2;
+                v[0] = fma(w, ldexp((double)c[o].x, up), v[0]);
+                v[1] = fma(w, ldexp((double)c[o].y, up), v[1]);
+                v[2] = fma(w, ldexp((double)c[o].z, up), v[2]);
+            }
+            for (int d = 0; d < 3; d++) acc[3 * (size_t)p + d] = v[d] * f * f2;
+            continue;
+        }
         const unsigned long long xy[4] = {wmul(s.win, s.wjn), wmul(s.wi, s.wjn), wmul(s.win, s.wj), wmul(s.wi, s.wj)};
         long long ax = 4, ay = 4, az = 4;  // eight products are cut off below: half a unit each
 #pragma unroll
@@ -303,11 +358,6 @@ __global__ void k_pm_interp(const double *__restrict__ pos, int n, int N, Norm64
             ay += __mul64hi(c[o].y, w) >> sh;
             az += __mul64hi(c[o].z, w) >> sh;
         }
-        // sums are in units of 2^(e - 1078); two factors stay inside the range of doubles
-        const int h = (e - 1078) >> 1, h2 = e - 1078 - h;
-        const double f2 = __longlong_as_double((long long)(h2 + 1023) << 52);
-        const double f = s.finite && e < 2047 ? invx6 * __longlong_as_double((long long)(h + 1023) << 52)
-                                              : __longlong_as_double(0x7ff8000000000000LL);
         acc[3 * (size_t)p] = (double)ax * f * f2;
         acc[3 * (size_t)p + 1] = (double)ay * f * f2;
         acc[3 * (size_t)p + 2] = (double)az * f * f2;

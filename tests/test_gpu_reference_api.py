@@ -248,6 +248,24 @@ def test_pm_weights_at_cell_edges_match_oracle(ph, nside, L):
     assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("nside,L", [(5, 1.0), (37, 10.0), (64, 3.0e-7)])
+def test_pm_of_positions_below_the_box_matches_oracle(ph, nside, L):
+    """Positions up to 2.9 cells below the box, where the reference's
+    truncated cell index gives weights between -0.5 and 1.5: the bar above."""
+    import pm_oracle
+    rng = np.random.default_rng(nside)
+    h = L / nside
+    below = np.concatenate([[-0.75 * h, -1.6 * h, -0.5 * h, -1.5 * h, -h, np.nextafter(-0.5 * h, -L)],
+                            rng.uniform(-2.9 * h, 0.0, 200)])
+    pos = np.concatenate([rng.choice(below, (300, 3)), rng.uniform(0.0, L, (300, 3))])
+    pos[300:500, 1] = rng.choice(below, 200)
+    p = dict(boxsize=L, theta=0.5, rs=1.25 * h, rcut=6.0 * h, eps=0.0, mass=2.5, maxleaf=16)
+    with contextlib.closing(ph.ForcePass(0)) as fp:
+        got = fp.pm_force(pos, p, nside)
+    want = pm_oracle.pm_force(pos, L, nside, p["rs"], p["mass"])
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
+
+
 def test_pm_of_a_position_that_is_not_finite_is_nan(ph):
     pos = np.random.default_rng(0).uniform(0.0, 8.0, (50, 3))
     pos[7, 1] = np.nan
