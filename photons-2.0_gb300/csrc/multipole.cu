@@ -104,10 +104,24 @@ __global__ void k_p2m(const double *px, const double *py, const double *pz, cons
 }
 
 // ---------------- M2M (one depth, parents gather their two children) ----------------
+// d^e(i) / e(i)! as (first two factors) (third / e(i)!): the order of the
+// lanes' monomials below
+__device__ __forceinline__ void paired_monomials(double dx, double dy, double dz, double *out)
+{
+    const double x[4] = {dx, dy, dz, 1.0};
+#pragma unroll
+    for (int i = 0; i < PH_NMULTI; i++) {
+        const int e0 = h_mi.e[i][0], e1 = e0 + h_mi.e[i][1], e2 = e1 + h_mi.e[i][2];
+        const int f0 = e0 > 0 ? 0 : (e1 > 0 ? 1 : (e2 > 0 ? 2 : 3)), f1 = e0 > 1 ? 0 : (e1 > 1 ? 1 : (e2 > 1 ? 2 : 3)),
+                  f2 = e0 > 2 ? 0 : (e1 > 2 ? 1 : (e2 > 2 ? 2 : 3));
+        out[i] = __dmul_rn(__dmul_rn(x[f0], x[f1]), __dmul_rn(x[f2], h_mi.invf[i]));
+    }
+}
+
 __device__ __forceinline__ void m2m_add(double dx, double dy, double dz, const double *Mc, double *out)
 {
     double mono[PH_NMULTI];
-    scaled_monomials(dx, dy, dz, mono);
+    paired_monomials(dx, dy, dz, mono);
 #pragma unroll
     for (int a = 0; a < PH_NMULTI; a++) {
         double s = 0.0;
@@ -116,7 +130,7 @@ __device__ __forceinline__ void m2m_add(double dx, double dy, double dz, const d
             const int g0 = h_mi.e[a][0] - h_mi.e[b][0], g1 = h_mi.e[a][1] - h_mi.e[b][1],
                       g2 = h_mi.e[a][2] - h_mi.e[b][2];
             if (g0 < 0 || g1 < 0 || g2 < 0) continue;
-            s += Mc[b] * mono[h_mi.idx[g0][g1][g2]];
+            s = fma(Mc[b], mono[h_mi.idx[g0][g1][g2]], s);
         }
         out[a] += s;
     }
@@ -131,6 +145,9 @@ __device__ __forceinline__ void m2m_add(double dx, double dy, double dz, const d
 // ~64 cycles).  Per launch at 250,047 halo particles (23 depths), threads
 // alone -> both forms: M2M 14.3 -> 8.2 us, L2L 10.0 -> 8.2; at 2,097,152 (26
 // depths) 11.3 and 11.2.
+// A depth holds the nodes of all boxes of a pass, so which form a box gets
+// depends on the others; both make the same roundings in the same order, and
+// a box's forces do not.
 #define WIDE_DEPTH 5000
 
 // Per lane, packed a byte each: the terms of its component.  M2M: M_b
@@ -209,13 +226,10 @@ __device__ __forceinline__ double m2m_lanes(double m, double mono, OpWarp &w, co
         w.mono[lane] = mono;
     }
     __syncwarp();
-    double v = 0.0, u = 0.0;
+    double v = 0.0;
 #pragma unroll
-    for (int n = 0; n < 8; n += 2) {
-        v = fma(w.src[term(tb, n)], w.mono[term(tg, n)], v);
-        u = fma(w.src[term(tb, n + 1)], w.mono[term(tg, n + 1)], u);
-    }
-    return v + u;
+    for (int n = 0; n < 8; n++) v = fma(w.src[term(tb, n)], w.mono[term(tg, n)], v);
+    return v;
 }
 
 __global__ void k_m2m_depth(const int *list, const int *depth_off, int d, const int *tree_cnt, const int *son0,
@@ -409,13 +423,9 @@ __global__ void k_l2l_depth(const int *list, const int *depth_off, int d, const 
                 w.mono[lane] = mono;
             }
             __syncwarp();
-            double v = 0.0, q = 0.0;
+            double v = 0.0;
 #pragma unroll
-            for (int n = 0; n < 10; n += 2) {
-                v = fma(w.src[term(tl, n)], w.mono[term(tg, n)], v);
-                q = fma(w.src[term(tl, n + 1)], w.mono[term(tg, n + 1)], q);
-            }
-            v += q;
+            for (int n = 0; n < 10; n++) v = fma(w.src[term(tl, n)], w.mono[term(tg, n)], v);
             const double second = __shfl_sync(0xffffffffu, v, PH_NMULTI);  // the second half of component 0
             if (lane == 0) v += second;
             if (lane < PH_NMULTI) L[(size_t)u * PH_NMULTI + lane] = own + v;
@@ -427,20 +437,22 @@ __global__ void k_l2l_depth(const int *list, const int *depth_off, int d, const 
         int p = parent[u];
         if (p < 0) continue;
         double mono[PH_NMULTI];
-        scaled_monomials(cx[u] - cx[p], cy[u] - cy[p], cz[u] - cz[p], mono);
+        paired_monomials(cx[u] - cx[p], cy[u] - cy[p], cz[u] - cz[p], mono);
         double Lp[PH_NMULTI];
 #pragma unroll
         for (int a = 0; a < PH_NMULTI; a++) Lp[a] = L[(size_t)p * PH_NMULTI + a];
 #pragma unroll
         for (int b = 0; b < PH_NMULTI; b++) {
-            double s = 0.0;
+            double s[2] = {0.0, 0.0};  // the first ten terms, the others
+            int n = 0;
 #pragma unroll
             for (int g = 0; g < PH_NMULTI; g++) {
                 if (h_mi.ord[b] + h_mi.ord[g] > 3) continue;
-                s += Lp[h_mi.idx[h_mi.e[b][0] + h_mi.e[g][0]][h_mi.e[b][1] + h_mi.e[g][1]][h_mi.e[b][2] + h_mi.e[g][2]]] *
-                     mono[g];
+                const int k = n++ < 10 ? 0 : 1;
+                s[k] = fma(Lp[h_mi.idx[h_mi.e[b][0] + h_mi.e[g][0]][h_mi.e[b][1] + h_mi.e[g][1]]
+                                      [h_mi.e[b][2] + h_mi.e[g][2]]], mono[g], s[k]);
             }
-            L[(size_t)u * PH_NMULTI + b] += s;
+            L[(size_t)u * PH_NMULTI + b] += b == 0 ? s[0] + s[1] : s[0];
         }
     }
 }

@@ -53,6 +53,23 @@ def test_boxes_mutual_pairs_match_separate_passes(ph, ics, maxleaf):
         assert np.array_equal(g, one.run(pos, p, precision=ph.FP32_SPLIT))
 
 
+@pytest.mark.parametrize("precision", ["FP64", "FP32_SPLIT"])
+def test_boxes_of_wide_depths_match_separate_passes(ph, ics, precision):
+    """A batch with depths of tens of thousands of nodes, each box alone far
+    below: the far field's translations take a thread per target in the
+    batch and a warp per target alone, with the same roundings."""
+    prec = getattr(ph, precision)
+    boxes = [(pos, dict(p, maxleaf=4, theta=0.6))
+             for pos, p in ics.plummer_boxes(nbox=20, seed=8, nmin=20 ** 3, nmax=24 ** 3)]
+    fp = ph.ForcePass(0)
+    got = fp.run_boxes(boxes, precision=prec)
+    assert fp.counters()["n_m2l"] > 0 and fp.counters()["nnode"] > 8 * 5000
+    one = ph.ForcePass(0)
+    for (pos, p), g in zip(boxes, got):
+        assert np.array_equal(g, one.run(pos, p, precision=prec))
+        assert one.counters()["nnode"] < 5000
+
+
 def test_boxes_graph_and_stage_paths_agree(ph, ics, monkeypatch):
     boxes = _boxes(ics, nbox=4)
     a = ph.ForcePass(0).run_boxes(boxes, precision=ph.FP32_SPLIT)
