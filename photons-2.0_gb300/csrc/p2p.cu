@@ -474,22 +474,13 @@ __device__ __forceinline__ int ow_stage(const P2PArgs &A, const uint32_t *list, 
     return nfit;
 }
 
-// compensated sums (s - c): b added to a, the rounding of s + s' kept in c
-__device__ __forceinline__ void comp_merge(float2 &a, float2 b)
+// the streams of each target (lanes equal modulo m) added up in FP64, in a
+// fixed tree: compensated sums (s, c) of FP32 terms in, their sum out
+__device__ __forceinline__ double comp_streams(float2 sc, int m)
 {
-    const float t = a.x + b.x, v = t - a.x;
-    const float err = (a.x - (t - v)) + (b.x - v);
-    a = make_float2(t, (a.y + b.y) - err);
-}
-
-// the streams of each target (lanes equal modulo m) into one, in a fixed tree
-__device__ __forceinline__ void comp_streams(float2 *v, int m)
-{
-    for (int o = m; o < 32; o <<= 1) {
-#pragma unroll
-        for (int d = 0; d < 3; d++)
-            comp_merge(v[d], make_float2(__shfl_xor_sync(0xffffffffu, v[d].x, o), __shfl_xor_sync(0xffffffffu, v[d].y, o)));
-    }
+    double v = (double)sc.x - (double)sc.y;
+    for (int o = m; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // Leaves whose lists are long against a warp's even share of their box's
@@ -621,32 +612,39 @@ __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A
                 __syncwarp();
             }
             // the streams of each target, then the group's warps, in a fixed order
-            comp_streams(v1, m1);
-            if (m2) comp_streams(v2, m2);
-            const double acc_scale = B.acc_scale;
-            double *const out[3] = {A.ax + it + tb, A.ay + it + tb, A.az + it + tb};
-            if (W == 1) {
+            double *const out[3] = {A.ax, A.ay, A.az};
+            // the warps' sums through their stages, [3][64] each
+            double *red = reinterpret_cast<double *>(sx);
+            static_assert(3 * 64 * sizeof(double) <= sizeof s_x[0], "the sums fit a stage");
 #pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    if (lane < m1) out[d][lane] += ((double)v1[d].x - (double)v1[d].y) * acc_scale;
-                    if (lane < rest) out[d][m1 + lane] += ((double)v2[d].x - (double)v2[d].y) * acc_scale;
+            for (int d = 0; d < 3; d++) {
+                // lane l has the sum of target l modulo the round's width, so up to 32
+                // targets are a lane each
+                double v = comp_streams(v1[d], m1);
+                if (m1 < 32 && m2) {
+                    const double v_2 = comp_streams(v2[d], m2);
+                    if (lane >= m1) v = v_2;
                 }
-            } else {
-                // the warps' sums through their stages, [3][64] each
-                float2 *red = reinterpret_cast<float2 *>(sx);
-                static_assert(3 * 64 * sizeof(float2) <= sizeof s_x[0], "the sums fit a stage");
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    if (lane < m1) red[64 * d + lane] = v1[d];
-                    if (lane < rest) red[64 * d + m1 + lane] = v2[d];
+                if (lane < nb) {
+                    if (W == 1) out[d][it + tb + lane] += v * B.acc_scale;
+                    else red[64 * d + lane] = v;
                 }
+                if (m1 == 32 && m2) {
+                    v = comp_streams(v2[d], m2);
+                    if (lane < rest) {
+                        if (W == 1) out[d][it + tb + 32 + lane] += v * B.acc_scale;
+                        else red[64 * d + 32 + lane] = v;
+                    }
+                }
+            }
+            if (W > 1) {
                 __syncthreads();
                 for (int i = threadIdx.x; i < 3 * nb; i += P2P_TB) {
                     const int d = i / nb, q = i - d * nb;
-                    float2 v = make_float2(0.f, 0.f);
+                    double v = 0.0;
 #pragma unroll
-                    for (int k = 0; k < P2P_WARPS; k++) comp_merge(v, reinterpret_cast<float2 *>(s_x[k])[64 * d + q]);
-                    (d == 0 ? out[0] : (d == 1 ? out[1] : out[2]))[q] += ((double)v.x - (double)v.y) * acc_scale;
+                    for (int k = 0; k < P2P_WARPS; k++) v += reinterpret_cast<double *>(s_x[k])[64 * d + q];
+                    (d == 0 ? A.ax : (d == 1 ? A.ay : A.az))[it + tb + q] += v * B.acc_scale;
                 }
                 __syncthreads();
             }
