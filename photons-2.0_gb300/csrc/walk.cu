@@ -220,6 +220,8 @@ __device__ __forceinline__ uint32_t get2(const uint32_t *s, int scap, const uint
     return pos < scap ? s[pos] : g[pos];
 }
 
+__device__ __forceinline__ void queue_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // The target at place t of the queue and its list (entries, offset in the
 // pool as 31 low bits and the rest), waited for until the warp that expands
 // its parent puts it there; id -1 if that takes more than two seconds.  The
@@ -235,7 +237,7 @@ __device__ __forceinline__ int4 queue_wait(const int4 *queue, long long t)
                      : "l"(queue + t)
                      : "memory");
         if ((v.x | v.y | v.z | v.w) >= 0) {  // every word is written once, none negative
-            __threadfence();
+            queue_fence();
             return v;
         }
         __nanosleep(20);
@@ -503,11 +505,12 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk(WalkArgs A)
             if (ok)
 #pragma unroll 4
                 for (int i = lane; i < n_pd; i += 32) W.pd_pool[off + i] = get2(sh_pd, WS_PD, st_pd, i);
-            // the list is complete: both children can be expanded
-            __threadfence();
+            // the list is complete: both children can be expanded (the barrier
+            // orders all lanes' stores before the fence of those that publish)
             __syncwarp();
             if (lane < 2) {
                 const long long o = ok ? off : 0;
+                queue_fence();
                 asm volatile("st.relaxed.gpu.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(W.queue + A.nbox + place + lane),
                              "r"(lane ? a1 : a0), "r"(ok ? n_pd : 0), "r"((int)(o & 0x7fffffff)), "r"((int)(o >> 31))
                              : "memory");
