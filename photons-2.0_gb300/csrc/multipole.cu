@@ -104,24 +104,10 @@ __global__ void k_p2m(const double *px, const double *py, const double *pz, cons
 }
 
 // ---------------- M2M (one depth, parents gather their two children) ----------------
-// d^e(i) / e(i)! as (first two factors) (third / e(i)!): the order of the
-// lanes' monomials below
-__device__ __forceinline__ void paired_monomials(double dx, double dy, double dz, double *out)
-{
-    const double x[4] = {dx, dy, dz, 1.0};
-#pragma unroll
-    for (int i = 0; i < PH_NMULTI; i++) {
-        const int e0 = h_mi.e[i][0], e1 = e0 + h_mi.e[i][1], e2 = e1 + h_mi.e[i][2];
-        const int f0 = e0 > 0 ? 0 : (e1 > 0 ? 1 : (e2 > 0 ? 2 : 3)), f1 = e0 > 1 ? 0 : (e1 > 1 ? 1 : (e2 > 1 ? 2 : 3)),
-                  f2 = e0 > 2 ? 0 : (e1 > 2 ? 1 : (e2 > 2 ? 2 : 3));
-        out[i] = __dmul_rn(__dmul_rn(x[f0], x[f1]), __dmul_rn(x[f2], h_mi.invf[i]));
-    }
-}
-
 __device__ __forceinline__ void m2m_add(double dx, double dy, double dz, const double *Mc, double *out)
 {
     double mono[PH_NMULTI];
-    paired_monomials(dx, dy, dz, mono);
+    scaled_monomials(dx, dy, dz, mono);
 #pragma unroll
     for (int a = 0; a < PH_NMULTI; a++) {
         double s = 0.0;
@@ -194,25 +180,30 @@ struct OpWarp {
 
 __device__ __forceinline__ int term(const unsigned *w, int n) { return (w[n >> 2] >> (8 * (n & 3))) & 255; }
 
-// lane i's scaled monomial d^e(i) / e(i)!: its exponents' running sums, 1 / e(i)!
+// lane i's scaled monomial d^e(i) / e(i)!: the axes of its factors (3: none)
+// in the order scaled_monomials multiplies them, and 1 / e(i)!
 struct LaneMono {
-    int e0, e1, e2;
+    int a, b, c;
     double invf;
 };
 
 __device__ __forceinline__ LaneMono lane_mono(int lane)
 {
     const int i = lane < PH_NMULTI ? lane : 0;
-    const int e0 = h_mi.e[i][0], e1 = e0 + h_mi.e[i][1];
-    return LaneMono{e0, e1, e1 + h_mi.e[i][2], h_mi.invf[i]};
+    const int e0 = h_mi.e[i][0], e1 = e0 + h_mi.e[i][1], e2 = e1 + h_mi.e[i][2];
+    const int a = e0 > 0 ? 0 : (e1 > 0 ? 1 : (e2 > 0 ? 2 : 3)), b = e0 > 1 ? 0 : (e1 > 1 ? 1 : (e2 > 1 ? 2 : 3)),
+              c = e0 > 2 ? 0 : (e1 > 2 ? 1 : (e2 > 2 ? 2 : 3));
+    // a square of the later axis comes first: x (y y)
+    if (c < 3 && a != b && b == c) return LaneMono{b, c, a, h_mi.invf[i]};
+    return LaneMono{a, b, c, h_mi.invf[i]};
 }
 
 __device__ __forceinline__ double lane_monomial(double dx, double dy, double dz, const LaneMono &q)
 {
-    const double f0 = q.e0 > 0 ? dx : (q.e1 > 0 ? dy : (q.e2 > 0 ? dz : 1.0)),
-                 f1 = q.e0 > 1 ? dx : (q.e1 > 1 ? dy : (q.e2 > 1 ? dz : 1.0)),
-                 f2 = q.e0 > 2 ? dx : (q.e1 > 2 ? dy : (q.e2 > 2 ? dz : 1.0));
-    return (f0 * f1) * (f2 * q.invf);
+    const double fa = q.a == 0 ? dx : (q.a == 1 ? dy : (q.a == 2 ? dz : 1.0)),
+                 fb = q.b == 0 ? dx : (q.b == 1 ? dy : (q.b == 2 ? dz : 1.0)),
+                 fc = q.c == 0 ? dx : (q.c == 1 ? dy : (q.c == 2 ? dz : 1.0));
+    return fa * fb * fc * q.invf;
 }
 
 // v_a = sum_{b <= a} M_b mono_(a-b): lane a's component of a multipole (lane
@@ -437,7 +428,7 @@ __global__ void k_l2l_depth(const int *list, const int *depth_off, int d, const 
         int p = parent[u];
         if (p < 0) continue;
         double mono[PH_NMULTI];
-        paired_monomials(cx[u] - cx[p], cy[u] - cy[p], cz[u] - cz[p], mono);
+        scaled_monomials(cx[u] - cx[p], cy[u] - cy[p], cz[u] - cz[p], mono);
         double Lp[PH_NMULTI];
 #pragma unroll
         for (int a = 0; a < PH_NMULTI; a++) Lp[a] = L[(size_t)p * PH_NMULTI + a];
