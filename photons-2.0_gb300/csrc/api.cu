@@ -468,6 +468,24 @@ static int stage_shortfall()
     return v && !strcmp(v, "1") ? 16 : 0;
 }
 
+// Test hook for the time limit of the walk's queue: with
+// PHOTONS_TEST_WALK_WITHHELD=k the target at the k-th place after the roots'
+// is never published, the warps that wait for it or for what lies below it
+// give up after two seconds, and the pass fails with an error.
+static int walk_withheld()
+{
+    const char *v = getenv("PHOTONS_TEST_WALK_WITHHELD");
+    return v && *v ? atoi(v) : -1;
+}
+
+// A walk whose wait ran out is repeated once (its clock runs on while
+// another program has the device), then reported
+static int walk_again(unsigned long long flags, int &waits)
+{
+    if (!(flags & PH_FLAG_WALK_WAIT) || waits++ == 0) return 0;
+    return ph_set_error(PH_ERR_STATE, "the walk did not finish in time");
+}
+
 // floats per reaction value: an FP64 pass keeps doubles in the float buffer
 static long long mu_per_value(int precision) { return precision == PHOTONS_FP64 ? 2 : 1; }
 
@@ -918,9 +936,11 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
     long long p2p_cap, pd_cap, m2l_cap;
     int stack_cap, stage_cap;
     walk_caps(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
+    int waits = 0;
     for (int attempt = 0; attempt < 6; attempt++) {
         PH_TRY(alloc_walk(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap));
-        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream, c->walk_imp));
+        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream, walk_withheld(),
+                              c->walk_imp));
         PH_CUDA_CHECK(cudaMemcpyAsync(c->ws.c, c->w.ctr, sizeof(c->ws.c), cudaMemcpyDeviceToHost, c->stream));
         PH_CUDA_CHECK(cudaStreamSynchronize(c->stream));
         unsigned long long fl = c->ws.c[ph::WC_FLAGS];
@@ -930,7 +950,7 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
             keep_walk_hints(c, p2p_cap, pd_cap, m2l_cap);  // a repeated pass allocates once
             return ph_record(c, EV_WALK);
         }
-        if (fl & PH_FLAG_WALK_WAIT) return ph_set_error(PH_ERR_STATE, "the walk did not finish in time");
+        PH_TRY(walk_again(fl, waits));
         grow_walk_caps(c, fl, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
     }
     return ph_set_error(PH_ERR_CAPACITY, "interaction lists did not fit after repeated growth");
@@ -1118,6 +1138,7 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
     k.stage_extra = stage_shortfall();
     k.far = capture_far(c, p);
     k.sub = c->b.sub;
+    k.withheld = walk_withheld();
     k.boxsize = p->boxsize; k.theta = p->theta; k.rs = p->rs; k.rcut = p->rcut; k.eps = p->eps; k.mass = p->mass;
     k.pos = dio ? (const void *)pos : nullptr;
     k.acc = dio ? (const void *)acc : nullptr;
@@ -1152,7 +1173,8 @@ static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double
                            unsigned mask)
 {
     PH_TRY(ph_enqueue_tree(c, src, levels));
-    PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream));
+    PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream,
+                          walk_withheld()));
     PH_TRY(ph_record(c, EV_WALK));
     PH_TRY(ph_stage_p2p(c, p->precision, 1));
     const bool far = capture_far(c, p);
@@ -1219,6 +1241,7 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
     walk_caps(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
     const double *src = dio ? pos : c->io;
     double *dst = dio ? acc : c->io;
+    int waits = 0;
     for (int attempt = 0; attempt < 16; attempt++) {
         PH_TRY(alloc_walk(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap));
         PH_TRY(alloc_mutual(c, p->precision));
@@ -1246,7 +1269,7 @@ static int force_pass_graph(photons_ctx *c, int nbox, const photons_params *p, c
         ph_tree_info_from(c, h, levels);
         c->have_tree = true;
         unsigned long long fl = c->ws.c[ph::WC_FLAGS];
-        if (fl & PH_FLAG_WALK_WAIT) return ph_set_error(PH_ERR_STATE, "the walk did not finish in time");
+        PH_TRY(walk_again(fl, waits));
         if (fl) {
             grow_walk_caps(c, fl, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap);
             continue;

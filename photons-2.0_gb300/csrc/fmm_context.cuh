@@ -163,10 +163,12 @@ struct WalkImports {
     int base = 0x7fffffff;      // unified id of the first received node
 };
 
-// image_mask: bit 0 the local tree, bit k the k-th periodic image;
-// ndepth = depths to launch (at least the tree's deepest + 1)
+// image_mask: bit 0 the local tree, bit k the k-th periodic image; nbox: the
+// boxes, whose roots are the queue's first places; withheld: a place after
+// them that is not published (-1, or a test's)
 int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
-               const PassParams &p, unsigned image_mask, cudaStream_t st, const WalkImports &imp = WalkImports());
+               const PassParams &p, unsigned image_mask, cudaStream_t st, int withheld,
+               const WalkImports &imp = WalkImports());
 
 // top: launched levels of wide nodes (<= levels); levels: depth bound
 int build_tree(BuildBufs &b, TreeBufs &t, const PassParams &p, int n, int levels, int top, cudaStream_t st);

@@ -141,6 +141,7 @@ struct WalkArgs {
     float prune_k2f;  // (0.95 theta)^2 in FP32: the image pruning rule's width test
     WalkImports imp;  // received trees (none outside a rank's domain pass)
     int maxleaf;
+    int withheld;     // a place after the roots' that is never published (-1; the test of the wait's limit)
 };
 
 // a source is a leaf: a local leaf, or a received node of <= MAXLEAF particles
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(WALK_TB, MINB) k_walk(WalkArgs A)
             // the list is complete: both children can be expanded (the barrier
             // orders all lanes' stores before the fence of those that publish)
             __syncwarp();
-            if (lane < 2) {
+            if (lane < 2 && place + lane != A.withheld) {
                 const long long o = ok ? off : 0;
                 queue_fence();
                 asm volatile("st.relaxed.gpu.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(W.queue + A.nbox + place + lane),
@@ -575,7 +576,7 @@ int launch_geom32(const TreeBufs &t, const int *tree_cnt, cudaStream_t st)
 
 // Enqueue the walk.  Counters and flags stay on the device (w.ctr).
 int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
-               const PassParams &p, unsigned image_mask, cudaStream_t st, const WalkImports &imp)
+               const PassParams &p, unsigned image_mask, cudaStream_t st, int withheld, const WalkImports &imp)
 {
     PH_CUDA_CHECK(cudaMemsetAsync(w.ctr, 0, sizeof(unsigned long long) * WC_N, st));
     PH_CUDA_CHECK(cudaMemsetAsync(w.queue, 0xff, sizeof(int4) * (size_t)w.queue_cap, st));
@@ -598,6 +599,7 @@ int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxPar
     A.theta2 = p.theta * p.theta;
     A.imp = imp;
     A.maxleaf = p.maxleaf;
+    A.withheld = withheld;
     const int blocks = (w.nwarps * 32 + WALK_TB - 1) / WALK_TB;
     if (w.nwarps == device_sm_count() * 3 * 8)
         ph::chain(k_walk<3>, blocks, WALK_TB, 0, st, A);

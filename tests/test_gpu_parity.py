@@ -234,6 +234,28 @@ def test_bulk_staging_wait_has_a_time_limit(ph, ics, monkeypatch):
     fp.close()
 
 
+@pytest.mark.parametrize("graph", ["1", "0"])
+def test_walk_wait_has_a_time_limit(ph, ics, monkeypatch, graph):
+    """A target that is never published (the test hook withholds one place of
+    the walk's queue): the warps that wait give up after their two-second
+    limit, the pass is repeated once and then fails with an error, and the
+    context runs the same pass correctly afterwards."""
+    import time
+
+    monkeypatch.setenv("PHOTONS_GRAPH", graph)
+    pos, p = ics.make("grid32", nside=12, maxleaf=16)
+    fp = ph.ForcePass(0)
+    good = fp.run(pos, p, precision=ph.FP64)
+    monkeypatch.setenv("PHOTONS_TEST_WALK_WITHHELD", "5")
+    t0 = time.time()
+    with pytest.raises(ph.PhotonsError, match="did not finish in time"):
+        fp.run(pos, p, precision=ph.FP64)
+    assert 3.5 < time.time() - t0 < 60
+    monkeypatch.delenv("PHOTONS_TEST_WALK_WITHHELD")
+    assert np.array_equal(fp.run(pos, p, precision=ph.FP64), good)
+    fp.close()
+
+
 def test_mutual_pairs_graph_and_stage_paths_agree(ph, ics, monkeypatch):
     """The mutual kernel inside the captured graph and launched stage by
     stage (where the reaction buffer is sized between the stages) agree
