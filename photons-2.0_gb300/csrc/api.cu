@@ -687,6 +687,7 @@ static BoxParams box_params(const photons_params *p, int first, int count)
     const double ia = 0.5 / p->rs;
     B.far_a = (float)ia;
     B.far_pa = (float)(SPLIT_P * ia);
+    B.pair64 = pair64_box(p->eps, p->rs, p->mass);
     B.first = first;
     B.count = count;
     B.root = -1;

@@ -70,7 +70,7 @@ __device__ __forceinline__ double direct_factor(double dx, double dy, double dz,
     const long long rb = __double_as_longlong(r2);
     const bool near = on && (rb < rmax2_bits || rb > 0x7ff0000000000000LL);
     double f = ph::pair64_f(dx, dy, dz, near, pc, tab);
-    if (near && rb == 0 && pc.eps == 0.0) f = INFINITY;  // coincident and unsoftened: m / r^3
+    if (near && rb == 0 && pc.box->eps == 0.0) f = INFINITY;  // coincident and unsoftened: m / r^3
     return f;
 }
 
@@ -79,8 +79,8 @@ __global__ void __launch_bounds__(DIRECT_TB) k_direct(const double *__restrict__
                                                       const int *__restrict__ cell_start, int ncell, double cellw,
                                                       const double *__restrict__ tx, const double *__restrict__ ty,
                                                       const double *__restrict__ tz, const int *__restrict__ tself,
-                                                      int nt, double L, double most, double rmax2, double eps,
-                                                      double mass, double rs, double *out)
+                                                      int nt, double L, double most, double rmax2,
+                                                      const __grid_constant__ Pair64Box box, double *out)
 {
     __shared__ int s_queue[DIRECT_WARPS][64];
     __shared__ double s_sum[DIRECT_WARPS][3];
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(DIRECT_TB) k_direct(const double *__restrict__
     const unsigned lt = (1u << lane) - 1u;
     int *queue = s_queue[warp];
     const ph::Pair64Tab tab = ph::pair64_global();
-    const ph::Pair64 pc = ph::pair64_consts(eps, rs);
+    const ph::Pair64 pc = ph::pair64_consts(box);
     const long long half_bits = __double_as_longlong(0.5 * L), rmax2_bits = __double_as_longlong(rmax2);
     const float Lf = (float)L, halff = 0.5f * Lf;
     const float limit = direct_limit(rmax2, most);
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(DIRECT_TB) k_direct(const double *__restrict__
         if (threadIdx.x < 3) {
             double v = 0.0;
             for (int w = 0; w < DIRECT_WARPS; w++) v += s_sum[w][threadIdx.x];
-            out[3 * (size_t)t + threadIdx.x] = v * ph::pair64_scale(mass, rs);
+            out[3 * (size_t)t + threadIdx.x] = v * box.scale;
         }
         __syncthreads();
     }
@@ -188,8 +188,9 @@ __global__ void k_direct_sources(const double *__restrict__ pos, int n, double L
 __global__ void __launch_bounds__(DIRECT_TB, 3) k_direct_all(const double4 *__restrict__ s8,
                                                              const float4 *__restrict__ s4, int n,
                                                              const int *__restrict__ targets, int nt, int slice,
-                                                             int nslice, double L, double rmax2, double eps, double rs,
-                                                             int *work, const int *outside, double *part)
+                                                             int nslice, double L, double rmax2,
+                                                             const __grid_constant__ Pair64Box box, int *work,
+                                                             const int *outside, double *part)
 {
     extern __shared__ __align__(16) unsigned char direct_smem[];
     __shared__ int s_queue[DIRECT_WARPS][DIRECT_TG][64];
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(DIRECT_TB, 3) k_direct_all(const double4 *__re
     const ph::Pair64Tab tab = ph::pair64_load(direct_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const ph::Pair64 pc = ph::pair64_consts(eps, rs);
+    const ph::Pair64 pc = ph::pair64_consts(box);
     const long long half_bits = __double_as_longlong(0.5 * L), rmax2_bits = __double_as_longlong(rmax2);
     const float Lf = (float)L, halff = 0.5f * Lf, limit = direct_limit(rmax2, L);
     const int groups = (nt + DIRECT_TG - 1) / DIRECT_TG, items = groups * nslice;
@@ -374,15 +375,15 @@ static int direct_all(const photons_params *p, int n, const double *pos, int nt,
     double *dpos = reinterpret_cast<double *>(d + b8 + b4), *part = reinterpret_cast<double *>(d + b8 + b4 + bp),
            *out = reinterpret_cast<double *>(d + b8 + b4 + bp + bs);
     int *tgt = reinterpret_cast<int *>(d + b8 + b4 + bp + bs + bo), *ctl = reinterpret_cast<int *>(d + b8 + b4 + bp + bs + bo + bt);
+    const Pair64Box box = pair64_box(p->eps, p->rs, p->mass);
     int outside = 0;
     cudaMemsetAsync(ctl, 0, 2 * sizeof(int));
     cudaMemcpyAsync(tgt, targets, sizeof(int) * (size_t)nt, cudaMemcpyHostToDevice);
     cudaMemcpyAsync(dpos, pos, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice);
     ph::note_launch(), k_direct_sources<<<ph::device_sm_count() * 8, 256>>>(dpos, n, p->boxsize, s8, s4, ctl + 1);
     ph::note_launch(), k_direct_all<<<blocks, DIRECT_TB, PAIR64_BYTES>>>(s8, s4, n, tgt, nt, slice, nslice, p->boxsize,
-                                                                        rmax * rmax, p->eps, p->rs, ctl, ctl + 1, part);
-    const double ia = 0.5 / p->rs;
-    ph::note_launch(), k_direct_reduce<<<(3 * nt + 255) / 256, 256>>>(part, nt, nslice, p->mass * (ia * ia * ia), out);
+                                                                        rmax * rmax, box, ctl, ctl + 1, part);
+    ph::note_launch(), k_direct_reduce<<<(3 * nt + 255) / 256, 256>>>(part, nt, nslice, box.scale, out);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&outside, ctl + 1, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(acc, out, sizeof(double) * 3 * (size_t)nt, cudaMemcpyDeviceToHost);
@@ -476,7 +477,7 @@ extern "C" int photons_direct_sum(const photons_params *p, int n, const double *
         const int blocks = ph::device_sm_count() * 8;
         ph::note_launch(), k_direct_f32<<<blocks, 256>>>(d_sx, d_sy, d_sz, n, d_s4);
         ph::note_launch(), k_direct<<<nt, DIRECT_TB>>>(d_sx, d_sy, d_sz, d_s4, d_cell, ncell, cw, d_tx, d_ty, d_tz, d_ts, nt, L, most, rmax * rmax,
-                                  p->eps, p->mass, p->rs, d_out);
+                                  pair64_box(p->eps, p->rs, p->mass), d_out);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpy(acc, d_out, sizeof(double) * 3 * nt, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = ph_set_cuda_error(e, "direct sum", __FILE__, __LINE__);

@@ -55,6 +55,37 @@ struct PassParams {
 // One periodic box of a pass.  A pass covers one box or many independent
 // boxes (their particles concatenated, one tree root each); every kernel
 // reads the constants of the box its target belongs to from this table.
+// The FP64 pair factor's constants for a softening, split scale and mass
+// (pair64.cuh): forces are scale f dx, f = g(r / 2rs) / (r / unit)^3, with
+// scale = mass / unit^3 and unit = 2rs.  q = (r / unit)^2 = r^2 k 2^(ke - 63);
+// the tables serve high words of q above qeps (that of (eps / unit)^2).
+// A split scale so large or small that its powers leave the range of doubles
+// (no split at all, say) has unit = 1 and no use of the tables.
+struct Pair64Box {
+    unsigned long long k;
+    int ke, qeps;
+    double eps, ieps3, hrs, cube, scale;  // eps, 1 / eps^3, 1 / 2rs, unit^3
+};
+
+__host__ __device__ inline Pair64Box pair64_box(double eps, double rs, double mass)
+{
+    Pair64Box b;
+    const bool tables = rs > 0x1p-200 && rs < 0x1p200;
+    const double ia = tables ? 0.5 / rs : 1.0, ia2 = ia * ia, qe = eps * eps * ia2;
+    unsigned long long u, v;
+    memcpy(&u, &ia2, sizeof u);
+    memcpy(&v, &qe, sizeof v);
+    b.k = (1ull << 63) | (u << 11);
+    b.ke = (int)(u >> 52) - 1023;
+    b.qeps = tables ? (int)(v >> 32) : 0x7fffffff;
+    b.eps = eps;
+    b.ieps3 = 1.0 / (eps * eps * eps);
+    b.hrs = 0.5 / rs;
+    b.cube = tables ? 8.0 * rs * rs * rs : 1.0;
+    b.scale = mass * (ia * ia * ia);
+    return b;
+}
+
 struct BoxParams {
     double boxsize, rs, rcut, eps, mass;
     double rcut2;       // rcut^2
@@ -67,6 +98,7 @@ struct BoxParams {
     int root;           // unified id of the box's root node (written by the build)
     int domain;         // 1: the root's box is dom_lo..dom_hi (a rank's domain), else [0, boxsize]^3
     double dom_lo[3], dom_hi[3];
+    Pair64Box pair64;   // FP64 pair force
 };
 
 // ------------------------------------------------------------------

@@ -679,8 +679,8 @@ __global__ void __launch_bounds__(P2P_TB) k_p2p_fp64(P2PArgs A)
         const int nt = A.npart[t], it = A.ipart[t];
         if (nt == 0) continue;
         const BoxParams &B = A.boxes[A.boxid[t]];
-        const double boxL = B.boxsize, scale = pair64_scale(B.mass, B.rs);
-        const Pair64 pc = pair64_consts(B.eps, B.rs);
+        const double boxL = B.boxsize, scale = B.pair64.scale;
+        const Pair64 pc = pair64_consts(B.pair64);
         const long long eoff = A.p2p_off[t];
         const int ecnt = A.p2p_cnt[t];
         for (int r0 = 0; r0 < nt; r0 += 32) {
@@ -1616,8 +1616,8 @@ __device__ __forceinline__ void mu64_chunk(const P2PArgs &A, const int2 *ev, int
     constexpr int SG = 32 / TG, T = 8;
     const int tg = lane / SG, sg = lane % SG;
     const BoxParams &B = A.boxes[A.boxid[t]];
-    const double boxL = B.boxsize, scale = pair64_scale(B.mass, B.rs);
-    const Pair64 pc = pair64_consts(B.eps, B.rs);
+    const double boxL = B.boxsize, scale = B.pair64.scale;
+    const Pair64 pc = pair64_consts(B.pair64);
     __syncwarp();
     for (int q = lane; q < TG * T; q += 32) {
         // slots past the last target repeat it; their pairs are switched off
@@ -1851,8 +1851,9 @@ __global__ void k_leaf_pair_fp64(const double *tpos, int nt, int tfirst, const d
     const double px = tpos[3 * q], py = tpos[3 * q + 1], pz = tpos[3 * q + 2];
     const double coeff = 2.0 / sqrt(M_PI), soft3 = mass / (eps * eps * eps);
     const Pair64Tab tab = pair64_global();
-    const Pair64 pc = pair64_consts(eps, rs);
-    const double scale = pair64_scale(mass, rs);
+    const Pair64Box box = pair64_box(eps, rs, mass);
+    const Pair64 pc = pair64_consts(box);
+    const double scale = box.scale;
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int j = 0; j < ns; j++) {
         if (sfirst + j == tfirst + q) continue;

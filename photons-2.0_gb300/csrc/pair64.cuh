@@ -120,43 +120,29 @@ __device__ __forceinline__ double pair64_poly(unsigned i, long long d, const Pai
 }
 
 // f where the tables do not reach (r < eps, q outside their range): 1/r
-// from rsqrt and g from its own polynomials; two coincident particles get
-// the softened factor.  Rare: not inlined.
-__device__ __noinline__ double pair64_slow(double dx, double dy, double dz, double eps, double rs)
+// from rsqrt and g from its own polynomials, ~30 FP64 instructions; two
+// coincident particles get the softened factor.  Not inlined; its constants
+// are read from memory, so that they take no registers of the callers, and
+// ahead of their use (volatile: read where they are needed, behind a branch,
+// they cost a halo's one-way lists 8 %).
+__device__ __noinline__ double pair64_slow(double dx, double dy, double dz, const volatile Pair64Box *b)
 {
-    const double hrs = 0.5 / rs, cube = 8.0 * rs * rs * rs;
+    const double eps = b->eps, ieps3 = b->ieps3, hrs = b->hrs, cube = b->cube;
     const double r2 = dx * dx + dy * dy + dz * dz;
     const double rinv = r2 > 0.0 ? rsqrt(r2) : 0.0;
     const double dr = r2 * rinv;
-    const double w = dr < eps ? 1.0 / (eps * eps * eps) : rinv * rinv * rinv;
-    return w * split_g_fp64(dr * hrs, &g_split64[0][0], 2.0 / sqrt(M_PI)) * cube;
+    const double w = dr < eps ? ieps3 : rinv * rinv * rinv;
+    return w * split_g_fp64(dr * hrs, &g_split64[0][0], 1.1283791670955126) * cube;
 }
 
-// Per-box constants: q = r^2 ia2 with ia2 = k 2^(ke - 63), k in [2^63, 2^64);
-// the tables serve high words of q above qeps (that of eps^2 ia2)
+// what a pair needs of the constants in registers
 struct Pair64 {
     unsigned long long k;
     int ke, qeps;
-    double eps, rs;
+    const Pair64Box *box;
 };
 
-__device__ __forceinline__ Pair64 pair64_consts(double eps, double rs)
-{
-    Pair64 c;
-    const double ia = 0.5 / rs, ia2 = ia * ia;
-    c.k = (1ull << 63) | ((unsigned long long)__double_as_longlong(ia2) << 11);
-    c.ke = (__double2hiint(ia2) >> 20) - 1023;
-    c.qeps = __double2hiint(eps * eps * ia2);
-    c.eps = eps;
-    c.rs = rs;
-    return c;
-}
-
-__device__ __forceinline__ double pair64_scale(double mass, double rs)
-{
-    const double ia = 0.5 / rs;
-    return mass * (ia * ia * ia);
-}
+__device__ __forceinline__ Pair64 pair64_consts(const Pair64Box &b) { return Pair64{b.k, b.ke, b.qeps, &b}; }
 
 // f for a source dx away; 0 where !on.  q = r^2 ia2 in fixed point too (the
 // squares of the components aligned to the largest, good to 2^-58), which
@@ -179,7 +165,7 @@ __device__ __forceinline__ double pair64_f(double dx, double dy, double dz, bool
     const unsigned i = ((unsigned)(eq - PAIR64_LO) << PAIR64_MB) + ((unsigned)(s >> (63 - PAIR64_MB)) & ((1u << PAIR64_MB) - 1u));
     const bool fast = i < PAIR64_NI && qhi > c.qeps;
     double f = pair64_poly(fast ? i : 0u, (long long)((s << (PAIR64_MB + 1)) ^ (1ull << 63)), tab);
-    if (on && !fast) f = pair64_slow(dx, dy, dz, c.eps, c.rs);
+    if (on && !fast) f = pair64_slow(dx, dy, dz, c.box);
     return on ? f : 0.0;
 }
 

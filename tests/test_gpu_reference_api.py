@@ -216,6 +216,39 @@ def test_direct_sum_filter_keeps_every_source(ph, n, rmax, eps, reach):
         assert np.abs(got[k] - want).max() <= 1e-13 * scale, (n, t)
 
 
+@pytest.mark.parametrize("rs", [1e-160, 1e-3, 0.7, 1e3, 1e50, 1e100, 1e160, np.inf])
+def test_fp64_forces_at_extreme_split_scales(ph, rs):
+    """From no long-range part at all (rs far above the box: Newtonian forces)
+    to nothing but it (rs far below the spacing: none): the FP64 pass, mutual
+    and one way, and the direct sum against numpy.  Tolerance: as above."""
+    from scipy.special import erfc
+    L, m, eps, n = 10.0, 2.5, 0.05, 400
+    pos = np.random.default_rng(1).uniform(0.0, L, (n, 3))
+    targets = np.arange(0, n, 10, dtype=np.int32)
+    # theta 0, a cutoff beyond the images: all 27 images of every pair
+    p = dict(boxsize=L, theta=0.0, rs=rs, rcut=4.0 * L, eps=eps, mass=m, maxleaf=8)
+
+    def check(got, near):
+        for k, t in enumerate(targets):
+            want, scale = np.zeros(3), 1e-300
+            d = pos - pos[t]
+            shifts = [(0, 0, 0)] if near else [(i, j, k) for i in (-1, 0, 1) for j in (-1, 0, 1) for k in (-1, 0, 1)]
+            for sh in shifts:
+                e = d - L * np.round(d / L) if near else d + L * np.array(sh)
+                r = np.sqrt((e ** 2).sum(1))
+                on = r > 0
+                u = 0.5 * r[on] / rs
+                f = m * (erfc(u) + 2.0 / np.sqrt(np.pi) * u * np.exp(-np.minimum(u, 1e3) ** 2)) / np.maximum(r[on], eps) ** 3
+                want += (f[:, None] * e[on]).sum(0)
+                scale += (f * r[on]).sum()
+            assert np.abs(got[k] - want).max() <= 1e-13 * scale
+
+    with contextlib.closing(ph.ForcePass(0)) as fp:
+        for flags in (0, ph.F_ONE_WAY):
+            check(fp.run(pos, p, precision=ph.FP64, flags=flags)[targets], False)
+    check(ph.direct_sum(pos, p, targets, 2.0 * L), True)
+
+
 @pytest.mark.parametrize("ntarget", [1, 9, 4096, 4097])
 def test_direct_sum_slices_and_bins_match_oracle(ph, port, ics, ntarget):
     """The direct sum with the sources in several slices (few targets) and
