@@ -940,8 +940,8 @@ int ph_stage_walk(photons_ctx *c, unsigned mask)
     int waits = 0;
     for (int attempt = 0; attempt < 6; attempt++) {
         PH_TRY(alloc_walk(c, p2p_cap, pd_cap, m2l_cap, stack_cap, stage_cap));
-        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream, walk_withheld(),
-                              c->walk_imp));
+        PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream, 2 * c->b.rule_cap,
+                              walk_withheld(), c->walk_imp));
         PH_CUDA_CHECK(cudaMemcpyAsync(c->ws.c, c->w.ctr, sizeof(c->ws.c), cudaMemcpyDeviceToHost, c->stream));
         PH_CUDA_CHECK(cudaStreamSynchronize(c->stream));
         unsigned long long fl = c->ws.c[ph::WC_FLAGS];
@@ -1140,6 +1140,7 @@ static PassKey pass_key(photons_ctx *c, const photons_params *p, int n, const do
     k.far = capture_far(c, p);
     k.sub = c->b.sub;
     k.withheld = walk_withheld();
+    k.rule_cap = c->b.rule_cap;
     k.boxsize = p->boxsize; k.theta = p->theta; k.rs = p->rs; k.rcut = p->rcut; k.eps = p->eps; k.mass = p->mass;
     k.pos = dio ? (const void *)pos : nullptr;
     k.acc = dio ? (const void *)acc : nullptr;
@@ -1175,7 +1176,7 @@ static int ph_enqueue_pass(photons_ctx *c, const photons_params *p, const double
 {
     PH_TRY(ph_enqueue_tree(c, src, levels));
     PH_TRY(ph::walk_lists(c->w, c->t, c->b.cnt, c->b.boxes, c->b.nbox, c->pp, mask, c->stream,
-                          walk_withheld()));
+                          2 * c->b.rule_cap, walk_withheld()));
     PH_TRY(ph_record(c, EV_WALK));
     PH_TRY(ph_stage_p2p(c, p->precision, 1));
     const bool far = capture_far(c, p);

@@ -164,10 +164,11 @@ struct WalkImports {
 };
 
 // image_mask: bit 0 the local tree, bit k the k-th periodic image; nbox: the
-// boxes, whose roots are the queue's first places; withheld: a place after
-// them that is not published (-1, or a test's)
+// boxes, whose roots are the queue's first places; targets: the most leaves
+// and nodes this pass can have; withheld: a place after the roots' that is
+// not published (-1, or a test's)
 int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
-               const PassParams &p, unsigned image_mask, cudaStream_t st, int withheld,
+               const PassParams &p, unsigned image_mask, cudaStream_t st, int targets, int withheld,
                const WalkImports &imp = WalkImports());
 
 // top: launched levels of wide nodes (<= levels); levels: depth bound

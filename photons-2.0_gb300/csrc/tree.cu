@@ -1395,8 +1395,9 @@ int build_tree(BuildBufs &b, TreeBufs &T, const PassParams &p, int n, int levels
         return ph_set_error(7, "tree deeper than %d levels", T.max_depth_cap - 1);
     if (top < 0 || top > levels) top = levels;
     const int ndepth = levels + 1;  // leaves can sit one level below the deepest nodes
-    const int nblk = T.depth_nblk;
-    if (nblk < 1 || nblk != depth_sort_blocks(T.cap_u)) return ph_set_error(7, "depth-sort buffers not allocated");
+    // blocks for as many nodes and leaves as this pass can have
+    const int nblk = depth_sort_blocks(2 * b.rule_cap);
+    if (nblk < 1 || nblk > T.depth_nblk) return ph_set_error(7, "depth-sort buffers not allocated");
     // shared memory above the 48 KB default, allowed once per device
     static std::atomic<bool> done[64];
     int dev = 0;

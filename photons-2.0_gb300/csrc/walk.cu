@@ -34,6 +34,7 @@
 //
 // Acceptance is evaluated in FP64 with explicit round-to-nearest operations
 // (no contraction) so that every decision equals the reference's.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -576,10 +577,11 @@ int launch_geom32(const TreeBufs &t, const int *tree_cnt, cudaStream_t st)
 
 // Enqueue the walk.  Counters and flags stay on the device (w.ctr).
 int walk_lists(WalkBufs &w, const TreeBufs &t, const int *tree_cnt, const BoxParams *boxes, int nbox,
-               const PassParams &p, unsigned image_mask, cudaStream_t st, int withheld, const WalkImports &imp)
+               const PassParams &p, unsigned image_mask, cudaStream_t st, int targets, int withheld,
+               const WalkImports &imp)
 {
     PH_CUDA_CHECK(cudaMemsetAsync(w.ctr, 0, sizeof(unsigned long long) * WC_N, st));
-    PH_CUDA_CHECK(cudaMemsetAsync(w.queue, 0xff, sizeof(int4) * (size_t)w.queue_cap, st));
+    PH_CUDA_CHECK(cudaMemsetAsync(w.queue, 0xff, sizeof(int4) * (size_t)std::min(w.queue_cap, targets), st));
     WalkArgs A{};
     A.g.cx = t.cx; A.g.cy = t.cy; A.g.cz = t.cz;
     A.g.wx = t.wx; A.g.wy = t.wy; A.g.wz = t.wz; A.g.wsum = t.wsum;

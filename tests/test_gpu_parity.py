@@ -235,6 +235,26 @@ def test_bulk_staging_wait_has_a_time_limit(ph, ics, monkeypatch):
 
 
 @pytest.mark.parametrize("graph", ["1", "0"])
+def test_small_passes_in_a_context_that_served_a_large_one(ph, ics, monkeypatch, graph):
+    """The launches and clears of a pass are sized by the pass, not by what
+    the context once held: the same forces and lists as on a fresh context."""
+    monkeypatch.setenv("PHOTONS_GRAPH", graph)
+    used = ph.ForcePass(0)
+    pos, p = ics.make("grid32", nside=48, maxleaf=1)
+    used.run(pos, p, precision=ph.FP64)
+    for workload, nside, maxleaf in (("grid32", 16, 16), ("nfw128", 24, 8), ("grid32", 8, 64), ("nfw128", 32, 24)):
+        pos, p = ics.make(workload, nside=nside, maxleaf=maxleaf)
+        fresh = ph.ForcePass(0)
+        for prec in (ph.FP64, ph.FP32_SPLIT):
+            assert np.array_equal(used.run(pos, p, precision=prec), fresh.run(pos, p, precision=prec))
+            a, b = used.counters(), fresh.counters()
+            for k in COUNTERS + ["depth"]:
+                assert a[k] == b[k], k
+        fresh.close()
+    used.close()
+
+
+@pytest.mark.parametrize("graph", ["1", "0"])
 def test_walk_wait_has_a_time_limit(ph, ics, monkeypatch, graph):
     """A target that is never published (the test hook withholds one place of
     the walk's queue): the warps that wait give up after their two-second
