@@ -216,6 +216,16 @@ def test_direct_sum_filter_keeps_every_source(ph, n, rmax, eps, reach):
         assert np.abs(got[k] - want).max() <= 1e-13 * scale, (n, t)
 
 
+def test_direct_sum_without_room_for_all_sources(ph, port, ics, monkeypatch):
+    """With the buffer of the unbinned sum refused (the test hook), the call
+    takes the binned sum: the bar of the direct sum above."""
+    pos, p = ics.make("nfw128", nside=24)
+    targets = np.random.default_rng(5).choice(pos.shape[0], 300, replace=False).astype(np.int32)
+    monkeypatch.setenv("PHOTONS_TEST_DIRECT_NO_ROOM", "1")
+    got = ph.direct_sum(pos, p, targets)
+    assert rel_err(got, port.direct_sum(pos, p, targets, nthreads=8), p).max() <= 1e-10
+
+
 @pytest.mark.parametrize("rs", [1e-160, 1e-3, 0.7, 1e3, 1e50, 1e100, 1e160, np.inf])
 def test_fp64_forces_at_extreme_split_scales(ph, rs):
     """From no long-range part at all (rs far above the box: Newtonian forces)
