@@ -919,6 +919,11 @@ static void walk_caps(photons_ctx *c, long long &p2p_cap, long long &pd_cap, lon
     // push-down entries: up to 51 16 / leaf a particle in halos (leaf 16), 4.7 16 / leaf
     // in a 256^3 Zel'dovich box (leaf 64); cut short, they also hide the P2P need
     pd_cap = c->hint_pd ? c->hint_pd : n * (per < 48 ? 64 : 32) * 16 / per + 4096;
+    // (the larger guess only where it is a small part of the free memory)
+    size_t free_b = 0, total_b = 0;
+    if (!c->hint_pd && per < 48 && pd_cap > (1 << 28) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+        (size_t)pd_cap * sizeof(uint32_t) > free_b / 8)
+        pd_cap /= 2;
     m2l_cap = c->hint_m2l ? c->hint_m2l : n * 2 + 4096;
     stack_cap = c->w.stack_cap ? c->w.stack_cap : 4096;
     stage_cap = c->w.stage_cap ? c->w.stage_cap : 16384;
