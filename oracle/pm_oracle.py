@@ -44,18 +44,19 @@ def _cic(pos, N, L):
             ((i, jj, kk), (win, wj, wk)), ((ii, jj, kk), (wi, wj, wk))]
 
 
-def green(N, L, rs):
+def green(N, L, rs, real=np.float64):
     """G on the half spectrum [N, N, N//2+1] (src/conv.f90:171-227)."""
+    pi = real(PM_PI)
     nhalf = N // 2
-    ismth2 = 2 * PM_PI * rs / L
+    ismth2 = 2 * pi * rs / L
     ismth2 = ismth2 * ismth2
-    pref = L * L / (PM_PI * N * N * N)
+    pref = L * L / (pi * N * N * N)
     a = np.arange(N)
     a = np.where(a > nhalf, a - N, a)
     c = np.arange(N // 2 + 1)
 
     def sinc(q):
-        f = PM_PI * q.astype(np.float64) / N
+        f = pi * q.astype(real) / N
         with np.errstate(invalid="ignore", divide="ignore"):
             s = np.sin(f) / f
         return np.where(q == 0, 1.0, s)
@@ -63,7 +64,7 @@ def green(N, L, rs):
     fx = sinc(a)[:, None, None]
     fy = sinc(a)[None, :, None]
     fz = sinc(c)[None, None, :]
-    k2 = (a[:, None, None] ** 2 + a[None, :, None] ** 2 + c[None, None, :] ** 2).astype(np.float64)
+    k2 = (a[:, None, None] ** 2 + a[None, :, None] ** 2 + c[None, None, :] ** 2).astype(real)
     ff = 1.0 / (fx * fy * fz)
     with np.errstate(invalid="ignore", divide="ignore"):
         gf = pref * np.exp(-k2 * ismth2) * ff * ff * ff * ff / k2
@@ -71,21 +72,23 @@ def green(N, L, rs):
     return gf
 
 
-def pm_force(pos, boxsize, nside, rs, mass):
-    """acc_pm (n, 3) of the reference's PM at one rank (G-free)."""
-    pos = np.ascontiguousarray(pos, np.float64).reshape(-1, 3)
-    N, L = int(nside), float(boxsize)
+def pm_force(pos, boxsize, nside, rs, mass, real=np.float64):
+    """acc_pm (n, 3) of the reference's PM at one rank (G-free); real:
+    np.longdouble for the same in extended precision."""
+    pos = np.ascontiguousarray(pos, real).reshape(-1, 3)
+    N, L = int(nside), real(boxsize)
+    rs, mass = real(rs), real(mass)
     corners = _cic(pos, N, L)
-    rho = np.zeros((N, N, N))
+    rho = np.zeros((N, N, N), real)
     for (ci, cj, ck), (a, b, c) in corners:
         np.add.at(rho, (ci, cj, ck), mass * a * b * c)
     renormal = N / L
     renormal = renormal * renormal * renormal
     rho *= renormal
-    rk = np.fft.rfftn(rho) * green(N, L, rs)
+    rk = np.fft.rfftn(rho) * green(N, L, rs, real)
     psi = np.fft.irfftn(rk, s=(N, N, N), axes=(0, 1, 2)) * (N * N * N)  # the unnormalised inverse
     invx = 0.5 * N / L
-    c1, c2 = (4.0 / 3.0) * invx, (1.0 / 6.0) * invx
+    c1, c2 = real(4) / 3 * invx, real(1) / 6 * invx
     grads = []
     for ax in range(3):
         g = c1 * (np.roll(psi, -1, ax) - np.roll(psi, 1, ax))

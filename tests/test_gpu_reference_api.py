@@ -309,6 +309,22 @@ def test_pm_of_positions_below_the_box_matches_oracle(ph, nside, L):
     assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("workload,n,nside", [("grid32", 24, 32), ("nfw128", 28, 40), ("zeldovich256", 24, 24)])
+def test_pm_is_as_accurate_as_an_fp64_evaluation(ph, ics, workload, n, nside):
+    """The 64-bit integer PM and the FP64 oracle, both against extended
+    precision: at most twice the oracle's rms error (their transforms round
+    differently; the terms the integers replace are a small part of it)."""
+    import pm_oracle
+    pos, p = ics.make(workload, nside=n)
+    args = (pos, p["boxsize"], nside, p["rs"], p["mass"])
+    want = pm_oracle.pm_force(*args, real=np.longdouble)
+    assert want.dtype == np.longdouble
+    with contextlib.closing(ph.ForcePass(0)) as fp:
+        got = fp.pm_force(pos, p, nside)
+    rms = lambda x: float(np.sqrt(((x - want) ** 2).mean()))  # noqa: E731
+    assert rms(got) <= 2.0 * rms(pm_oracle.pm_force(*args)), (rms(got), rms(pm_oracle.pm_force(*args)))
+
+
 def test_pm_of_a_position_that_is_not_finite_is_nan(ph):
     pos = np.random.default_rng(0).uniform(0.0, 8.0, (50, 3))
     pos[7, 1] = np.nan
