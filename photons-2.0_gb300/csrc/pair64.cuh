@@ -27,13 +27,14 @@ namespace {
 // ---------------------------------------------------------------------
 // g(u) = erfc(u) + (2/sqrt(pi)) u exp(-u^2) (src/fmm.c:846-848) in FP64:
 // piecewise polynomials of degree 8 on intervals of 1/16 (coefficients by
-// fit_split_fp64.py, within 5.3e-17 of g on [0, 8)), erfc and exp beyond.
+// fit_split_fp64.py, within 5.3e-17 of g on [0, 8)), erfc and exp elsewhere
+// (below 0 too: a negative split scale is not refused everywhere).
 // tab: the coefficients k-major, [k][interval].
 __device__ const double g_split64[SPLIT64_DEG + 1][SPLIT64_NI] = SPLIT64_C_INIT;
 
 __device__ __forceinline__ double split_g_fp64(double u, const double *tab, double coeff)
 {
-    if (u < SPLIT64_NI * SPLIT64_W) {
+    if (__double2hiint(u) >= 0 && u < SPLIT64_NI * SPLIT64_W) {
         const int i = (int)(u * SPLIT64_INVW);
         const double d = u - ((double)i + 0.5) * SPLIT64_W;
         double acc = tab[SPLIT64_DEG * SPLIT64_NI + i];

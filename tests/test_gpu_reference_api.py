@@ -226,6 +226,28 @@ def test_direct_sum_without_room_for_all_sources(ph, port, ics, monkeypatch):
     assert rel_err(got, port.direct_sum(pos, p, targets, nthreads=8), p).max() <= 1e-10
 
 
+@pytest.mark.parametrize("rs", [-0.7, -1e3, -1e-3])
+def test_direct_sum_of_a_negative_split_scale(ph, rs):
+    """The direct sum does not refuse rs < 0: the reference's expressions at
+    u < 0, binned and not.  Tolerance: 1e-13 of the sum of the magnitudes."""
+    from scipy.special import erfc
+    L, m, eps, n = 10.0, 2.5, 0.05, 300
+    rng = np.random.default_rng(2)
+    p = dict(boxsize=L, theta=0.5, rs=rs, rcut=3.0, eps=eps, mass=m, maxleaf=16)
+    for pos in (rng.uniform(0.0, L, (n, 3)), rng.uniform(-1.0, L, (n, 3))):
+        targets = np.arange(0, n, 10, dtype=np.int32)
+        got = ph.direct_sum(pos, p, targets, 2.0 * L)
+        for k, t in enumerate(targets):
+            d = pos - pos[t]
+            d = np.where(d > 0.5 * L, d - L, np.where(d < -0.5 * L, d + L, d))
+            r = np.sqrt((d ** 2).sum(1))
+            on = np.arange(n) != t
+            u = 0.5 * r[on] / rs
+            with np.errstate(over="ignore"):
+                f = m * (erfc(u) + 2.0 / np.sqrt(np.pi) * u * np.exp(-u * u)) / np.maximum(r[on], eps) ** 3
+            assert np.abs(got[k] - (f[:, None] * d[on]).sum(0)).max() <= 1e-13 * (np.abs(f) * r[on]).sum()
+
+
 @pytest.mark.parametrize("rs", [1e-160, 1e-3, 0.7, 1e3, 1e50, 1e100, 1e160, np.inf])
 def test_fp64_forces_at_extreme_split_scales(ph, rs):
     """From no long-range part at all (rs far above the box: Newtonian forces)
