@@ -491,8 +491,8 @@ __device__ __forceinline__ double comp_streams(float2 sc, int m)
 // about a tenth of it is long; lists of up to 32 entries (one batch) never
 // are.  The rule looks at the leaf's own box only, so a box gives the same
 // forces in a batch and alone.  P2P of a pass, a warp per leaf -> with the
-// long leaves split: 4,096 grid particles leaf 16, 0.129 -> 0.046 ms; 32,768,
-// 0.199 -> 0.159; 250,047 half in halos, leaf 24, 3.60 -> 3.00; 2,097,152 of
+// long leaves split: 4,096 grid particles leaf 16, 0.129 -> 0.047 ms; 32,768,
+// 0.199 -> 0.164; 250,047 half in halos, leaf 24, 3.60 -> 3.02; 2,097,152 of
 // them 26.0 -> 25.9; 100,003, leaf 8, 1.74 -> 1.34.
 __device__ __forceinline__ int ow_limit(const BoxParams &B, int maxleaf) { return max(32, B.count / (100 * maxleaf)); }
 

@@ -86,15 +86,15 @@ __device__ __forceinline__ long long order_key(double x)
     return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
 }
 
-// one root per box: its particle range and the box [0, L]^3 as
-// src/fmm.c:194-197 derives the root from the domain box (centre 0.5*(L+0),
-// width L-0, src/toptree.c:150-159)
 // the state of a node of len particles not yet split
 __device__ __forceinline__ int open_mode(const BuildBufs &b, int len)
 {
     return len <= b.sub ? MODE_DEFERRED : (len <= b.mid ? MODE_MID : MODE_PENDING);
 }
 
+// one root per box: its particle range and the box [0, L]^3 as
+// src/fmm.c:194-197 derives the root from the domain box (centre 0.5*(L+0),
+// width L-0, src/toptree.c:150-159)
 __global__ void k_init_roots(BuildBufs b, int n, int top)
 {
     ph::chain_begin();
