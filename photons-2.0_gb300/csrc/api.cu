@@ -793,8 +793,8 @@ static int ph_enqueue_tree(photons_ctx *c, const double *src, int levels)
 }
 
 // build flags after the stream has finished: capacity overflow is an error
-// of the reference's rule; PH_FLAG_SUBTREE asks for smaller subtrees; PH_FLAG_TOP asks for more levels of wide nodes,
-// PH_FLAG_DEPTH for a deeper bound (*grow: the bound to build again with)
+// of the reference's rule; PH_FLAG_SUBTREE asks for smaller subtrees,
+// PH_FLAG_TOP for more levels of wide nodes, PH_FLAG_DEPTH for a deeper bound (*grow: the bound to build again with)
 static int ph_check_build(photons_ctx *c, int flags, int levels, int *grow)
 {
     *grow = 0;
@@ -832,6 +832,7 @@ static void ph_tree_info_from(photons_ctx *c, const int *h, int levels)
     c->info.depth = h[ph::BC_DEPTH];
     c->info.levels = h[ph::BC_NLEVELS];
     c->info.flags = h[ph::BC_FLAGS];
+    if (h[ph::BC_EMPTY] == 0) c->sub_n = 0;  // small subtrees are for trees with empty leaves
     // keep the launch counts while they cover the tree with a small margin,
     // so repeated passes over similar trees reuse one captured graph: the
     // depth bound over the deepest depth, the levels of wide nodes over the
@@ -875,6 +876,7 @@ static int ph_stage_build_boxes(photons_ctx *c, int nbox, const photons_params *
         h[ph::BC_DEPTH] = info.depth;
         h[ph::BC_NLEVELS] = info.levels;
         h[ph::BC_FLAGS] = info.flags;
+        h[ph::BC_EMPTY] = c->b.sub == PH_SUB_SMALL;  // (not read back here: taken to need them)
         ph_tree_info_from(c, h, levels);
         c->ndepth = info.depth + 1;
         break;

@@ -3,11 +3,12 @@ coordinate (sheets, lines, lattices), the rounded mean can fall below every
 one of them, and the lower child then holds nothing (as in the reference).
 
 The GPU's mean is a lane-strided sum, the oracle's a sequential one, so on
-such input the two round differently and the oracle's tree is another.  The
-tree is therefore compared with a replay of the split rule in the GPU's
-order of additions, and the forces with a direct sum over all 27 images
-(theta 0 and a cutoff beyond the images: every leaf pair is evaluated, so
-the forces do not depend on the tree)."""
+such input the two mostly round differently and the oracle's tree is
+another.  The tree is therefore compared with a replay of the split rule in
+the GPU's order of additions, and the forces with a direct sum over all 27
+images (theta 0 and a cutoff beyond the images: every leaf pair is
+evaluated, so the forces do not depend on the tree).  A few small sets where
+both orders give one tree pin the lists, moments and forces to the oracle."""
 import numpy as np
 import pytest
 from scipy.special import erfc
@@ -211,3 +212,33 @@ def test_subtree_with_more_leaves_than_one_block_holds(ph, graph, monkeypatch):
     fp.run(sheet(3000, 1.3), dict(p, maxleaf=16), precision=ph.FP64)
     check_tree(fp, sheet(3000, 1.3), 16)
     fp.close()
+
+
+@pytest.mark.parametrize("n,maxleaf,z,seed,axis,sheet_only", [
+    (342, 2, 89.47, 72207, 2, False), (286, 2, 7.35, 199521, 2, False), (248, 2, 99.85, 905296, 2, False),
+    (111, 2, 90.09, 864797, 1, True), (266, 2, 29.37, 523163, 1, False), (355, 2, 53.93, 810033, 1, False),
+    (54, 2, 50.42, 939406, 2, True), (369, 2, 30.37, 564142, 0, False)])
+def test_lists_and_forces_with_empty_leaves_match_oracle(ph, fp, port, n, maxleaf, z, seed, axis, sheet_only):
+    """Sets with empty leaves whose tree is the oracle's: every list, the
+    moments and the forces (FP64 bar) as the oracle's, mutual and one way."""
+    rng = np.random.default_rng(seed)
+    pos = rng.uniform(0.0, 100.0, (n, 3))
+    pos[:, axis] = z
+    if not sheet_only:
+        pos[n // 2:] = rng.uniform(0.0, 100.0, (n - n // 2, 3))
+    p = dict(boxsize=100.0, theta=0.7, rs=8.0, rcut=36.0, eps=0.1, mass=1.0, maxleaf=maxleaf)
+    r = port.run(pos, p, capture=True, tree=True, nthreads=4)
+    assert (r["tree"]["leaf_npart"] == 0).any()
+    for flags in (0, ph.F_ONE_WAY):
+        acc = fp.run(pos, p, precision=ph.FP64, flags=flags | ph.F_TREE_ORDER | ph.F_KEEP_LISTS | ph.F_MULTIPOLES)
+        tr = fp.tree()
+        for k in ("leaf_ipart", "leaf_npart", "node_npart", "node_son"):
+            assert np.array_equal(tr[k], r["tree"][k]), k
+        for kind, (t, s, im) in fp.lists().items():
+            a = np.stack([t, s, im], 1)
+            b = np.stack([np.asarray(x) for x in r["lists"][kind]], 1)
+            assert np.array_equal(a[np.lexsort(a.T)], b[np.lexsort(b.T)]), kind
+        for k in ("leaf_M", "node_M"):
+            assert np.abs(tr[k] - r["tree"][k]).max() <= 1e-11 * np.abs(r["tree"][k]).max(), k
+        scale = np.linalg.norm(r["acc"], axis=1)
+        assert (np.linalg.norm(acc - r["acc"], axis=1) <= 1e-10 * scale).all()
