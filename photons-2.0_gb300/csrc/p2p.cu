@@ -474,32 +474,13 @@ __device__ __forceinline__ int ow_stage(const P2PArgs &A, const uint32_t *list, 
     return nfit;
 }
 
-// a compensated FP32 sum (s, c) in FP64
-__device__ __forceinline__ double comp_d(float2 v) { return (double)v.x - (double)v.y; }
-
 // the streams of each target (lanes equal modulo m) added up in FP64, in a
-// fixed tree
-__device__ __forceinline__ double comp_streams(float2 v, int m)
+// fixed tree: compensated sums (s, c) of FP32 terms in, their sum out
+__device__ __forceinline__ double comp_streams(float2 sc, int m)
 {
-    double r = comp_d(v);
-    for (int o = 16; o >= m; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    return r;
-}
-
-// the same for two rounds of at most 16 targets at once: the lower half of
-// the warp ends with the first one's sums, the upper half with the second's
-__device__ __forceinline__ double comp_streams2(float2 v1, float2 v2, int m1, int m2, int lane)
-{
-    const bool up = lane & 16;
-    const float2 own = up ? v2 : v1, give = up ? v1 : v2;
-    const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, give.x, 16), __shfl_xor_sync(0xffffffffu, give.y, 16));
-    double r = comp_d(own) + comp_d(got);
-    const int m = up ? m2 : m1, low = min(m1, m2);
-    for (int o = 8; o >= low; o >>= 1) {
-        const double t = __shfl_xor_sync(0xffffffffu, r, o);
-        if (o >= m) r += t;
-    }
-    return r;
+    double v = (double)sc.x - (double)sc.y;
+    for (int o = m; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // Leaves whose lists are long against a warp's even share of their box's
@@ -637,18 +618,16 @@ __global__ void __launch_bounds__(P2P_TB, P2P_MINB) k_p2p_split_packed(P2PArgs A
             static_assert(3 * 64 * sizeof(double) <= sizeof s_x[0], "the sums fit a stage");
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                double v;
-                int q = lane;  // the target whose sum this lane has (nb or more: none)
+                // lane l has the sum of target l modulo the round's width, so up to 32
+                // targets are a lane each
+                double v = comp_streams(v1[d], m1);
                 if (m1 < 32 && m2) {
-                    v = comp_streams2(v1[d], v2[d], m1, m2, lane);
-                    q = lane < 16 ? (lane < m1 ? lane : nb) : lane - 16 + m1;
-                } else {
-                    v = comp_streams(v1[d], m1);
-                    if (lane >= m1) q = nb;
+                    const double v_2 = comp_streams(v2[d], m2);
+                    if (lane >= m1) v = v_2;
                 }
-                if (q < nb) {
-                    if (W == 1) out[d][it + tb + q] += v * B.acc_scale;
-                    else red[64 * d + q] = v;
+                if (lane < nb) {
+                    if (W == 1) out[d][it + tb + lane] += v * B.acc_scale;
+                    else red[64 * d + lane] = v;
                 }
                 if (m1 == 32 && m2) {
                     v = comp_streams(v2[d], m2);
